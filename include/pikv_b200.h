@@ -381,6 +381,14 @@ int pikv_quant_block(const void* x, int32_t dtype, int32_t N, int32_t H, int32_t
                      const float* params_in, float* params_out,
                      float* dq_out, float* q_out, float* sq_err,
                      void* workspace, size_t workspace_bytes, pikv_stream_t stream);
+/* K and V of one forward, in one launch of each pass.  dq_k / dq_v [N][H] have the input's dtype; params_in as
+ * above, shared by both.  *mse = mean squared error of V's last group (what QuantizedCompressor.forward keeps);
+ * sample_count (optional, fp32) is increased by count_add. */
+size_t pikv_quant_block_pair_workspace_bytes(int32_t N, int32_t H, int32_t group_size);
+int pikv_quant_block_pair(const void* k, const void* v, int32_t dtype, int32_t N, int32_t H, int32_t group_size,
+                          int32_t qmin, int32_t qmax, int32_t symmetric, const float* params_in,
+                          void* dq_k, void* dq_v, float* mse, float* sample_count, float count_add,
+                          void* workspace, size_t workspace_bytes, pikv_stream_t stream);
 
 /* ------------------------------------------------------------------------
  * H2O scoring and eviction.

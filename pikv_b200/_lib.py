@@ -163,6 +163,8 @@ SIGNATURES = {
     "pikv_cache_gather": (i32, [vp, vp, i32, vp, i32, i32, i32, i32, i32, vp, vp, vp, vp, vp, vp, vp]),
     "pikv_quant_block_workspace_bytes": (sz, [i32, i32, i32]),
     "pikv_quant_block": (i32, [vp, i32, i32, i32, i32, i32, i32, i32, vp, vp, vp, vp, vp, vp, sz, vp]),
+    "pikv_quant_block_pair_workspace_bytes": (sz, [i32, i32, i32]),
+    "pikv_quant_block_pair": (i32, [vp, vp, i32, i32, i32, i32, i32, i32, i32, vp, vp, vp, vp, vp, f32, vp, sz, vp]),
     "pikv_h2o_accumulate": (i32, [vp, vp, i32, vp, vp, i32, f32, f32, vp, vp]),
     "pikv_h2o_select": (i32, [vp, vp, i32, i32, vp, i32, i32, i32, vp, vp, i32, vp, vp]),
     "pikv_h2o_compact": (i32, [C.POINTER(CompactParams), vp]),

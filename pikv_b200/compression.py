@@ -184,10 +184,6 @@ class QuantizedCompressor(BaseCompressor):
     def _qrange(self) -> Tuple[int, int]:
         return 0, 2 ** self.bits - 1
 
-    def _run(self, flat: torch.Tensor, params_in):
-        qmin, qmax = self._qrange()
-        return ops.quant_block(flat, self.group_size, qmin, qmax, self.symmetric, params_in=params_in)
-
     def _static_params(self, keys_flat: torch.Tensor, groups: int):
         # the first block quantised (keys, group 0) fixes one scale / zero point for everything after
         if not self.calibrated:
@@ -205,13 +201,12 @@ class QuantizedCompressor(BaseCompressor):
         vf = values.reshape(-1, shape[-1])
         groups = (shape[-1] + self.group_size - 1) // self.group_size
         params_in = None if self.dynamic_quantization else self._static_params(kf, groups)
-        dk, _, _, _ = self._run(kf, params_in)
-        dv, _, _, err = self._run(vf, params_in)
         with torch.no_grad():
-            last_w = shape[-1] - (groups - 1) * self.group_size
-            self.quantization_error = err[-1] / float(vf.shape[0] * last_w)   # the last block quantised: values, last group
-            self.sample_count += 2 * groups
-        return dk.to(keys.dtype).reshape(shape), dv.to(values.dtype).reshape(shape)
+            qmin, qmax = self._qrange()
+            dk, dv, self.quantization_error = ops.quant_block_pair(
+                kf, vf, self.group_size, qmin, qmax, self.symmetric, params_in=params_in,
+                sample_count=self.sample_count, count_add=2.0 * groups)
+        return dk.view(shape), dv.view(shape)
 
     def get_compression_stats(self) -> Dict[str, float]:
         stats = super().get_compression_stats()

@@ -151,14 +151,11 @@ class QuantizedCompressor(BaseCompressor):
         groups = (shape[-1] + self.group_size - 1) // self.group_size
         qmin, qmax = self._qrange()
         params_in = None if self.dynamic else self._static_params(kf[:, : self.group_size], groups)
-        dk, _, _, _ = ops.quant_block(kf, self.group_size, qmin, qmax, self.symmetric, params_in=params_in)
-        dv, _, _, err = ops.quant_block(vf, self.group_size, qmin, qmax, self.symmetric, params_in=params_in)
-        with torch.no_grad():
-            last_w = shape[-1] - (groups - 1) * self.group_size
-            self.quantization_error = err[-1] / float(vf.shape[0] * last_w)
+        dk, dv, self.quantization_error = ops.quant_block_pair(kf, vf, self.group_size, qmin, qmax, self.symmetric,
+                                                               params_in=params_in)
         original = keys.numel() + values.numel()
         self._update_stats(original, int(original * self.bits / 32))
-        return dk.to(keys.dtype).reshape(shape), dv.to(values.dtype).reshape(shape)
+        return dk.view(shape), dv.view(shape)
 
     def get_compression_stats(self) -> Dict[str, float]:
         stats = super().get_compression_stats()

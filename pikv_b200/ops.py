@@ -198,6 +198,35 @@ def quant_block(x: torch.Tensor, group_size: int, qmin: int, qmax: int, symmetri
     return dq, q, params, err
 
 
+def quant_block_pair(k: torch.Tensor, v: torch.Tensor, group_size: int, qmin: int, qmax: int, symmetric: bool,
+                     params_in: Optional[torch.Tensor] = None, sample_count: Optional[torch.Tensor] = None,
+                     count_add: float = 0.0):
+    """quant_block on K and V [N,H] of one forward, both tensors in each launch when they agree in shape and dtype.
+    Returns (dk, dv in the input's dtype, mean squared error of V's last group as a 0-dim tensor); sample_count (a
+    one-element counter) grows by count_add."""
+    k, v = _req(k, "keys"), _req(v, "values")
+    if sample_count is not None and (sample_count.dtype != torch.float32 or sample_count.device != k.device):
+        sample_count += count_add                     # not a word the kernel can add to
+        sample_count = None
+    if k.shape != v.shape or k.dtype != v.dtype:
+        dk, _, _, _ = quant_block(k, group_size, qmin, qmax, symmetric, params_in=params_in, want_err=False)
+        dv, _, _, err = quant_block(v, group_size, qmin, qmax, symmetric, params_in=params_in)
+        if sample_count is not None:
+            sample_count += count_add
+        last = v.shape[1] - (err.numel() - 1) * group_size
+        return dk.to(k.dtype), dv.to(v.dtype), err[-1] / float(v.shape[0] * last)
+    N, H = k.shape
+    dk, dv = torch.empty_like(k), torch.empty_like(v)
+    mse = torch.empty((), dtype=torch.float32, device=k.device)
+    if params_in is not None:
+        params_in = _req(params_in, "params_in", torch.float32)
+    ws = _workspace(k.device, lib().pikv_quant_block_pair_workspace_bytes(N, H, group_size), "qb2")
+    check(lib().pikv_quant_block_pair(_p(k), _p(v), _dtype_code(k, "keys"), N, H, group_size, qmin, qmax,
+                                      int(bool(symmetric)), _p(params_in), _p(dk), _p(dv), _p(mse), _p(sample_count),
+                                      float(count_add), _p(ws), ws.numel(), _stream()), "pikv_quant_block_pair")
+    return dk, dv, mse
+
+
 # ------------------------------------------------------------------ H2O
 def h2o_accumulate(acc: torch.Tensor, ts: torch.Tensor, idx: Optional[torch.Tensor], w: torch.Tensor, now: float,
                    decay: float = 1.0, status: Optional[torch.Tensor] = None) -> None:
