@@ -579,6 +579,16 @@ int pikv_h2o_accumulate_probs(const void* probs16, int32_t probs_stride, const f
 int pikv_lowrank_project(const void* x, const void* w, const float* bias, const void* residual,
                          void* out, int32_t out_dtype, int32_t M, int32_t N, int32_t K, int32_t relu,
                          pikv_stream_t stream);
+/* the same with the bias in the dtype of the layer that owns it (PIKV_F32 or PIKV_BF16) */
+int pikv_lowrank_project_bias(const void* x, const void* w, const void* bias, int32_t bias_dtype, const void* residual,
+                              void* out, int32_t out_dtype, int32_t M, int32_t N, int32_t K, int32_t relu,
+                              pikv_stream_t stream);
+/* Round trip of K and V in one launch: out[t] = relu(x[t] . w1[t]^T + b1[t]) . w2[t]^T + b2[t], t = 0, 1 (host arrays of
+ * device pointers); x [M,K], w1 [R,K], w2 [N,R], out [M,N] bf16, biases (or NULL) in bias_dtype, the latent rounded to
+ * bf16 in between.  R a multiple of 16 up to 64, N <= 4096. */
+int pikv_lowrank_pair(const void* const* x, const void* const* w1, const void* const* b1, const void* const* w2,
+                      const void* const* b2, int32_t bias_dtype, void* const* out, int32_t M, int32_t K, int32_t R,
+                      int32_t N, pikv_stream_t stream);
 /* Reads and clears the sticky device error word of the projection kernel (non-zero: a
  * bounded mbarrier wait ran out and the output is invalid).  Copies from the device, so
  * it waits for the work queued before it. */

@@ -177,6 +177,9 @@ SIGNATURES = {
     "pikv_h2o_accumulate_probs": (i32, [vp, i32, vp, i32, vp, vp, i32, i32, i32, vp, i32, vp]),
     "pikv_h2o_accumulate_attn": (i32, [vp, i32, vp, vp, i32, i32, i32, vp, i32, vp]),
     "pikv_lowrank_project": (i32, [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, vp]),
+    "pikv_lowrank_project_bias": (i32, [vp, vp, vp, i32, vp, vp, i32, i32, i32, i32, i32, vp]),
+    "pikv_lowrank_pair": (i32, [C.POINTER(vp), C.POINTER(vp), C.POINTER(vp), C.POINTER(vp), C.POINTER(vp), i32, C.POINTER(vp),
+                                i32, i32, i32, i32, vp]),
     "pikv_lowrank_error_state": (i32, []),
     "pikv_a2a_record_bytes": (sz, [i32]),
     "pikv_a2a_pack": (i32, [vp, vp, i32, i32, i32, i32, vp, vp, vp, vp, vp, vp]),

@@ -151,9 +151,24 @@ class SVDCompressor(BaseCompressor):
     def reconstruct(self, latent: torch.Tensor, which: str = "key") -> torch.Tensor:
         return _linear(self.key_reconstructor if which == "key" else self.value_reconstructor, latent, False)
 
+    #: rows of K (and of V) from which the round trip of both is one kernel: it has one CTA per 128 rows, and below
+    #: this (64 CTAs) the separate products, which also spread over their columns, use more of the chip
+    PAIR_ROWS = 4096
+
+    def _round_trip(self, keys: torch.Tensor, values: torch.Tensor):
+        H, R = self.hidden_size, self.rank
+        if (keys.shape == values.shape and keys.dtype == values.dtype == torch.bfloat16 and keys.is_cuda and R % 16 == 0 and R <= 64
+                and H % 16 == 0 and H <= 4096 and keys.numel() >= self.PAIR_ROWS * H):
+            down, up = (self.key_projector, self.value_projector), (self.key_reconstructor, self.value_reconstructor)
+            rk, rv = ops.lowrank_pair((keys.reshape(-1, H), values.reshape(-1, H)),
+                                      [m.weight.detach().to(torch.bfloat16) for m in down], [m.bias.detach() for m in down],
+                                      [m.weight.detach().to(torch.bfloat16) for m in up], [m.bias.detach() for m in up])
+            return rk.view(keys.shape), rv.view(values.shape)
+        return (self.reconstruct(self.project(keys, "key"), "key"),
+                self.reconstruct(self.project(values, "value"), "value"))
+
     def forward(self, keys: torch.Tensor, values: torch.Tensor, importance: Optional[torch.Tensor] = None):
-        rk = self.reconstruct(self.project(keys, "key"), "key")
-        rv = self.reconstruct(self.project(values, "value"), "value")
+        rk, rv = self._round_trip(keys, values)
         with torch.no_grad():
             self.sample_count += 1
         return rk, rv

@@ -7,6 +7,7 @@
 #include <stdint.h>
 #include <stdio.h>
 #include <stdarg.h>
+#include <atomic>
 
 #include "../../include/pikv_b200.h"
 
@@ -25,6 +26,19 @@ int  check_launch(const char* what);   // cudaGetLastError -> status
             return (code);                                 \
         }                                                  \
     } while (0)
+
+// lets a kernel without static shared memory have all 227 KB of an SM; asks the runtime once per device
+template <auto Kernel>
+static inline bool allow_smem() {
+    static std::atomic<uint64_t> done{0};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    const uint64_t bit = 1ull << (dev & 63);
+    if (done.load(std::memory_order_acquire) & bit) return true;
+    if (cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess) return false;
+    done.fetch_or(bit, std::memory_order_release);
+    return true;
+}
 
 static inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 static inline int64_t ceil_div64(int64_t a, int64_t b) { return (a + b - 1) / b; }

@@ -36,6 +36,14 @@ __device__ __forceinline__ void lr_tma_load_2d(uint32_t dst, const CUtensorMap* 
         "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
         ::"r"(dst), "l"(tm), "r"(c0), "r"(c1), "r"(bar) : "memory");
 }
+// whole 2D tile from shared memory; rows and columns past the tensor's end are not written
+__device__ __forceinline__ void lr_tma_store_2d(const CUtensorMap* tm, uint32_t src, int c0, int c1) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];"
+                 ::"l"(tm), "r"(c0), "r"(c1), "r"(src) : "memory");
+}
+__device__ __forceinline__ void lr_mbar_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
 __device__ __forceinline__ void lr_prefetch_tmap(const CUtensorMap* tm) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(tm) : "memory");
 }
@@ -76,6 +84,21 @@ __device__ __forceinline__ void lr_tmem_ld16(uint32_t taddr, float (&v)[16]) {
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// 32 columns of this thread's lane, one wait
+__device__ __forceinline__ void lr_tmem_ld32(uint32_t taddr, float* v) {
+    uint32_t r[32];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr) : "memory");
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+}
+
 #endif  // __CUDACC__
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -94,18 +117,18 @@ static inline EncodeTiledFn encode_fn() {
     return fn;
 }
 
-// 2D bf16 row-major [rows, cols] tensor, box [box_rows, 64 cols], 128-byte swizzle
-static inline int make_tmap(CUtensorMap* tm, const void* base, int rows, int cols, int box_rows) {
+// 2D row-major [rows, cols] tensor of 2- or 4-byte elements, box [box_rows, 128 bytes], 128-byte swizzle
+static inline int make_tmap_of(CUtensorMap* tm, CUtensorMapDataType type, int elem, const void* base, int rows, int cols, int box_rows) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) {
         set_error("tensor map: cuTensorMapEncodeTiled entry point not available");
         return PIKV_ECUDA;
     }
     cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
-    cuuint32_t box[2] = {(cuuint32_t)LR_BK, (cuuint32_t)box_rows};
+    cuuint64_t strides[1] = {(cuuint64_t)cols * elem};
+    cuuint32_t box[2] = {(cuuint32_t)(128 / elem), (cuuint32_t)box_rows};
     cuuint32_t estr[2] = {1, 1};
-    CUresult r = fn(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+    CUresult r = fn(tm, type, 2, const_cast<void*>(base), dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
@@ -113,6 +136,12 @@ static inline int make_tmap(CUtensorMap* tm, const void* base, int rows, int col
         return PIKV_ECUDA;
     }
     return PIKV_OK;
+}
+static inline int make_tmap(CUtensorMap* tm, const void* base, int rows, int cols, int box_rows) {
+    return make_tmap_of(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, rows, cols, box_rows);
+}
+static inline int make_tmap_f32(CUtensorMap* tm, const void* base, int rows, int cols, int box_rows) {
+    return make_tmap_of(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, rows, cols, box_rows);
 }
 
 }  // namespace pikv

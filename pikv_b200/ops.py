@@ -286,14 +286,36 @@ def lowrank_project(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tenso
     if w.shape[1] != K:
         raise PikvError(f"w is {tuple(w.shape)}, expected [N,{K}]")
     if bias is not None:
-        bias = _req(bias.to(torch.float32), "bias", torch.float32)
+        bias = _req(bias if bias.dtype in (torch.float32, torch.bfloat16) else bias.to(torch.float32), "bias")
     if residual is not None:
         residual = _req(residual, "residual", torch.bfloat16)
     out = torch.empty(M, N, dtype=out_dtype, device=x.device)
     code = _lib.PIKV_BF16 if out_dtype == torch.bfloat16 else _lib.PIKV_F32
-    check(lib().pikv_lowrank_project(_p(x), _p(w), _p(bias), _p(residual), _p(out), code, M, N, K, int(bool(relu)),
-                                     _stream()), "pikv_lowrank_project")
+    check(lib().pikv_lowrank_project_bias(_p(x), _p(w), _p(bias), _lib.PIKV_F32 if bias is None else _dtype_code(bias, "bias"),
+                                          _p(residual), _p(out), code, M, N, K, int(bool(relu)), _stream()),
+          "pikv_lowrank_project_bias")
     return out
+
+
+def lowrank_pair(xs, w1s, b1s, w2s, b2s):
+    """relu(x @ w1.T + b1) @ w2.T + b2 for the two (x, w1, b1, w2, b2) of K and V in one launch; bf16, biases all fp32,
+    all bf16 or None.  See pikv_lowrank_pair for the shapes it takes."""
+    xs, w1s, w2s = ([_req(t, n, torch.bfloat16) for t in ts] for ts, n in ((xs, "x"), (w1s, "w1"), (w2s, "w2")))
+    M, K = xs[0].shape
+    R, N = w1s[0].shape[0], w2s[0].shape[0]
+    for x, w1, w2 in zip(xs, w1s, w2s):
+        if x.shape != (M, K) or w1.shape != (R, K) or w2.shape != (N, R):
+            raise PikvError(f"lowrank_pair: x {tuple(x.shape)}, w1 {tuple(w1.shape)}, w2 {tuple(w2.shape)} do not fit")
+    biases = [b for b in (*b1s, *b2s) if b is not None]
+    code = _dtype_code(biases[0], "bias") if biases else _lib.PIKV_F32
+    if any(b.dtype != biases[0].dtype for b in biases):
+        raise PikvError("lowrank_pair: the biases must share their dtype")
+    keep = [None if b is None else _req(b, "bias") for b in (*b1s, *b2s)]
+    outs = [torch.empty(M, N, dtype=torch.bfloat16, device=xs[0].device) for _ in range(2)]
+    arr = lambda ts: (C.c_void_p * 2)(*[None if t is None else t.data_ptr() for t in ts])   # noqa: E731
+    check(lib().pikv_lowrank_pair(arr(xs), arr(w1s), arr(keep[:2]), arr(w2s), arr(keep[2:]), code, arr(outs), M, K, R, N,
+                                  _stream()), "pikv_lowrank_pair")
+    return outs
 
 
 # ------------------------------------------------------------------ all-to-all records
