@@ -121,22 +121,43 @@ typedef struct {
 #define PIKV_GATE_FORCE_SIMT 0x100
 
 size_t pikv_gate_workspace_bytes(int32_t T, int32_t E, int32_t top_k);
+/* what pikv_gate_fused and pikv_route_append need of it (no partial logits of the two-layer net) */
+size_t pikv_gate_tail_workspace_bytes(int32_t T, int32_t E, int32_t top_k);
 int    pikv_gate_fused(const pikv_gate_params* p, pikv_stream_t stream);
 /* bf16 activations run on the tcgen05 kernel (TMA + tensor memory), fp32 ones on the SIMT
  * kernel.  Reads and clears the tensor-core kernel's sticky error word (non-zero: a bounded
  * mbarrier wait ran out and the outputs are invalid); waits for the work queued before it. */
 int    pikv_gate_error_state(void);
 
-/* The whole gate net in one kernel: logits = relu(x . w1^T + b1) . w2^T + b2, then the same tail and outputs as
+/* The whole gate net: logits = relu(x . w1^T + b1) . w2^T + b2, then the same tail and outputs as
  * pikv_gate_fused (the router's nn.Sequential(Linear, ReLU, Linear), core/single/pikv_routing.py:34-38, whose
  * first layer is the one dense contraction of "route": [T,K] x [K,H] on tcgen05 tensor cores, fp32 accumulation
- * in tensor memory).  The hidden activations never go to HBM: each 128-token tile keeps them in shared memory,
- * 256 hidden units at a time, as the operand of the second product.
- *   p: as for pikv_gate_fused with H = hidden units (inputs of w2 [E,H]); p->act is ignored; bf16; E <= 32;
- *   T <= 131072 per call; phase PIKV_GATE_WHOLE.
+ * in tensor memory).  The hidden activations never go to HBM: a pair of CTAs turns its 256 tokens x 256 hidden units
+ * into partial logits, which a second kernel sums in a fixed order.
+ *   p: as for pikv_gate_fused with H = hidden units (inputs of w2 [E,H]); p->act is ignored; bf16;
+ *   T <= 131072 per call; phase PIKV_GATE_WHOLE; workspace of pikv_gate_workspace_bytes.
  *   x [T,K] bf16, w1 [H,K] bf16, b1 [H] fp32 or NULL. */
 int pikv_gate_mlp_fused(const pikv_gate_params* p, const void* x, int32_t K, const void* w1, const float* b1,
                         pikv_stream_t stream);
+
+/* Dense [T,E,capacity] dispatch / combine tensors of a gate and the router's auxiliary loss:
+ *   position_mode 0: slot (running count, core/single/module/pikv_routing.py:93-104); 1: the positions
+ *   core/single/pikv_routing.py:107-128 produces ("number of earlier k-columns in which this expert was chosen
+ *   by any token").
+ *   p = prob_sum / T ; *aux = sum p log(p E + 1e-9) + coefficient times the balance term of TopKBalancedRouter
+ *   (core/single/pikv_routing.py:155-159, 185-222): balance 0 none, 1 entropy, 2 cv, 3 l2. */
+typedef struct {
+    float*  dispatch;          /* [T,E,capacity], 16-byte aligned                */
+    float*  combine;
+    int32_t capacity, position_mode, balance;
+    float   coefficient;
+    float*  aux;               /* one float, or NULL                             */
+} pikv_dense_out;
+
+/* pikv_gate_mlp_fused with both biases in bias_dtype (p->b2 is ignored) and, dense != NULL, the dense outputs: the
+ * first kernel clears them while its tensor cores work (T * E * capacity a multiple of 4), the last one fills them. */
+int pikv_gate_mlp_dense(const pikv_gate_params* p, const void* x, int32_t K, const void* w1, const void* b1,
+                        const void* b2, int32_t bias_dtype, const pikv_dense_out* dense, pikv_stream_t stream);
 
 /* Dense [T,E,capacity] dispatch / combine tensors (zero-filled by this call)
  * for callers that read them.  position_mode 0: slot as given (running count,
@@ -147,6 +168,10 @@ int pikv_dispatch_scatter(const int32_t* topk_idx, const float* topk_w, const in
                           const int32_t* counts_k, int32_t T, int32_t E, int32_t top_k,
                           int32_t capacity, int32_t position_mode,
                           float* dispatch, float* combine, pikv_stream_t stream);
+/* the same with the loss, from a gate's outputs (prob_sum may be NULL without aux) */
+int pikv_dispatch_loss(const int32_t* topk_idx, const float* topk_w, const int32_t* slot, const int32_t* counts_k,
+                       const float* prob_sum, int32_t T, int32_t E, int32_t top_k, const pikv_dense_out* dense,
+                       pikv_stream_t stream);
 
 /* ------------------------------------------------------------------------
  * Routed KV append fused with per-(token, head) group quantisation.

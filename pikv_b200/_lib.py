@@ -38,6 +38,11 @@ class GateParams(C.Structure):
     ]
 
 
+class DenseOut(C.Structure):
+    _fields_ = [("dispatch", vp), ("combine", vp), ("capacity", i32), ("position_mode", i32), ("balance", i32),
+                ("coefficient", f32), ("aux", vp)]
+
+
 class AppendParams(C.Structure):
     _fields_ = [
         ("k", vp), ("v", vp), ("dtype", i32), ("T", i32), ("n_kv", i32), ("top_k", i32),
@@ -141,9 +146,12 @@ SIGNATURES = {
     "pikv_last_error": (C.c_char_p, []),
     "pikv_launch_count": (u64, []),
     "pikv_gate_workspace_bytes": (sz, [i32, i32, i32]),
+    "pikv_gate_tail_workspace_bytes": (sz, [i32, i32, i32]),
     "pikv_gate_fused": (i32, [C.POINTER(GateParams), vp]),
     "pikv_gate_error_state": (i32, []),
     "pikv_gate_mlp_fused": (i32, [C.POINTER(GateParams), vp, i32, vp, vp, vp]),
+    "pikv_gate_mlp_dense": (i32, [C.POINTER(GateParams), vp, i32, vp, vp, vp, i32, C.POINTER(DenseOut), vp]),
+    "pikv_dispatch_loss": (i32, [vp, vp, vp, vp, vp, i32, i32, i32, C.POINTER(DenseOut), vp]),
     "pikv_dispatch_scatter": (i32, [vp, vp, vp, vp, i32, i32, i32, i32, i32, vp, vp, vp]),
     "pikv_kv_append_quant": (i32, [C.POINTER(AppendParams), vp]),
     "pikv_kv_append_rope": (i32, [C.POINTER(AppendParams), vp, vp, vp, i32, vp]),

@@ -27,15 +27,16 @@ int  check_launch(const char* what);   // cudaGetLastError -> status
         }                                                  \
     } while (0)
 
-// lets a kernel without static shared memory have all 227 KB of an SM; asks the runtime once per device
+// lets a kernel have that much dynamic shared memory (all 227 KB of an SM when it has no static shared memory); asks
+// the runtime once per device
 template <auto Kernel>
-static inline bool allow_smem() {
+static inline bool allow_smem(int bytes = 227 * 1024) {
     static std::atomic<uint64_t> done{0};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return false;
     const uint64_t bit = 1ull << (dev & 63);
     if (done.load(std::memory_order_acquire) & bit) return true;
-    if (cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess) return false;
+    if (cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return false;
     done.fetch_or(bit, std::memory_order_release);
     return true;
 }

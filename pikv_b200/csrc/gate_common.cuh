@@ -124,6 +124,16 @@ __device__ __forceinline__ void token_tail(float (&l)[EP], const GateDev& g, int
 enum : int { GATE_DO_SCORE = 1, GATE_DO_SLOTS = 2, GATE_RANKS_TO_WS = 4 };
 int gate_run(const pikv_gate_params* p, cudaStream_t st, int what, GateDev* out);
 
+// partial logits of the two-layer gate net (gate_mlp.cu), behind everything else in the workspace: at most
+// gate_max_partials(T) blocks of [T][E].  Short batches use narrow blocks of hidden units to fill the GPU, so they get
+// more of them.
+static inline int gate_max_partials(int T) { return T <= 2048 ? 64 : 16; }
+float* gate_partials(const GateDev& g);
+// the tail of the gate from partial logits, slot finalisation and (dense != null) the dense outputs included; the
+// tensors of `dense` are zero already
+int gate_from_partials(GateDev& g, const float* part, int groups, const void* b2, bool b2_bf16, const pikv_dense_out* dense,
+                       cudaStream_t st);
+
 // tensor-core path (gate_tc.cu): bf16 activations through TMA + tcgen05
 bool gate_tc_supported(const GateDev& g, int dtype);
 void gate_tc_geometry(GateDev& g);                  // sets g.chunk and g.G

@@ -48,16 +48,36 @@ __device__ __forceinline__ void lr_prefetch_tmap(const CUtensorMap* tm) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(tm) : "memory");
 }
 
-// K-major operand tile, 128-byte swizzle: rows of 128 bytes, 8-row groups 1024 bytes apart
-__device__ __forceinline__ uint64_t lr_smem_desc(uint32_t saddr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);          // start address, 16-byte units
-    d |= (uint64_t)1 << 16;                            // leading byte offset (unused for swizzled K-major)
-    d |= (uint64_t)(1024 >> 4) << 32;                  // stride byte offset between 8-row groups
-    d |= (uint64_t)1 << 46;                            // descriptor version (sm_100)
-    d |= (uint64_t)2 << 61;                            // layout: SWIZZLE_128B
-    return d;
+// One lane of a converged warp.  The loops that issue TMA and MMA run on whole warps and only the issuing instructions
+// are inside `if (lr_elect())`: the operands stay warp-uniform values.  (With the whole loop inside `if (lane == 0)` and
+// the stage index taken modulo the ring, a k block cost its issuing thread about 0.5 us whatever its size.)
+__device__ __forceinline__ bool lr_elect() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
+    return p != 0;
 }
+// position in a ring of `stages` buffers: index and the parity its full barrier completes with
+struct LrRing {
+    int s = 0;
+    uint32_t ph = 0;
+    __device__ __forceinline__ void next(int stages) {
+        if (++s == stages) {
+            s = 0;
+            ph ^= 1u;
+        }
+    }
+};
+
+// K-major operand tile, 128-byte swizzle: rows of 128 bytes, 8-row groups 1024 bytes apart.  The low word holds the
+// start address in 16-byte units (16 bf16 further along K: + 2), the high word is the same for every tile.
+constexpr uint32_t LR_DESC_HI = (1024u >> 4)       // stride byte offset between 8-row groups
+                                | (1u << 14)       // descriptor version (sm_100)
+                                | (2u << 29);      // layout: SWIZZLE_128B
+__device__ __forceinline__ uint32_t lr_desc_lo(uint32_t saddr) {
+    return ((saddr & 0x3FFFFu) >> 4) | (1u << 16); // leading byte offset (unused for swizzled K-major)
+}
+__device__ __forceinline__ uint64_t lr_desc(uint32_t lo) { return ((uint64_t)LR_DESC_HI << 32) | lo; }
+__device__ __forceinline__ uint64_t lr_smem_desc(uint32_t saddr) { return lr_desc(lr_desc_lo(saddr)); }
 // kind::f16 instruction descriptor: D=f32, A=B=bf16, both K-major, M=128, N=bn
 __device__ __forceinline__ uint32_t lr_instr_desc(int bn) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(LR_BM >> 4) << 24);

@@ -79,7 +79,7 @@ def gate_fused(act: Optional[torch.Tensor] = None, w2: Optional[torch.Tensor] = 
                expert_mask: Optional[torch.Tensor] = None, mask_mode: int = _lib.MASK_SINGLE,
                correction: Optional[torch.Tensor] = None, temperature: float = 1.0, renorm_eps: float = 0.0,
                capacity: int = 0, slot_base: Optional[torch.Tensor] = None, want_probs: bool = True,
-               out: Optional[GateResult] = None, phase: int = 0, _mlp=None) -> GateResult:
+               out: Optional[GateResult] = None, phase: int = 0, _mlp=None, _dense=None) -> GateResult:
     """Fused gate tail; see pikv_gate_fused in include/pikv_b200.h.
 
     Give either (act [T,H], w2 [E,H], b2 [E]) or logits [T,E] fp32.  phase 1 (scoring kernel only) and
@@ -117,7 +117,7 @@ def gate_fused(act: Optional[torch.Tensor] = None, w2: Optional[torch.Tensor] = 
             topk_idx=torch.empty(T, top_k, **i32), topk_w=torch.empty(T, top_k, **f32),
             slot=torch.empty(T, top_k, **i32), counts_k=torch.empty(top_k, E, **i32),
             prob_sum=torch.empty(E, **f32), new_len=torch.empty(E, **i32))
-    nws = lib().pikv_gate_workspace_bytes(T, E, top_k)
+    nws = (lib().pikv_gate_tail_workspace_bytes if _mlp is None else lib().pikv_gate_workspace_bytes)(T, E, top_k)
     if phase != 0 or out.workspace is not None:
         if out.workspace is None or out.workspace.numel() < nws:
             if phase == 2:
@@ -137,7 +137,7 @@ def gate_fused(act: Optional[torch.Tensor] = None, w2: Optional[torch.Tensor] = 
 
     p = GateParams()
     p.act, p.w2, p.b2, p.logits_in = _p(act) if logits is None else None, _p(w2) if logits is None else None, \
-        f(b2) if logits is None else None, _p(logits)
+        f(b2) if logits is None and _mlp is None else None, _p(logits)
     if _mlp is not None:
         p.act = None
     p.dtype, p.T, p.H, p.E, p.top_k = dt, T, H, E, top_k
@@ -152,8 +152,11 @@ def gate_fused(act: Optional[torch.Tensor] = None, w2: Optional[torch.Tensor] = 
     p.counts_k, p.prob_sum, p.new_len = _p(out.counts_k), _p(out.prob_sum), _p(out.new_len)
     p.workspace, p.workspace_bytes, p.phase = _p(ws), ws.numel(), int(phase)
     if _mlp is not None:
-        b1f = f(b1)
-        check(lib().pikv_gate_mlp_fused(C.byref(p), _p(x), Kin, _p(w1), b1f, _stream()), "pikv_gate_mlp_fused")
+        biases = [b for b in (b1, b2) if b is not None]
+        code = _lib.PIKV_BF16 if biases and all(b.dtype == torch.bfloat16 for b in biases) else _lib.PIKV_F32
+        b1, b2 = (None if b is None else _req(b if code == _lib.PIKV_BF16 else b.to(torch.float32), "bias") for b in (b1, b2))
+        check(lib().pikv_gate_mlp_dense(C.byref(p), _p(x), Kin, _p(w1), _p(b1), _p(b2), code,
+                                        None if _dense is None else C.byref(_dense), _stream()), "pikv_gate_mlp_dense")
         return out
     check(lib().pikv_gate_fused(C.byref(p), _stream()), "pikv_gate_fused")
     return out
@@ -166,15 +169,46 @@ def gate_mlp_fused(x: torch.Tensor, w1: torch.Tensor, b1: Optional[torch.Tensor]
     return gate_fused(None, w2, b2, _mlp=(x, w1, b1), **kw)
 
 
+BALANCE = {None: 0, "entropy": 1, "cv": 2, "l2": 3}
+
+
+def _dense_out(T: int, num_experts: int, capacity: int, position_mode: int, balance: Optional[str], coefficient: float, device):
+    """(dispatch, combine, auxiliary loss) buffers and the descriptor of them the kernels take."""
+    d = torch.empty(T, num_experts, capacity, dtype=torch.float32, device=device)
+    c = torch.empty_like(d)
+    aux = torch.empty((), dtype=torch.float32, device=device)
+    o = _lib.DenseOut()
+    o.dispatch, o.combine, o.aux = d.data_ptr(), c.data_ptr(), aux.data_ptr()
+    o.capacity, o.position_mode, o.balance, o.coefficient = capacity, position_mode, BALANCE[balance], float(coefficient)
+    return (d, c, aux), o
+
+
 def dispatch_scatter(g: GateResult, num_experts: int, capacity: int, position_mode: int = 0):
     """Dense [T,E,capacity] fp32 dispatch and combine tensors from a gate result."""
+    return dispatch_loss(g, num_experts, capacity, position_mode)[:2]
+
+
+def dispatch_loss(g: GateResult, num_experts: int, capacity: int, position_mode: int = 0, balance: Optional[str] = None,
+                  coefficient: float = 0.0):
+    """dispatch_scatter and the router's auxiliary loss (0-dim): the base term of core/single/pikv_routing.py:155-159
+    plus `coefficient` times the balance term of :185-222."""
     T, k = g.topk_idx.shape
-    dev = g.topk_idx.device
-    d = torch.empty(T, num_experts, capacity, dtype=torch.float32, device=dev)
-    c = torch.empty_like(d)
-    check(lib().pikv_dispatch_scatter(_p(g.topk_idx), _p(g.topk_w), _p(g.slot), _p(g.counts_k), T, num_experts, k,
-                                      capacity, position_mode, _p(d), _p(c), _stream()), "pikv_dispatch_scatter")
-    return d, c
+    dense, o = _dense_out(T, num_experts, capacity, position_mode, balance, coefficient, g.topk_idx.device)
+    check(lib().pikv_dispatch_loss(_p(g.topk_idx), _p(g.topk_w), _p(g.slot), _p(g.counts_k), _p(g.prob_sum), T, num_experts, k,
+                                   C.byref(o), _stream()), "pikv_dispatch_loss")
+    return dense
+
+
+def gate_mlp_dense(x: torch.Tensor, w1: torch.Tensor, b1: Optional[torch.Tensor], w2: torch.Tensor, b2: Optional[torch.Tensor],
+                   rows: int, position_mode: int, balance: Optional[str] = None, coefficient: float = 0.0, **kw):
+    """gate_mlp_fused and dispatch_loss (`rows` = capacity dimension of the dense tensors) in one call: the dense tensors
+    are cleared beside the tensor-core work.  Returns (gate result, (dispatch, combine, aux))."""
+    T, E = x.shape[0], w2.shape[0]
+    if T * E * rows % 4:
+        g = gate_mlp_fused(x, w1, b1, w2, b2, **kw)
+        return g, dispatch_loss(g, E, rows, position_mode, balance, coefficient)
+    dense, o = _dense_out(T, E, rows, position_mode, balance, coefficient, x.device)
+    return gate_fused(None, w2, b2, _mlp=(x, w1, b1), _dense=o, **kw), dense
 
 
 # ------------------------------------------------------------------ block-wide fake quantisation

@@ -1,12 +1,13 @@
 """Routers with the constructor / forward surface of core/single/pikv_routing.py.
 
 Same class names, keyword arguments, parameter and buffer names (state_dicts of
-the reference load unchanged) and return tuples.  The gate net's hidden layer
-stays a torch (cuBLAS) GEMM; everything after it - last-layer logits, mask,
-softmax, top-k, renormalisation, per-expert counts and slot assignment - is one
-call of the fused CUDA gate kernel.  The dense dispatch / combine tensors the
-reference returns are produced by a scatter kernel from the compact result,
-which stays available as `router.last_gate`.
+the reference load unchanged) and return tuples.  The gate net's hidden layer is
+a torch (cuBLAS) GEMM in fp32 and part of the tensor-core gate net in bf16;
+everything after it - last-layer logits, mask, softmax, top-k, renormalisation,
+per-expert counts and slot assignment - is one call of the fused CUDA gate
+kernels.  The dense dispatch / combine tensors the reference returns and its
+auxiliary loss come out of the same kernels or of a scatter kernel behind them;
+the compact result stays available as `router.last_gate`.
 
 Modules must live on a CUDA device; there is no CPU path.
 """
@@ -25,6 +26,17 @@ from . import _lib, ops
 def _aux_base(p_mean: torch.Tensor, num_experts: int) -> torch.Tensor:
     # core/single/pikv_routing.py:155-159
     return torch.sum(p_mean * torch.log(p_mean * num_experts + 1e-9))
+
+
+def _balance_term(p: torch.Tensor, mode: Optional[str], coefficient: float, num_experts: int):
+    # core/single/pikv_routing.py:185-222
+    if mode is None:
+        return 0.0
+    if mode == "entropy":
+        return -coefficient * (-torch.sum(p * torch.log(p + 1e-9)) / math.log(num_experts))
+    if mode == "cv":
+        return coefficient * (p.std() / (p.mean() + 1e-9))
+    return coefficient * torch.sum((p - 1.0 / num_experts) ** 2)
 
 
 class BaseRouter(nn.Module):
@@ -63,11 +75,13 @@ class BaseRouter(nn.Module):
         self.last_gate = g
         return g
 
-    def _dense(self, g: ops.GateResult, batch_size: int, seq_len: int, capacity: int):
+    def _dense(self, g: ops.GateResult, batch_size: int, seq_len: int, capacity: int, balance: Optional[str] = None,
+               coefficient: float = 0.0):
+        """(dispatch, combine, auxiliary loss with the balance term)."""
         if self.expert_backend == "fairscale":
-            d, c = ops.dispatch_scatter(g, self.num_experts, capacity, self.position_mode)
-            return (d.view(batch_size, seq_len, self.num_experts, capacity),
-                    c.view(batch_size, seq_len, self.num_experts, capacity))
+            d, c, aux = ops.dispatch_loss(g, self.num_experts, capacity, self.position_mode, balance, coefficient)
+            shape = (batch_size, seq_len, self.num_experts, capacity)
+            return d.view(shape), c.view(shape), aux
         # the "basic" backend of the reference: capacity dimension of 1, every choice written to position 0
         T, k = g.topk_idx.shape
         d = torch.zeros(T, self.num_experts, dtype=torch.float32, device=g.topk_idx.device)
@@ -75,35 +89,52 @@ class BaseRouter(nn.Module):
         idx = g.topk_idx.long()
         d.scatter_(1, idx, 1.0)
         c.scatter_(1, idx, g.topk_w)
-        return (d.view(batch_size, seq_len, self.num_experts, 1), c.view(batch_size, seq_len, self.num_experts, 1))
+        p_mean = g.prob_sum / float(T)
+        return (d.view(batch_size, seq_len, self.num_experts, 1), c.view(batch_size, seq_len, self.num_experts, 1),
+                _aux_base(p_mean, self.num_experts) + _balance_term(p_mean, balance, coefficient, self.num_experts))
 
     def _hidden(self, mlp: nn.Sequential, x2d: torch.Tensor) -> torch.Tensor:
         return F.relu(mlp[0](x2d))
 
+    def _fused_net(self, mlp: nn.Sequential, x2d: torch.Tensor) -> bool:
+        return x2d.dtype == torch.bfloat16 and self.num_experts <= 32 and x2d.shape[1] % 8 == 0 and mlp[0].out_features % 8 == 0
+
+    def _net_weights(self, mlp: nn.Sequential):
+        w = lambda layer: layer.weight.detach().to(torch.bfloat16)              # noqa: E731
+        b = lambda layer: None if layer.bias is None else layer.bias.detach()   # noqa: E731
+        return w(mlp[0]), b(mlp[0]), w(mlp[2]), b(mlp[2])
+
     def _gate_net(self, mlp: nn.Sequential, x2d: torch.Tensor, **kw) -> ops.GateResult:
-        """Gate net + tail.  bf16 inputs: one tensor-core kernel for both layers and the tail (the hidden
-        activations stay on chip).  fp32 inputs (the reference's dtype, 1e-5 parity): the first layer is a torch
-        fp32 GEMM and the kernel takes over from the hidden activations."""
-        if x2d.dtype == torch.bfloat16 and self.num_experts <= 32 and x2d.shape[1] % 8 == 0 and mlp[0].out_features % 8 == 0:
+        """Gate net + tail.  bf16 inputs: both layers and the tail on the tensor-core kernels (the hidden activations
+        stay on chip).  fp32 inputs (the reference's dtype, 1e-5 parity): the first layer is a torch fp32 GEMM and the
+        kernel takes over from the hidden activations."""
+        if self._fused_net(mlp, x2d):
             k = kw.pop("top_k", None) or self.top_k
-            first, last = mlp[0], mlp[2]
-            g = ops.gate_mlp_fused(x2d, first.weight.detach().to(torch.bfloat16),
-                                   None if first.bias is None else first.bias.detach(),
-                                   last.weight.detach().to(torch.bfloat16), None if last.bias is None else last.bias.detach(),
-                                   top_k=k, mask_mode=self.mask_mode, renorm_eps=self.renorm_eps, **kw)
+            g = ops.gate_mlp_fused(x2d, *self._net_weights(mlp), top_k=k, mask_mode=self.mask_mode, renorm_eps=self.renorm_eps, **kw)
             self.last_gate = g
             return g
         return self._gate(self._hidden(mlp, x2d), mlp[2], **kw)
 
-    def forward(self, hidden_states: torch.Tensor, expert_mask: Optional[torch.Tensor] = None):
+    def _route(self, hidden_states: torch.Tensor, expert_mask: Optional[torch.Tensor], balance: Optional[str] = None,
+               coefficient: float = 0.0):
         batch_size, seq_len, hidden_size = hidden_states.shape
         x2d = hidden_states.reshape(-1, hidden_size)
         capacity = self._compute_capacity(batch_size, seq_len)
-        g = self._gate_net(self.router, x2d, expert_mask=expert_mask, capacity=capacity)
-        dispatch, combine = self._dense(g, batch_size, seq_len, max(capacity, 1))
-        p_mean = g.prob_sum / float(batch_size * seq_len)
-        aux_loss = _aux_base(p_mean, self.num_experts)
+        rows = max(capacity, 1)
+        if self.expert_backend == "fairscale" and self._fused_net(self.router, x2d):
+            g, (dispatch, combine, aux_loss) = ops.gate_mlp_dense(
+                x2d, *self._net_weights(self.router), rows, self.position_mode, balance, coefficient, top_k=self.top_k,
+                expert_mask=expert_mask, mask_mode=self.mask_mode, renorm_eps=self.renorm_eps, capacity=capacity)
+            self.last_gate = g
+            shape = (batch_size, seq_len, self.num_experts, rows)
+            dispatch, combine = dispatch.view(shape), combine.view(shape)
+        else:
+            g = self._gate_net(self.router, x2d, expert_mask=expert_mask, capacity=capacity)
+            dispatch, combine, aux_loss = self._dense(g, batch_size, seq_len, rows, balance, coefficient)
         return dispatch, combine, g.probs.view(batch_size, seq_len, self.num_experts), aux_loss
+
+    def forward(self, hidden_states: torch.Tensor, expert_mask: Optional[torch.Tensor] = None):
+        return self._route(hidden_states, expert_mask)
 
 
 class TopKBalancedRouter(BaseRouter):
@@ -116,17 +147,8 @@ class TopKBalancedRouter(BaseRouter):
         self.balance_mode = balance_mode
 
     def forward(self, hidden_states: torch.Tensor, expert_mask: Optional[torch.Tensor] = None):
-        dispatch, combine, probs, aux_loss = super().forward(hidden_states, expert_mask)
-        p = self.last_gate.prob_sum / float(hidden_states.shape[0] * hidden_states.shape[1])
-        if self.balance_mode == "entropy":
-            term = -torch.sum(p * torch.log(p + 1e-9)) / math.log(self.num_experts)
-            balance = -self.balance_coefficient * term
-        elif self.balance_mode == "cv":
-            balance = self.balance_coefficient * (p.std() / (p.mean() + 1e-9))
-        else:
-            uniform = torch.ones_like(p) / self.num_experts
-            balance = self.balance_coefficient * torch.sum((p - uniform) ** 2)
-        return dispatch, combine, probs, aux_loss + balance
+        mode = self.balance_mode if self.balance_mode in ("entropy", "cv") else "l2"
+        return self._route(hidden_states, expert_mask, mode, self.balance_coefficient)
 
 
 class AdaptiveRouter(BaseRouter):
@@ -155,10 +177,8 @@ class AdaptiveRouter(BaseRouter):
         capacity = self._compute_capacity(batch_size, seq_len)
         g = self._gate(None, None, logits=logits.reshape(-1, self.num_experts).float(), expert_mask=expert_mask,
                        capacity=capacity)
-        dispatch, combine = self._dense(g, batch_size, seq_len, max(capacity, 1))
+        dispatch, combine, entropy_loss = self._dense(g, batch_size, seq_len, max(capacity, 1))
         probs = g.probs.view(batch_size, seq_len, self.num_experts)
-        p_mean = g.prob_sum / float(batch_size * seq_len)
-        entropy_loss = _aux_base(p_mean, self.num_experts)
         imp_sum = (probs * imp_mask).sum(dim=[0, 1]) + 1e-9             # :365-372
         imp_per = imp_sum / imp_sum.sum()
         imp_entropy = -torch.sum(imp_per * torch.log(imp_per + 1e-9)) / math.log(self.num_experts)
@@ -203,10 +223,9 @@ class PiKVRouter(AdaptiveRouter):
         capacity = self._compute_capacity(batch_size, seq_len)
         g = self._gate(None, None, logits=logits.reshape(-1, self.num_experts).float(), expert_mask=expert_mask,
                        correction=self.cache_correction_factor.detach(), capacity=capacity)
-        dispatch, combine = self._dense(g, batch_size, seq_len, max(capacity, 1))
+        dispatch, combine, aux_base = self._dense(g, batch_size, seq_len, max(capacity, 1))
         probs = g.probs.view(batch_size, seq_len, self.num_experts)
         usage_norm = g.prob_sum / g.prob_sum.sum()
         self.update_cache_usage(usage_norm)
-        p_mean = g.prob_sum / float(batch_size * seq_len)
-        aux_loss = _aux_base(p_mean, self.num_experts) + 0.05 * torch.sum(self.cache_usage_history * usage_norm)
+        aux_loss = aux_base + 0.05 * torch.sum(self.cache_usage_history * usage_norm)
         return dispatch, combine, probs, aux_loss, importance
