@@ -184,46 +184,44 @@ __global__ void __launch_bounds__(LR_THREADS, 1) lowrank_gemm_kernel(const __gri
     bool failed = false;
 
     if (warp == 0) {
-        if (lane == 0) {
-            int it = 0;
-            for (int item = blockIdx.x; item < a.items && !failed; item += gridDim.x) {
-                const int m0 = item / a.nblocks * LR_BM, n0 = item % a.nblocks * a.bn;
-                for (int kb = 0; kb < num_kb; ++kb, ++it) {
-                    const int s = it % a.stages;
-                    const uint32_t ph = (uint32_t)(it / a.stages) & 1u;
-                    if (!lr_mbar_wait(empty0 + 8 * s, ph ^ 1u)) { failed = true; break; }
-                    lr_mbar_expect_tx(full0 + 8 * s, (uint32_t)stage_bytes);
-                    const uint32_t dst = ring + (uint32_t)s * stride;
-                    lr_tma_load_2d(dst, &tm_x, kb * LR_BK, m0, full0 + 8 * s);
-                    lr_tma_load_2d(dst + stage_a, &tm_w, kb * LR_BK, n0, full0 + 8 * s);
+        LrRing r;
+        for (int item = blockIdx.x; item < a.items && !failed; item += gridDim.x) {
+            const int m0 = item / a.nblocks * LR_BM, n0 = item % a.nblocks * a.bn;
+            for (int kb = 0; kb < num_kb; ++kb, r.next(a.stages)) {
+                if (!lr_mbar_wait(empty0 + 8 * r.s, r.ph ^ 1u)) { failed = true; break; }
+                if (lr_elect()) {
+                    lr_mbar_expect_tx(full0 + 8 * r.s, (uint32_t)stage_bytes);
+                    const uint32_t dst = ring + (uint32_t)r.s * stride;
+                    lr_tma_load_2d(dst, &tm_x, kb * LR_BK, m0, full0 + 8 * r.s);
+                    lr_tma_load_2d(dst + stage_a, &tm_w, kb * LR_BK, n0, full0 + 8 * r.s);
                 }
+                __syncwarp();
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t idesc = lr_instr_desc(a.bn);
-            int it = 0, local = 0;
-            for (int item = blockIdx.x; item < a.items && !failed; item += gridDim.x, ++local) {
-                const int slot = local & 1;
-                if (!lr_mbar_wait(tempty0 + 8 * slot, (((uint32_t)local >> 1) & 1u) ^ 1u)) { failed = true; break; }
+        const uint32_t idesc = lr_instr_desc(a.bn);
+        const uint32_t a_lo = lr_desc_lo(ring), b_lo = lr_desc_lo(ring + stage_a), stage_lo = stride >> 4;
+        LrRing r;
+        int local = 0;
+        for (int item = blockIdx.x; item < a.items && !failed; item += gridDim.x, ++local) {
+            const int slot = local & 1;
+            if (!lr_mbar_wait(tempty0 + 8 * slot, (((uint32_t)local >> 1) & 1u) ^ 1u)) { failed = true; break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t d = tmem_base + (uint32_t)(slot * a.bn);
+            for (int kb = 0; kb < num_kb; ++kb, r.next(a.stages)) {
+                if (!lr_mbar_wait(full0 + 8 * r.s, r.ph)) { failed = true; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t d = tmem_base + (uint32_t)(slot * a.bn);
-                for (int kb = 0; kb < num_kb; ++kb, ++it) {
-                    const int s = it % a.stages;
-                    const uint32_t ph = (uint32_t)(it / a.stages) & 1u;
-                    if (!lr_mbar_wait(full0 + 8 * s, ph)) { failed = true; break; }
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t sa = ring + (uint32_t)s * stride;
-                    const uint32_t sb = sa + stage_a;
+                if (lr_elect()) {
+                    const uint32_t off = (uint32_t)r.s * stage_lo;
 #pragma unroll
-                    for (int k = 0; k < LR_BK / 16; ++k) {
-                        // 16 bf16 = 32 bytes further along K inside the 128-byte swizzle row
-                        lr_mma(d, lr_smem_desc(sa + 32 * k), lr_smem_desc(sb + 32 * k), idesc, (kb | k) ? 1u : 0u);
-                    }
-                    lr_commit(empty0 + 8 * s);       // frees the stage once these MMAs have read it
+                    for (int k = 0; k < LR_BK / 16; ++k)
+                        lr_mma(d, lr_desc(a_lo + off + 2 * k), lr_desc(b_lo + off + 2 * k), idesc, (kb | k) ? 1u : 0u);
+                    lr_commit(empty0 + 8 * r.s);     // frees the stage once these MMAs have read it
                 }
-                lr_commit(tfull0 + 8 * slot);        // accumulator complete (or as far as it got)
+                __syncwarp();
             }
+            if (lr_elect()) lr_commit(tfull0 + 8 * slot);    // accumulator complete (or as far as it got)
+            __syncwarp();
         }
     } else {
         const int lg = warp & 3;                     // tensor-memory lane group of this warp

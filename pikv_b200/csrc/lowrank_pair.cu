@@ -114,74 +114,81 @@ __global__ void __launch_bounds__(LP_THREADS, 1) lowrank_pair_kernel(const __gri
     bool failed = false;
 
     if (warp == 0) {
-        if (lane == 0) {
-            int it = 0;
-            for (int item = blockIdx.x; item < a.items && !failed; item += gridDim.x) {
-                const int t = item / a.tiles, m0 = item % a.tiles * LR_BM;
-                for (int kb = 0; kb < num_kb; ++kb, ++it) {
-                    const int s = it % a.stages;
-                    if (!lr_mbar_wait(empty0 + 8 * s, ((uint32_t)(it / a.stages) & 1u) ^ 1u)) { failed = true; break; }
-                    lr_mbar_expect_tx(full0 + 8 * s, (uint32_t)stage_bytes);
-                    const uint32_t dst = ring + (uint32_t)(s * stage_bytes);
-                    lr_tma_load_2d(dst, &tm.x[t], kb * LR_BK, m0, full0 + 8 * s);
-                    lr_tma_load_2d(dst + LP_TILE, &tm.w1[t], kb * LR_BK, 0, full0 + 8 * s);
+        LrRing r;
+        for (int item = blockIdx.x; item < a.items && !failed; item += gridDim.x) {
+            const int t = item / a.tiles, m0 = item % a.tiles * LR_BM;
+            for (int kb = 0; kb < num_kb; ++kb, r.next(a.stages)) {
+                if (!lr_mbar_wait(empty0 + 8 * r.s, r.ph ^ 1u)) { failed = true; break; }
+                if (lr_elect()) {
+                    lr_mbar_expect_tx(full0 + 8 * r.s, (uint32_t)stage_bytes);
+                    const uint32_t dst = ring + (uint32_t)(r.s * stage_bytes);
+                    lr_tma_load_2d(dst, &tm.x[t], kb * LR_BK, m0, full0 + 8 * r.s);
+                    lr_tma_load_2d(dst + LP_TILE, &tm.w1[t], kb * LR_BK, 0, full0 + 8 * r.s);
                 }
+                __syncwarp();
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t idesc = lr_instr_desc(a.R);
-            int it = 0, n = 0;
-            for (int item = blockIdx.x; item < a.items && !failed; item += gridDim.x, ++n) {
-                const int b = n & 1;
-                if (!lr_mbar_wait(d1_empty + 8 * b, (((uint32_t)n >> 1) & 1u) ^ 1u)) { failed = true; break; }
+        const uint32_t idesc = lr_instr_desc(a.R);
+        const uint32_t a_lo = lr_desc_lo(ring), b_lo = lr_desc_lo(ring + LP_TILE), stage_lo = (uint32_t)stage_bytes >> 4;
+        LrRing r;
+        int n = 0;
+        for (int item = blockIdx.x; item < a.items && !failed; item += gridDim.x, ++n) {
+            const int b = n & 1;
+            if (!lr_mbar_wait(d1_empty + 8 * b, (((uint32_t)n >> 1) & 1u) ^ 1u)) { failed = true; break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            for (int kb = 0; kb < num_kb; ++kb, r.next(a.stages)) {
+                if (!lr_mbar_wait(full0 + 8 * r.s, r.ph)) { failed = true; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                for (int kb = 0; kb < num_kb; ++kb, ++it) {
-                    const int s = it % a.stages;
-                    if (!lr_mbar_wait(full0 + 8 * s, (uint32_t)(it / a.stages) & 1u)) { failed = true; break; }
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t sa = ring + (uint32_t)(s * stage_bytes), sb = sa + LP_TILE;
+                if (lr_elect()) {
+                    const uint32_t off = (uint32_t)r.s * stage_lo;
 #pragma unroll
                     for (int k = 0; k < LR_BK / 16; ++k)
-                        lr_mma(d1_base + (uint32_t)(64 * b), lr_smem_desc(sa + 32 * k), lr_smem_desc(sb + 32 * k), idesc, (kb | k) ? 1u : 0u);
-                    lr_commit(empty0 + 8 * s);
+                        lr_mma(d1_base + (uint32_t)(64 * b), lr_desc(a_lo + off + 2 * k), lr_desc(b_lo + off + 2 * k), idesc, (kb | k) ? 1u : 0u);
+                    lr_commit(empty0 + 8 * r.s);
                 }
-                lr_commit(d1_full + 8 * b);
+                __syncwarp();
             }
+            if (lr_elect()) lr_commit(d1_full + 8 * b);
+            __syncwarp();
         }
     } else if (warp == 2) {
-        if (lane == 0) {
-            int it = 0;
-            for (int item = blockIdx.x; item < a.items && !failed; item += gridDim.x) {
-                const int t = item / a.tiles;
-                for (int c = 0; c < chunks; ++c, ++it) {
-                    const int s = it % LP_BUF;
-                    if (!lr_mbar_wait(w2_empty + 8 * s, ((uint32_t)(it / LP_BUF) & 1u) ^ 1u)) { failed = true; break; }
-                    lr_mbar_expect_tx(w2_full + 8 * s, (uint32_t)LP_W2_TILE);
-                    lr_tma_load_2d(w2s + (uint32_t)(s * LP_W2_TILE), &tm.w2[t], 0, c * LP_CHUNK, w2_full + 8 * s);
+        LrRing r;
+        for (int item = blockIdx.x; item < a.items && !failed; item += gridDim.x) {
+            const int t = item / a.tiles;
+            for (int c = 0; c < chunks; ++c, r.next(LP_BUF)) {
+                if (!lr_mbar_wait(w2_empty + 8 * r.s, r.ph ^ 1u)) { failed = true; break; }
+                if (lr_elect()) {
+                    lr_mbar_expect_tx(w2_full + 8 * r.s, (uint32_t)LP_W2_TILE);
+                    lr_tma_load_2d(w2s + (uint32_t)(r.s * LP_W2_TILE), &tm.w2[t], 0, c * LP_CHUNK, w2_full + 8 * r.s);
                 }
+                __syncwarp();
             }
         }
     } else if (warp == 3) {
-        if (lane == 0) {
-            const uint32_t idesc = lr_instr_desc(LP_CHUNK);
-            int it = 0, n = 0;
-            for (int item = blockIdx.x; item < a.items && !failed; item += gridDim.x, ++n) {
-                const int b = n & 1;
-                if (!lr_mbar_wait(lat_full + 8 * b, ((uint32_t)n >> 1) & 1u)) { failed = true; break; }
-                for (int c = 0; c < chunks; ++c, ++it) {
-                    const int s = it % LP_BUF;
-                    const uint32_t ph = (uint32_t)(it / LP_BUF) & 1u;
-                    if (!lr_mbar_wait(w2_full + 8 * s, ph) || !lr_mbar_wait(d2_empty + 8 * s, ph ^ 1u)) { failed = true; break; }
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    for (int k = 0; k < a.R / 16; ++k)
-                        lr_mma(d2_base + (uint32_t)(64 * s), lr_smem_desc(lat + (uint32_t)(b * LP_TILE + 32 * k)),
-                               lr_smem_desc(w2s + (uint32_t)(s * LP_W2_TILE + 32 * k)), idesc, k ? 1u : 0u);
-                    lr_commit(d2_full + 8 * s);
-                    lr_commit(w2_empty + 8 * s);
+        const uint32_t idesc = lr_instr_desc(LP_CHUNK);
+        const uint32_t a_lo = lr_desc_lo(lat), b_lo = lr_desc_lo(w2s);
+        const int steps = a.R / 16;
+        LrRing r;
+        int n = 0;
+        for (int item = blockIdx.x; item < a.items && !failed; item += gridDim.x, ++n) {
+            const int b = n & 1;
+            if (!lr_mbar_wait(lat_full + 8 * b, ((uint32_t)n >> 1) & 1u)) { failed = true; break; }
+            for (int c = 0; c < chunks; ++c, r.next(LP_BUF)) {
+                if (!lr_mbar_wait(w2_full + 8 * r.s, r.ph) || !lr_mbar_wait(d2_empty + 8 * r.s, r.ph ^ 1u)) { failed = true; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (lr_elect()) {
+                    const uint32_t alo = a_lo + (uint32_t)b * (LP_TILE >> 4), blo = b_lo + (uint32_t)r.s * (LP_W2_TILE >> 4);
+#pragma unroll
+                    for (int k = 0; k < LR_BK / 16; ++k)
+                        if (k < steps) lr_mma(d2_base + (uint32_t)(64 * r.s), lr_desc(alo + 2 * k), lr_desc(blo + 2 * k), idesc, k ? 1u : 0u);
+                    lr_commit(d2_full + 8 * r.s);
+                    lr_commit(w2_empty + 8 * r.s);
                 }
-                lr_commit(lat_empty + 8 * b);            // the latent has been read for the last time
+                __syncwarp();
             }
+            if (lr_elect()) lr_commit(lat_empty + 8 * b);     // the latent has been read for the last time
+            __syncwarp();
         }
     } else {
         const int group = (warp - 4) >> 2, lg = warp & 3;
