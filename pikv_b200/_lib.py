@@ -1,8 +1,9 @@
 """ctypes binding of libpikv_b200.so (the C ABI declared in include/pikv_b200.h).
 
-The library is loaded lazily by `lib()`.  There is no fallback: if the shared
-object is missing or does not load, `lib()` raises and every operator of this
-package fails with that error.
+The library is loaded lazily by `lib()`, the native host module that marshals
+the operators' tensors for it (csrc/host/host.cpp) by `host()`.  There is no
+fallback: if a shared object is missing or does not load, they raise and every
+operator of this package fails with that error.
 """
 from __future__ import annotations
 
@@ -216,6 +217,22 @@ def lib() -> C.CDLL:
         raise PikvError(f"libpikv_b200.so has ABI {got}, this package expects {ABI_VERSION}")
     _LIB = handle
     return _LIB
+
+
+_HOST = None
+
+
+def host():
+    """The native host module: each operator's checks, output allocation and C ABI call in one call."""
+    global _HOST
+    if _HOST is None:
+        lib()
+        try:
+            from . import _host
+        except ImportError as e:
+            raise PikvError(f"pikv_b200/_host.so: {e}: build it with `python -m pikv_b200.build` (there is no fallback)") from e
+        _HOST = _host
+    return _HOST
 
 
 def check(rc: int, what: str) -> None:

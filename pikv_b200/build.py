@@ -1,4 +1,5 @@
-"""Compile the CUDA sources under csrc/ into pikv_b200/libpikv_b200.so for sm_100a.
+"""Compile the CUDA sources under csrc/ into pikv_b200/libpikv_b200.so for sm_100a, and the native host module
+csrc/host/host.cpp into pikv_b200/_host.so.
 
     python -m pikv_b200.build [--force] [--verbose]
 
@@ -12,12 +13,14 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(CSRC, "build")
 LIB = os.path.join(HERE, "libpikv_b200.so")
+HOST = os.path.join(HERE, "_host.so")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
 # no -use_fast_math: bit-exact codes need IEEE division and rint
@@ -75,7 +78,28 @@ def build(force: bool = False, verbose: bool = False, ptxas_v: bool = False) -> 
         res = subprocess.run(cmd, capture_output=True, text=True)
         if res.returncode != 0:
             raise RuntimeError(f"link failed:\n{res.stdout}\n{res.stderr}")
+    _build_host(force)
     return LIB
+
+
+def _build_host(force: bool) -> str:
+    """The Python extension that marshals tensors for the library (needs torch's and Python's headers, no GPU)."""
+    src = os.path.join(CSRC, "host", "host.cpp")
+    newest = max(os.path.getmtime(f) for f in (src, os.path.join(INCLUDE, "pikv_b200.h")))
+    if not force and os.path.exists(HOST) and os.path.getmtime(HOST) >= newest:
+        return HOST
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(nvcc()))
+    inc = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+           sysconfig.get_paths()["include"], os.path.join(cuda, "include"), INCLUDE]
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *(f"-I{d}" for d in inc), src, "-o", HOST, "-L" + os.path.join(root, "lib"), "-ltorch", "-ltorch_cpu", "-lc10",
+           "-lc10_cuda", "-ltorch_python", "-L" + HERE, "-l:libpikv_b200.so", "-Wl,-rpath,$ORIGIN"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"g++ failed for {src}:\n{res.stdout}\n{res.stderr}")
+    return HOST
 
 
 if __name__ == "__main__":

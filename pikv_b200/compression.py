@@ -37,9 +37,8 @@ def _linear(layer: nn.Linear, x: torch.Tensor, relu: bool) -> torch.Tensor:
     """One Linear (+ReLU): tcgen05 kernel for bf16 inputs whose shapes fit, cuBLAS otherwise."""
     K, N = layer.in_features, layer.out_features
     if x.dtype == torch.bfloat16 and x.is_cuda and K % 16 == 0 and N % 16 == 0 and (N <= 256 or N % 256 == 0):
-        lead = x.shape[:-1]
-        y = ops.lowrank_project(x.reshape(-1, K), layer.weight.detach().to(torch.bfloat16), layer.bias, relu=relu)
-        return y.view(*lead, N)
+        p = layer._parameters
+        return ops.lowrank_project(x, p["weight"].to(torch.bfloat16), p["bias"], relu=relu)
     y = F.linear(x, layer.weight.to(x.dtype), None if layer.bias is None else layer.bias.to(x.dtype))
     return F.relu(y) if relu else y
 
@@ -159,11 +158,10 @@ class SVDCompressor(BaseCompressor):
         H, R = self.hidden_size, self.rank
         if (keys.shape == values.shape and keys.dtype == values.dtype == torch.bfloat16 and keys.is_cuda and R % 16 == 0 and R <= 64
                 and H % 16 == 0 and H <= 4096 and keys.numel() >= self.PAIR_ROWS * H):
-            down, up = (self.key_projector, self.value_projector), (self.key_reconstructor, self.value_reconstructor)
-            rk, rv = ops.lowrank_pair((keys.reshape(-1, H), values.reshape(-1, H)),
-                                      [m.weight.detach().to(torch.bfloat16) for m in down], [m.bias.detach() for m in down],
-                                      [m.weight.detach().to(torch.bfloat16) for m in up], [m.bias.detach() for m in up])
-            return rk.view(keys.shape), rv.view(values.shape)
+            m = self._modules
+            down, up = ([m[f"{which}_{part}"]._parameters for which in ("key", "value")] for part in ("projector", "reconstructor"))
+            return ops.lowrank_pair((keys, values), [p["weight"] for p in down], [p["bias"] for p in down],
+                                    [p["weight"] for p in up], [p["bias"] for p in up])
         return (self.reconstruct(self.project(keys, "key"), "key"),
                 self.reconstruct(self.project(values, "value"), "value"))
 
@@ -211,17 +209,16 @@ class QuantizedCompressor(BaseCompressor):
         return torch.stack([self.scale.reshape(()), self.zero_point.reshape(())]).float().repeat(groups, 1).contiguous()
 
     def forward(self, keys: torch.Tensor, values: torch.Tensor, importance: Optional[torch.Tensor] = None):
-        shape = keys.shape
-        kf = keys.reshape(-1, shape[-1])
-        vf = values.reshape(-1, shape[-1])
-        groups = (shape[-1] + self.group_size - 1) // self.group_size
-        params_in = None if self.dynamic_quantization else self._static_params(kf, groups)
+        groups = (keys.shape[-1] + self.group_size - 1) // self.group_size
+        params_in = None
+        if not self.dynamic_quantization:
+            params_in = self._static_params(keys.reshape(-1, keys.shape[-1]), groups)
         with torch.no_grad():
             qmin, qmax = self._qrange()
             dk, dv, self.quantization_error = ops.quant_block_pair(
-                kf, vf, self.group_size, qmin, qmax, self.symmetric, params_in=params_in,
+                keys, values, self.group_size, qmin, qmax, self.symmetric, params_in=params_in,
                 sample_count=self.sample_count, count_add=2.0 * groups)
-        return dk.view(shape), dv.view(shape)
+        return dk, dv.view(keys.shape)
 
     def get_compression_stats(self) -> Dict[str, float]:
         stats = super().get_compression_stats()

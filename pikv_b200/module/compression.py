@@ -147,11 +147,11 @@ class QuantizedCompressor(BaseCompressor):
 
     def forward(self, keys: torch.Tensor, values: torch.Tensor, importance: Optional[torch.Tensor] = None):
         shape = keys.shape
-        kf, vf = keys.reshape(-1, shape[-1]), values.reshape(-1, shape[-1])
+        kf = keys.reshape(-1, shape[-1])
         groups = (shape[-1] + self.group_size - 1) // self.group_size
         qmin, qmax = self._qrange()
         params_in = None if self.dynamic else self._static_params(kf[:, : self.group_size], groups)
-        dk, dv, self.quantization_error = ops.quant_block_pair(kf, vf, self.group_size, qmin, qmax, self.symmetric,
+        dk, dv, self.quantization_error = ops.quant_block_pair(keys, values, self.group_size, qmin, qmax, self.symmetric,
                                                                params_in=params_in)
         original = keys.numel() + values.numel()
         self._update_stats(original, int(original * self.bits / 32))

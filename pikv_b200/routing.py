@@ -96,13 +96,18 @@ class BaseRouter(nn.Module):
     def _hidden(self, mlp: nn.Sequential, x2d: torch.Tensor) -> torch.Tensor:
         return F.relu(mlp[0](x2d))
 
-    def _fused_net(self, mlp: nn.Sequential, x2d: torch.Tensor) -> bool:
-        return x2d.dtype == torch.bfloat16 and self.num_experts <= 32 and x2d.shape[1] % 8 == 0 and mlp[0].out_features % 8 == 0
+    def _fused_net(self, mlp: nn.Sequential, x: torch.Tensor) -> bool:
+        return (x.dtype == torch.bfloat16 and self.num_experts <= 32 and x.shape[-1] % 8 == 0
+                and mlp._modules["0"].out_features % 8 == 0)
 
     def _net_weights(self, mlp: nn.Sequential):
-        w = lambda layer: layer.weight.detach().to(torch.bfloat16)              # noqa: E731
-        b = lambda layer: None if layer.bias is None else layer.bias.detach()   # noqa: E731
-        return w(mlp[0]), b(mlp[0]), w(mlp[2]), b(mlp[2])
+        """w1, b1, w2, b2, the weights in bf16."""
+        out = []
+        for name in ("0", "2"):
+            p = mlp._modules[name]._parameters
+            w = p["weight"]
+            out += [w if w.dtype == torch.bfloat16 else w.detach().to(torch.bfloat16), p["bias"]]
+        return out
 
     def _gate_net(self, mlp: nn.Sequential, x2d: torch.Tensor, **kw) -> ops.GateResult:
         """Gate net + tail.  bf16 inputs: both layers and the tail on the tensor-core kernels (the hidden activations
@@ -118,18 +123,16 @@ class BaseRouter(nn.Module):
     def _route(self, hidden_states: torch.Tensor, expert_mask: Optional[torch.Tensor], balance: Optional[str] = None,
                coefficient: float = 0.0):
         batch_size, seq_len, hidden_size = hidden_states.shape
-        x2d = hidden_states.reshape(-1, hidden_size)
         capacity = self._compute_capacity(batch_size, seq_len)
         rows = max(capacity, 1)
-        if self.expert_backend == "fairscale" and self._fused_net(self.router, x2d):
+        net = self.router
+        if self.expert_backend == "fairscale" and self._fused_net(net, hidden_states):
             g, (dispatch, combine, aux_loss) = ops.gate_mlp_dense(
-                x2d, *self._net_weights(self.router), rows, self.position_mode, balance, coefficient, top_k=self.top_k,
+                hidden_states, *self._net_weights(net), rows, self.position_mode, balance, coefficient, top_k=self.top_k,
                 expert_mask=expert_mask, mask_mode=self.mask_mode, renorm_eps=self.renorm_eps, capacity=capacity)
             self.last_gate = g
-            shape = (batch_size, seq_len, self.num_experts, rows)
-            dispatch, combine = dispatch.view(shape), combine.view(shape)
         else:
-            g = self._gate_net(self.router, x2d, expert_mask=expert_mask, capacity=capacity)
+            g = self._gate_net(net, hidden_states.reshape(-1, hidden_size), expert_mask=expert_mask, capacity=capacity)
             dispatch, combine, aux_loss = self._dense(g, batch_size, seq_len, rows, balance, coefficient)
         return dispatch, combine, g.probs.view(batch_size, seq_len, self.num_experts), aux_loss
 
