@@ -176,7 +176,11 @@ __device__ __forceinline__ void kv_append_body(const AppendDev& a) {
     AppendRoute<TOPK> r0, r1, r2;
     int pg0[TOPK], pg1[TOPK];
     typename GQ::Raw k0, v0, k1, v1;
-    // prologue: the loads that need nothing from the gate go out first
+    // a decode step's few rows: whatever follows may become resident at once (not behind a grid that fills the GPU: its
+    // waiting CTAs would hold the registers that kernels of other streams need)
+    if (gridDim.x <= 148) dependency_release();
+    // MODE 2: the K / V loads need nothing from the gate and go out before the wait
+    if (MODE != 2) dependency_wait();
     if (any) append_stage_kv<TIn, BITS, SYM>(a, pair, total, sub, k0, v0);
     // MODE 2 is launched as a programmatic dependent of the gate kernel: its CTAs may become resident, and their
     // first K/V loads go out, while the gate is still running; everything the gate writes is read after this wait
@@ -442,10 +446,10 @@ static int launch_append(const AppendDev& a, int bits, int symmetric, cudaStream
     const int grid = (int)(want < cap_ctas ? want : cap_ctas);
 #define PIKV_APPEND_LAUNCH(BITS, SYM)                                                                   \
     do {                                                                                                \
-        if (a.top_k <= 1) kv_append_quant_kernel<TIn, BITS, SYM, 1, 0><<<grid, APPEND_THREADS, 0, st>>>(a);      \
-        else if (a.top_k <= 2) kv_append_quant_kernel<TIn, BITS, SYM, 2, 0><<<grid, APPEND_THREADS, 0, st>>>(a); \
-        else if (a.top_k <= 4) kv_append_quant_kernel<TIn, BITS, SYM, 4, 0><<<grid, APPEND_THREADS, 0, st>>>(a); \
-        else kv_append_quant_kernel<TIn, BITS, SYM, 8, 0><<<grid, APPEND_THREADS, 0, st>>>(a);                   \
+        if (a.top_k <= 1) launch_dependent(kv_append_quant_kernel<TIn, BITS, SYM, 1, 0>, grid, APPEND_THREADS, 0, st, a);      \
+        else if (a.top_k <= 2) launch_dependent(kv_append_quant_kernel<TIn, BITS, SYM, 2, 0>, grid, APPEND_THREADS, 0, st, a); \
+        else if (a.top_k <= 4) launch_dependent(kv_append_quant_kernel<TIn, BITS, SYM, 4, 0>, grid, APPEND_THREADS, 0, st, a); \
+        else launch_dependent(kv_append_quant_kernel<TIn, BITS, SYM, 8, 0>, grid, APPEND_THREADS, 0, st, a);                   \
     } while (0)
     if (bits == 8 && symmetric) PIKV_APPEND_LAUNCH(8, true);
     else if (bits == 8) PIKV_APPEND_LAUNCH(8, false);
@@ -504,10 +508,10 @@ extern "C" int pikv_kv_append_rope(const pikv_append_params* p, const float* rop
     const long long lanes = (long long)a.T * a.n_kv * 8;
     long long want = ceil_div64(lanes, APPEND_THREADS), cap_ctas = (long long)sm_count() * 3;
     const int grid = (int)(want < cap_ctas ? want : cap_ctas);
-    if (a.top_k <= 1) kv_append_quant_kernel<__nv_bfloat16, 8, true, 1, 4><<<grid, APPEND_THREADS, 0, st>>>(a);
-    else if (a.top_k <= 2) kv_append_quant_kernel<__nv_bfloat16, 8, true, 2, 4><<<grid, APPEND_THREADS, 0, st>>>(a);
-    else if (a.top_k <= 4) kv_append_quant_kernel<__nv_bfloat16, 8, true, 4, 4><<<grid, APPEND_THREADS, 0, st>>>(a);
-    else kv_append_quant_kernel<__nv_bfloat16, 8, true, 8, 4><<<grid, APPEND_THREADS, 0, st>>>(a);
+    if (a.top_k <= 1) launch_dependent(kv_append_quant_kernel<__nv_bfloat16, 8, true, 1, 4>, grid, APPEND_THREADS, 0, st, a);
+    else if (a.top_k <= 2) launch_dependent(kv_append_quant_kernel<__nv_bfloat16, 8, true, 2, 4>, grid, APPEND_THREADS, 0, st, a);
+    else if (a.top_k <= 4) launch_dependent(kv_append_quant_kernel<__nv_bfloat16, 8, true, 4, 4>, grid, APPEND_THREADS, 0, st, a);
+    else launch_dependent(kv_append_quant_kernel<__nv_bfloat16, 8, true, 8, 4>, grid, APPEND_THREADS, 0, st, a);
     count_launch(1);
     return check_launch("kv_append_quant_kernel (rotary)");
 }

@@ -41,11 +41,34 @@ static inline bool allow_smem(int bytes = 227 * 1024) {
     return true;
 }
 
+// Launches a kernel that may become resident before the previous kernel of the stream has finished: it executes
+// griddepcontrol.wait before it touches memory, so only its start-up overlaps the predecessor's end (the gap between two
+// dependent launches is 2 to 2.5 us without it).
+template <typename... KArgs, typename... Args>
+static inline void launch_dependent(void (*kern)(KArgs...), dim3 grid, int block, size_t smem, cudaStream_t st, const Args&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    (void)cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);      // reported by check_launch
+}
+
 static inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 static inline int64_t ceil_div64(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 // ---- device helpers ----------------------------------------------------------
 #ifdef __CUDACC__
+
+// see launch_dependent
+__device__ __forceinline__ void dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// the next kernel of the stream may become resident from here on (if it was launched with launch_dependent)
+__device__ __forceinline__ void dependency_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 __device__ __forceinline__ float bf16_bits_to_f32(uint32_t lo16) { return __uint_as_float(lo16 << 16); }
 

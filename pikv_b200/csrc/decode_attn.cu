@@ -2,8 +2,8 @@
 // dequantised in registers.
 //
 // The pages of all requests form one list (per KV head), cut into blocks of equal length whatever the
-// lengths of the requests; a work item is (block, head).  The grid is persistent (three CTAs of four warps per
-// SM) and every WARP is a worker that claims items from a counter until none is left: fast and slow SMs even
+// lengths of the requests; a work item is (block, head).  The grid is persistent (three or four CTAs of four warps
+// per SM) and every WARP is a worker that claims items from a counter until none is left: fast and slow SMs even
 // out, there is no wave quantisation and no tail, the eight heads of a block are claimed one after the other
 // (so the heads of a page are read at about the same time), and a block may start and end in the middle of a
 // request.  A worker streams its pages (16 tokens x 128 channels of K and of V plus their scales and, for 4
@@ -25,13 +25,16 @@ namespace pikv {
 
 constexpr int DA_WARPS = 4;
 constexpr int DA_THREADS = DA_WARPS * 32;
-constexpr int DA_CTAS_PER_SM = 3;
+constexpr int da_ctas_per_sm(int bits) { return bits == 8 ? 3 : 4; }   // what the rings leave room for
 constexpr int DA_MAX_GROUP = 8;
 constexpr int DA_MIN_BLOCK = 16;                        // pages per block, at least (more than a ring holds)
 constexpr int DA_ITEMS_PER_WORKER = 8;                  // blocks aimed at per worker of a head, at most
 constexpr int DA_ITEM_PAGES = 48;                       // ... while an item keeps this many pages
 constexpr int DA_MAX_REQ = 12000;                       // requests per call: their page prefix is scanned in shared memory
 constexpr int DA_PLAN_THREADS = 1024;
+constexpr int DA_DIRECT_PAGES = 64;                     // direct plan: at most this many pages per worker ...
+constexpr int DA_DIRECT_REQ = 512;                      // ... and this many requests
+constexpr int DA_DIRECT_BLOCK = 4;                      // pages per block of a direct plan, at least
 constexpr int DA_FOLD_STEPS = 8;                        // softmax steps between two folds of the carried bias term
 constexpr unsigned DA_WAIT_LIMIT = 1u << 24;            // mbarrier polls before giving up
 
@@ -56,6 +59,7 @@ struct DecodeDev {
     __half* probs16;  // [B][n_q][probs_stride] exp2(score - step maximum) as f16, or null
     float* step_max;  // [B][n_q][step_stride] the step maximum (log2 domain) of every 16-position page
     int probs_stride, step_stride;
+    int probs_pairs;  // rows of probs16 start at 4-byte boundaries
     int* head;        // workspace header: [0] item counter, [1] pages per block, [2] blocks (written by the plan kernel)
     int* prefix;      // [B+1] pages of the requests before each request
     int2* blk_start;  // [max_blocks] (request, page inside it) at which every block starts
@@ -157,6 +161,9 @@ __device__ __forceinline__ uint32_t nib_pair(uint32_t w) {
 template <uint32_t SEL>
 __device__ __forceinline__ uint32_t bytes_to_h2_biased(uint32_t w) { return __byte_perm(w, 0x64646464u, SEL); }
 
+// What a page costs its warp beside the arithmetic: its page id (read 32 at a time), and the rescale of O (skipped while
+// no maximum moves).  64 streams x 32768, 8 bit: 749 -> 706 us = 6.2 TB/s; 4 bit, bound by instructions (four CTAs per SM
+// hide more of their latency than three): 914 -> 745 us.
 // The legacy mma.sync path is what bounds this kernel on this GPU (one m16n8k16 holds a sub-core's tensor
 // pipe for about 32 cycles), so the shapes are chosen to waste as few of its rows as possible:
 //   S^T[pos, head] = Kcode[pos, :] . Q[head, :]    A = the page's 16 positions (all rows used), B = Q^T:
@@ -199,6 +206,7 @@ __global__ void __launch_bounds__(DA_PLAN_THREADS) decode_plan_kernel(DecodeDev 
     const int R = d.B;
     const int max_len = d.max_pages * PIKV_PAGE_TOKENS;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");      // the attention kernel may be scheduled
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     if constexpr (SHARD) {
         __shared__ int ok_s;
         if (tid == 0) ok_s = 1;
@@ -287,8 +295,13 @@ __global__ void __launch_bounds__(DA_PLAN_THREADS) decode_plan_kernel(DecodeDev 
 // (the f16 path spends half its softmax on padding heads).  The second product stays in f16 (P' is not an
 // integer); the rescale factors travel from the thread that owns a head's statistics to the two threads that
 // own its accumulators by two shuffles per step.
-template <int BITS, bool GS>
-__global__ void __launch_bounds__(DA_THREADS, DA_CTAS_PER_SM) decode_attn_kernel(DecodeDev d) {
+//
+// DIRECT (short lists, see decode_attn_run): no plan kernel.  Every CTA scans the request lengths itself, the list is cut
+// into at most one block per worker of a head, down to DA_DIRECT_BLOCK pages, and worker w takes item w; CTA 0 leaves what
+// the merge kernel needs.  One stream of 1500 tokens: 48 items of 16 pages behind a 4 us plan kernel took 24 us a step; 192
+// items of 4 pages take 10.  24 streams of 3300 tokens, 4 bit: 69 -> 41 us.
+template <int BITS, bool GS, bool DIRECT>
+__global__ void __launch_bounds__(DA_THREADS, da_ctas_per_sm(BITS)) decode_attn_kernel(DecodeDev d) {
     using GEO = DAGeom<BITS>;
     constexpr int STAGES = GEO::STAGES, STAGE_BYTES = GEO::STAGE, PAGE_BYTES = GEO::PAGE, ROW = GEO::ROW;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -315,7 +328,53 @@ __global__ void __launch_bounds__(DA_THREADS, DA_CTAS_PER_SM) decode_attn_kernel
     for (int i2 = lane; i2 < DA_PBUF_BYTES / 4; i2 += 32) reinterpret_cast<uint32_t*>(pbuf)[i2] = 0u;   // rows of absent heads stay zero
     __syncwarp();
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int blk_pages = __ldg(d.head + 1), nblocks = __ldg(d.head + 2), P = __ldg(d.prefix + R);
+    int* pre = reinterpret_cast<int*>(smem + da_smem_bytes<BITS>());      // DIRECT: [R + 1] pages before every request
+    int blk_pages, nblocks, P;
+    if constexpr (DIRECT) {
+        __shared__ int wtot[DA_WARPS];
+        const int per = (R + DA_THREADS - 1) / DA_THREADS, lo = tid * per, hi = min(R, lo + per);
+        int sum = 0;
+        for (int q = lo; q < hi; ++q) {
+            const int seq = d.seq_ids ? __ldg(d.seq_ids + q) : q;
+            const bool ok = seq >= 0 && seq < d.num_seqs;
+            if (!ok && blockIdx.x == 0 && d.status) atomicOr(d.status, PIKV_ST_BAD_SEQ);
+            const int len = ok ? max(0, min(__ldg(d.seq_len + q), max_len)) : 0;
+            const int pages = (len + PIKV_PAGE_TOKENS - 1) / PIKV_PAGE_TOKENS;
+            pre[q + 1] = pages;
+            sum += pages;
+        }
+        int inc = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int n = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += n;
+        }
+        if (lane == 31) wtot[warp] = inc;
+        if (tid == 0) pre[0] = 0;
+        __syncthreads();
+        int run = inc - sum;
+        for (int w = 0; w < warp; ++w) run += wtot[w];
+        for (int q = lo; q < hi; ++q) {
+            run += pre[q + 1];
+            pre[q + 1] = run;
+        }
+        __syncthreads();
+        P = pre[R];
+        const int most = max(1, min(d.max_blocks, d.workers / n_kv));
+        blk_pages = max(DA_DIRECT_BLOCK, (P + most - 1) / most);
+        nblocks = (P + blk_pages - 1) / blk_pages;
+        if (blockIdx.x == 0) {
+            if (tid == 0) {
+                d.head[1] = blk_pages;
+                d.head[2] = nblocks;
+            }
+            for (int q = tid; q <= R; q += DA_THREADS) d.prefix[q] = pre[q];
+        }
+    } else {
+        blk_pages = __ldg(d.head + 1);
+        nblocks = __ldg(d.head + 2);
+        P = __ldg(d.prefix + R);
+    }
     const int nitems = nblocks * n_kv;
 
     auto request = [&](int rq, int& len, int& row) {          // clamped length and page-table row of a request
@@ -325,7 +384,13 @@ __global__ void __launch_bounds__(DA_THREADS, DA_CTAS_PER_SM) decode_attn_kernel
         row = ok ? seq : -1;
     };
     // the next item of the list (warp-uniform); the claims of a block's heads go to consecutive callers
+    bool claimed = false;
     auto claim = [&]() {
+        if constexpr (DIRECT) {              // one item at most, consecutive items on different SMs
+            const int id = claimed ? nitems : warp * (int)gridDim.x + (int)blockIdx.x;
+            claimed = true;
+            return id;
+        }
         int id = 0;
         if (lane == 0) id = atomicAdd(d.head, 1);
         return __shfl_sync(0xffffffffu, id, 0);
@@ -333,9 +398,20 @@ __global__ void __launch_bounds__(DA_THREADS, DA_CTAS_PER_SM) decode_attn_kernel
     auto load_item = [&](int id, DAItem& it) {
         it.blk = id / n_kv;
         it.h = id % n_kv;
-        const int2 st = __ldg(d.blk_start + it.blk);
-        it.cur.r = st.x;
-        it.cur.p = st.y;
+        if constexpr (DIRECT) {
+            const int f = it.blk * blk_pages;
+            int lo = 0, hi = R - 1;                       // last request whose first page is at or before f
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (pre[mid] <= f) lo = mid; else hi = mid - 1;
+            }
+            it.cur.r = lo;
+            it.cur.p = f - pre[lo];
+        } else {
+            const int2 st = __ldg(d.blk_start + it.blk);
+            it.cur.r = st.x;
+            it.cur.p = st.y;
+        }
         request(it.cur.r, it.cur.len, it.cur.row);
         it.cur.pages = (it.cur.len + PIKV_PAGE_TOKENS - 1) / PIKV_PAGE_TOKENS;
         it.left = it.blk == nblocks - 1 ? P - it.blk * blk_pages : blk_pages;
@@ -353,9 +429,19 @@ __global__ void __launch_bounds__(DA_THREADS, DA_CTAS_PER_SM) decode_attn_kernel
             x.pages = (x.len + PIKV_PAGE_TOKENS - 1) / PIKV_PAGE_TOKENS;
         } while (x.pages == 0);
     };
-    auto issue = [&](const DACursor& x, int h, int i) {   // lane 0 only: load the page under the cursor into stage i % STAGES
+    // page ids of the issuing cursor, 32 at a time (lane l holds page pt_base + l of row pt_row): one at a time, every page
+    // held up its warp for a trip to L2
+    int pt_ids = -1, pt_row = -2, pt_base = 0;
+    auto page_id = [&](const DACursor& x) {
+        if (x.row != pt_row || x.p < pt_base || x.p >= pt_base + 32) {
+            pt_row = x.row;
+            pt_base = x.p;
+            pt_ids = x.row >= 0 && x.p + lane < d.max_pages ? __ldg(d.page_table + (size_t)x.row * d.max_pages + x.p + lane) : -1;
+        }
+        return __shfl_sync(0xffffffffu, pt_ids, x.p - pt_base);
+    };
+    auto issue = [&](int page, int h, int i) {   // lane 0 only: load the page into stage i % STAGES
         const int s = i % STAGES;
-        int page = x.row >= 0 ? __ldg(d.page_table + (size_t)x.row * d.max_pages + x.p) : -1;
         if (page < 0 || page >= d.num_pages) {
             if (d.status) atomicOr(d.status, PIKV_ST_BAD_PAGE);
             page = 0;
@@ -393,7 +479,8 @@ __global__ void __launch_bounds__(DA_THREADS, DA_CTAS_PER_SM) decode_attn_kernel
                 pend_id = next_id;
                 next_id = claim();
             }
-            if (lane == 0) issue(is.cur, is.h, issued);
+            const int page = page_id(is.cur);
+            if (lane == 0) issue(page, is.h, issued);
             advance(is.cur, 1);
             --is.left;
             ++issued;
@@ -496,7 +583,7 @@ __global__ void __launch_bounds__(DA_THREADS, DA_CTAS_PER_SM) decode_attn_kernel
     auto page_scores = [&](const unsigned char* st, float (&t)[4], float& vw_lo, float& vw_hi) {
         if constexpr (GS) {
             // integer path: t[0] / t[2] = head j at positions r / r+8 (t[1], t[3] unused)
-            int acc[4] = {0, 0, 0, 0};
+            int acc[4] = {0, 0, 0, 0}, acc2[4] = {0, 0, 0, 0};        // two chains: the sums are exact integers
             if (BITS == 8) {
                 const unsigned char* klo = st + r * 128;
                 const unsigned char* khi = st + (r + 8) * 128;
@@ -507,7 +594,7 @@ __global__ void __launch_bounds__(DA_THREADS, DA_CTAS_PER_SM) decode_attn_kernel
                 const uint32_t wl[8] = {la.x, la.y, la.z, la.w, lb.x, lb.y, lb.z, lb.w};
                 const uint32_t wh[8] = {ha.x, ha.y, ha.z, ha.w, hb.x, hb.y, hb.z, hb.w};
 #pragma unroll
-                for (int m = 0; m < 4; ++m) mma_s8(acc, wl[2 * m], wh[2 * m], wl[2 * m + 1], wh[2 * m + 1], qf[2 * m], qf[2 * m + 1]);
+                for (int m = 0; m < 4; ++m) mma_s8((m & 1) ? acc2 : acc, wl[2 * m], wh[2 * m], wl[2 * m + 1], wh[2 * m + 1], qf[2 * m], qf[2 * m + 1]);
             } else {
                 const unsigned char* klo = st + r * 64;
                 const unsigned char* khi = st + (r + 8) * 64;
@@ -517,13 +604,13 @@ __global__ void __launch_bounds__(DA_THREADS, DA_CTAS_PER_SM) decode_attn_kernel
                 const uint32_t wh[4] = {hq.x, hq.y, hq.z, hq.w};
 #pragma unroll
                 for (int m = 0; m < 4; ++m)
-                    mma_s8(acc, wl[m] & 0x0f0f0f0fu, wh[m] & 0x0f0f0f0fu, (wl[m] >> 4) & 0x0f0f0f0fu, (wh[m] >> 4) & 0x0f0f0f0fu,
+                    mma_s8((m & 1) ? acc2 : acc, wl[m] & 0x0f0f0f0fu, wh[m] & 0x0f0f0f0fu, (wl[m] >> 4) & 0x0f0f0f0fu, (wh[m] >> 4) & 0x0f0f0f0fu,
                            qf[2 * m], qf[2 * m + 1]);
             }
             const uint16_t* ksc = reinterpret_cast<const uint16_t*>(st + 2 * PAGE_BYTES);
             const float ks_lo = __uint_as_float((uint32_t)ksc[r] << 16), ks_hi = __uint_as_float((uint32_t)ksc[r + 8] << 16);
-            t[0] = (float)(acc[0] * 128 + acc[1]);
-            t[2] = (float)(acc[2] * 128 + acc[3]);
+            t[0] = (float)((acc[0] + acc2[0]) * 128 + (acc[1] + acc2[1]));
+            t[2] = (float)((acc[2] + acc2[2]) * 128 + (acc[3] + acc2[3]));
             if (BITS == 4) {
                 const float* kzp = reinterpret_cast<const float*>(st + 2 * PAGE_BYTES + 64);
                 const float* vzp = reinterpret_cast<const float*>(st + 2 * PAGE_BYTES + 128);
@@ -719,14 +806,24 @@ __global__ void __launch_bounds__(DA_THREADS, DA_CTAS_PER_SM) decode_attn_kernel
                 const float vs_lo = __uint_as_float((uint32_t)vsc[r] << 16), vs_hi = __uint_as_float((uint32_t)vsc[r + 8] << 16);
                 if constexpr (GS) {
                     const float p0 = exp2f(t[0] - mu0), p2 = exp2f(t[2] - mu0);
-                    if (d.probs16 && j < G) {
+                    if (d.probs16) {
                         // the H2O update needs exp(score - lse) summed over the heads of the group: lse is known only at
                         // the end, so the probabilities go out relative to this step's maximum (f16: uniform relative
                         // precision), with the maximum of every page beside them
                         const size_t hq = (size_t)c.cur.r * d.n_q + (size_t)c.h * G + j;
-                        if (pos0 + r < c.cur.len && pos0 + r < d.probs_stride) d.probs16[hq * d.probs_stride + pos0 + r] = __float2half_rn(p0);
-                        if (pos0 + r + 8 < c.cur.len && pos0 + r + 8 < d.probs_stride) d.probs16[hq * d.probs_stride + pos0 + r + 8] = __float2half_rn(p2);
-                        if (r == 0 && (pos0 >> 4) < d.step_stride) d.step_max[hq * d.step_stride + (pos0 >> 4)] = mu0;
+                        if (d.probs_pairs) {
+                            // the lanes of a head trade their positions r and r + 8 for 2r and 2r + 1: the page's 16
+                            // probabilities leave as one 32-byte sector (a pair past the end is written as zero)
+                            const uint32_t own = pack_h2(p0, p2);
+                            const uint32_t wa = __shfl_sync(0xffffffffu, own, ((8 * r) & 31) | j), wb = __shfl_sync(0xffffffffu, own, ((8 * r + 4) & 31) | j);
+                            const int ps = pos0 + 2 * r;
+                            if (j < G && ps < c.cur.len && ps + 1 < d.probs_stride)
+                                *reinterpret_cast<uint32_t*>(d.probs16 + hq * d.probs_stride + ps) = __byte_perm(wa, wb, r < 4 ? 0x5410 : 0x7632);
+                        } else if (j < G) {
+                            if (pos0 + r < c.cur.len && pos0 + r < d.probs_stride) d.probs16[hq * d.probs_stride + pos0 + r] = __float2half_rn(p0);
+                            if (pos0 + r + 8 < c.cur.len && pos0 + r + 8 < d.probs_stride) d.probs16[hq * d.probs_stride + pos0 + r + 8] = __float2half_rn(p2);
+                        }
+                        if (j < G && r == 0 && (pos0 >> 4) < d.step_stride) d.step_max[hq * d.step_stride + (pos0 >> 4)] = mu0;
                     }
                     la += p0 + p2;
                     const __half h0 = __float2half_rn(p0 * vs_lo), h2 = __float2half_rn(p2 * vs_hi);
@@ -770,16 +867,19 @@ __global__ void __launch_bounds__(DA_THREADS, DA_CTAS_PER_SM) decode_attn_kernel
             l1 = l1 * al1 + lb;
             corr0 = corr0 * al0 + ca;
             corr1 = corr1 * al1 + cb;
-            if constexpr (GS) {
-                // the accumulators of heads 2j, 2j+1 live here, their rescale factors in the lanes with j' = head
-                const float mine = al0;
-                al0 = __shfl_sync(0xffffffffu, mine, (lane & ~3) | ((2 * j) & 3));
-                al1 = __shfl_sync(0xffffffffu, mine, (lane & ~3) | ((2 * j + 1) & 3));
-            }
-            // rescale O: this thread's columns are query heads 2j and 2j+1
+            // rescale O when a maximum has moved (seldom, after the first few pages): this thread's columns are query heads
+            // 2j and 2j+1
+            if (__any_sync(0xffffffffu, al0 != 1.f || al1 != 1.f)) {
+                if constexpr (GS) {
+                    // the accumulators of heads 2j, 2j+1 live here, their rescale factors in the lanes with j' = head
+                    const float mine = al0;
+                    al0 = __shfl_sync(0xffffffffu, mine, (lane & ~3) | ((2 * j) & 3));
+                    al1 = __shfl_sync(0xffffffffu, mine, (lane & ~3) | ((2 * j + 1) & 3));
+                }
 #pragma unroll
-            for (int m = 0; m < 8; ++m) {
-                o[m][0] *= al0; o[m][1] *= al1; o[m][2] *= al0; o[m][3] *= al1;
+                for (int m = 0; m < 8; ++m) {
+                    o[m][0] *= al0; o[m][1] *= al1; o[m][2] *= al0; o[m][3] *= al1;
+                }
             }
             __syncwarp();
             page_pv(stA, *reinterpret_cast<const uint32_t*>(pbuf + r * 32 + 2 * j),
@@ -854,22 +954,18 @@ __device__ __forceinline__ void da_merge_blocks(const DecodeDev& d, int rq, int 
         M = mm;
         const float w_l = (ml.x == -INFINITY) ? 0.f : exp2f(ml.x - M), l_l = ml.y;
         int i = 0;
-        for (; i + 4 <= cnt; i += 4) {
-            float4 o4[4];
+        for (; i < cnt; i += 8) {
+            float4 o4[8];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) o4[u] = reinterpret_cast<const float4*>(d.part_o + slot(g0 + i + u) * 128)[lane];
+            for (int u = 0; u < 8; ++u)
+                if (i + u < cnt) o4[u] = reinterpret_cast<const float4*>(d.part_o + slot(g0 + i + u) * 128)[lane];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
+            for (int u = 0; u < 8; ++u) {
+                if (i + u >= cnt) break;
                 const float w = __shfl_sync(0xffffffffu, w_l, i + u);
                 acc.x += o4[u].x * w; acc.y += o4[u].y * w; acc.z += o4[u].z * w; acc.w += o4[u].w * w;
                 l += __shfl_sync(0xffffffffu, l_l, i + u) * w;
             }
-        }
-        for (; i < cnt; ++i) {
-            const float4 o = reinterpret_cast<const float4*>(d.part_o + slot(g0 + i) * 128)[lane];
-            const float w = __shfl_sync(0xffffffffu, w_l, i);
-            acc.x += o.x * w; acc.y += o.y * w; acc.z += o.z * w; acc.w += o.w * w;
-            l += __shfl_sync(0xffffffffu, l_l, i) * w;
         }
         return;
     }
@@ -897,30 +993,60 @@ __device__ __forceinline__ void da_merge_blocks(const DecodeDev& d, int rq, int 
     }
 }
 
-constexpr int DA_MERGE_THREADS = 128;     // four warps, one (request, query head) unit each
+constexpr int DA_MERGE_THREADS = 128;     // four warps: one (request, query head) unit each, or all four on one
 
-// One warp per (request, query head): merges the partials of the workers that covered the unit.
+// Merges the partials of the workers that covered a (request, query head).  WIDE: four warps share a unit, a quarter of its
+// blocks each (few units, many short blocks: the loads of a unit were a chain of dependent batches in one warp).
+template <bool WIDE>
 __global__ void __launch_bounds__(DA_MERGE_THREADS) decode_merge_kernel(DecodeDev d) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int lane = threadIdx.x & 31;
-    const int unit = blockIdx.x * (DA_MERGE_THREADS / 32) + (threadIdx.x >> 5);
+    constexpr int WARPS = DA_MERGE_THREADS / 32;
+    dependency_release();
+    dependency_wait();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int unit = WIDE ? (int)blockIdx.x : (int)blockIdx.x * WARPS + warp;
     if (unit >= d.B * d.n_q) return;
     const int rq = unit / d.n_q, qg = unit % d.n_q;
     const int h = qg / d.G, qh = qg % d.G;
     const int blk_pages = d.head[1], nblocks = d.head[2];
-    const int pages = d.prefix[rq + 1] - d.prefix[rq];
+    const int f0 = d.prefix[rq], f1 = d.prefix[rq + 1];
     const size_t bq = (size_t)rq * d.n_q + qg;
     uint2* out2 = reinterpret_cast<uint2*>(d.out + bq * 128) + lane;      // four bf16 channels
-    if (pages == 0) {
+    if (f1 == f0) {
+        if (WIDE && warp != 0) return;
         *out2 = make_uint2(0u, 0u);
         if (lane == 0 && d.lse) d.lse[bq] = -INFINITY;
         return;
     }
     // the blocks that covered the request
-    const int g0 = da_block_of(d.prefix[rq], blk_pages, nblocks), g1 = da_block_of(d.prefix[rq + 1] - 1, blk_pages, nblocks);
+    int g0 = da_block_of(f0, blk_pages, nblocks), g1 = da_block_of(f1 - 1, blk_pages, nblocks);
     float M, l;
     float4 acc;
-    da_merge_blocks(d, rq, h, qh, g0, g1, lane, M, acc, l);
+    if constexpr (WIDE) {
+        __shared__ float4 acc_s[WARPS][32];
+        __shared__ float2 ml_s[WARPS];
+        const int per = (g1 - g0 + WARPS) / WARPS, mine = g0 + warp * per;
+        da_merge_blocks(d, rq, h, qh, mine, min(g1, mine + per - 1), lane, M, acc, l);
+        acc_s[warp][lane] = acc;
+        if (lane == 0) ml_s[warp] = make_float2(M, l);
+        __syncthreads();
+        if (warp != 0) return;
+#pragma unroll
+        for (int w = 1; w < WARPS; ++w) M = fmaxf(M, ml_s[w].x);
+        const float2 first = ml_s[0];
+        float s = first.x == -INFINITY ? 0.f : exp2f(first.x - M);
+        acc.x *= s; acc.y *= s; acc.z *= s; acc.w *= s;
+        l = first.y * s;
+#pragma unroll
+        for (int w = 1; w < WARPS; ++w) {
+            const float2 ml = ml_s[w];
+            const float4 o = acc_s[w][lane];
+            s = ml.x == -INFINITY ? 0.f : exp2f(ml.x - M);
+            acc.x += o.x * s; acc.y += o.y * s; acc.z += o.z * s; acc.w += o.w * s;
+            l += ml.y * s;
+        }
+    } else {
+        da_merge_blocks(d, rq, h, qh, g0, g1, lane, M, acc, l);
+    }
     const __nv_bfloat162 lo = __floats2bfloat162_rn(l > 0.f ? acc.x / l : 0.f, l > 0.f ? acc.y / l : 0.f);
     const __nv_bfloat162 hi = __floats2bfloat162_rn(l > 0.f ? acc.z / l : 0.f, l > 0.f ? acc.w / l : 0.f);
     *out2 = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
@@ -975,22 +1101,7 @@ __global__ void __launch_bounds__(DA_MERGE_THREADS) decode_return_kernel(DecodeD
         asm volatile("st.release.sys.global.u32 [%0], %1;" ::"l"(t.peer_done_flags[threadIdx.x] + t.rank), "r"(step_s) : "memory");
 }
 
-static int da_workers() { return sm_count() * DA_CTAS_PER_SM * DA_WARPS; }
-
-// launch configuration of a kernel that may start before the previous kernel of the stream has finished (it orders
-// itself with griddepcontrol.wait)
-static cudaLaunchConfig_t da_pdl_config(int grid, int block, size_t smem, cudaStream_t st, cudaLaunchAttribute* attr) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3((unsigned)block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cfg;
-}
+static int da_workers(int bits) { return sm_count() * da_ctas_per_sm(bits) * DA_WARPS; }
 
 // workspace: header, request prefix, block starts, partials of (max_blocks + B) x n_kv slots
 struct DALayout {
@@ -1007,7 +1118,7 @@ static DALayout da_layout(int B, int n_q, int n_kv, int max_blocks) {
     l.total = l.part_ml + slots * G * 2 * sizeof(float);
     return l;
 }
-static int da_default_blocks(int n_kv) { return DA_ITEMS_PER_WORKER * max(1, da_workers() / n_kv); }
+static int da_default_blocks(int n_kv) { return DA_ITEMS_PER_WORKER * max(1, da_workers(8) / n_kv); }
 // the most blocks a workspace of `bytes` has room for (0: not even one)
 static int da_blocks_for(size_t bytes, int B, int n_q, int n_kv) {
     int lo = 0, hi = da_default_blocks(n_kv);
@@ -1043,7 +1154,7 @@ int pikv::decode_attn_run(const pikv_decode_params* p, cudaStream_t st, int bits
     PIKV_REQUIRE(p->n_q / p->n_kv <= DA_MAX_GROUP, PIKV_EUNSUPPORTED, "decode_attn: %d query heads per KV head (max %d)",
                  p->n_q / p->n_kv, DA_MAX_GROUP);
     PIKV_REQUIRE(p->num_seqs > 0 && p->max_pages > 0 && p->num_pages > 0, PIKV_EINVAL, "decode_attn: bad cache geometry");
-    PIKV_REQUIRE(p->n_kv <= da_workers(), PIKV_ELIMIT, "decode_attn: n_kv=%d exceeds the %d workers of the grid", p->n_kv, da_workers());
+    PIKV_REQUIRE(p->n_kv <= da_workers(bits), PIKV_ELIMIT, "decode_attn: n_kv=%d exceeds the %d workers of the grid", p->n_kv, da_workers(bits));
     PIKV_REQUIRE((long long)p->B * p->max_pages < (1ll << 31), PIKV_ELIMIT, "decode_attn: B * max_pages must stay below 2^31");
     PIKV_REQUIRE(p->B <= DA_MAX_REQ, PIKV_ELIMIT, "decode_attn: at most %d streams per call (got %d)", DA_MAX_REQ, p->B);
     PIKV_REQUIRE((long long)p->B * p->n_q < (1ll << 21), PIKV_ELIMIT, "decode_attn: B * n_q too large for one call");
@@ -1061,11 +1172,12 @@ int pikv::decode_attn_run(const pikv_decode_params* p, cudaStream_t st, int bits
     PIKV_REQUIRE(d.scores == nullptr || d.score_stride > 0, PIKV_EINVAL, "decode_attn: score_stride");
     d.probs16 = static_cast<__half*>(p->probs16); d.step_max = p->step_max;
     d.probs_stride = p->probs_stride; d.step_stride = p->step_stride;
+    d.probs_pairs = (reinterpret_cast<uintptr_t>(p->probs16) & 3) == 0 && (p->probs_stride & 1) == 0;
     PIKV_REQUIRE(d.probs16 == nullptr || (d.step_max != nullptr && d.probs_stride > 0 && d.step_stride > 0 && d.lse != nullptr),
                  PIKV_EINVAL, "decode_attn: probs16 needs step_max, both strides and lse");
     PIKV_REQUIRE(p->workspace != nullptr, PIKV_EINVAL, "decode_attn: null workspace");
     PIKV_REQUIRE((reinterpret_cast<uintptr_t>(p->workspace) & 15) == 0, PIKV_EINVAL, "decode_attn: workspace must be 16-byte aligned");
-    d.workers = da_workers();
+    d.workers = da_workers(bits);
     d.max_blocks = da_blocks_for(p->workspace_bytes, p->B, p->n_q, p->n_kv);
     PIKV_REQUIRE(d.max_blocks >= 1, PIKV_EINVAL, "decode_attn: workspace too small (%zu bytes at least, %zu for full speed)",
                  da_layout(p->B, p->n_q, p->n_kv, 1).total, da_layout(p->B, p->n_q, p->n_kv, da_default_blocks(p->n_kv)).total);
@@ -1076,41 +1188,53 @@ int pikv::decode_attn_run(const pikv_decode_params* p, cudaStream_t st, int bits
     d.blk_start = reinterpret_cast<int2*>(ws + lay.blk_start);
     d.part_o = reinterpret_cast<float*>(ws + lay.part_o);
     d.part_ml = reinterpret_cast<float*>(ws + lay.part_ml);
-    if (plan != nullptr) decode_plan_kernel<true><<<1, DA_PLAN_THREADS, (size_t)(p->B + 1) * sizeof(int), st>>>(d, *plan);
-    else decode_plan_kernel<false><<<1, DA_PLAN_THREADS, (size_t)(p->B + 1) * sizeof(int), st>>>(d, ShardPlan{});
-    int rc = check_launch("decode_plan_kernel");
-    if (rc != PIKV_OK) return rc;
+    // A list that is short for certain (by the page table's width; the lengths are only known on the device) is planned by
+    // the attention CTAs themselves: above DA_DIRECT_PAGES pages a worker the plan kernel's few microseconds no longer
+    // show and the claimed items even out fast and slow SMs.
+    const bool direct = plan == nullptr && ret == nullptr && p->B <= DA_DIRECT_REQ &&
+                        (long long)p->B * p->max_pages * p->n_kv <= (long long)d.workers * DA_DIRECT_PAGES;
+    int rc = PIKV_OK;
+    if (!direct) {
+        if (plan != nullptr) decode_plan_kernel<true><<<1, DA_PLAN_THREADS, (size_t)(p->B + 1) * sizeof(int), st>>>(d, *plan);
+        else launch_dependent(decode_plan_kernel<false>, 1, DA_PLAN_THREADS, (size_t)(p->B + 1) * sizeof(int), st, d, ShardPlan{});
+        rc = check_launch("decode_plan_kernel");
+        if (rc != PIKV_OK) return rc;
+    }
     const int grid = d.workers / DA_WARPS;
     const bool gs = d.G <= 4;      // integer first product (see decode_attn_kernel)
-    cudaLaunchAttribute attr[1];   // programmatic dependent launch of the attention and the merge kernel
-#define PIKV_DA_LAUNCH(BITS, GS)                                                                                          \
+#define PIKV_DA_LAUNCH(BITS, GS, DIRECT)                                                                                  \
     do {                                                                                                                  \
-        const size_t smem = da_smem_bytes<BITS>();                                                                        \
-        auto kern = decode_attn_kernel<BITS, GS>;                                                                         \
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)            \
+        const size_t smem = da_smem_bytes<BITS>() + (DIRECT ? (size_t)(p->B + 1) * sizeof(int) : 0);                      \
+        if (!allow_smem<decode_attn_kernel<BITS, GS, DIRECT>>((int)da_smem_bytes<BITS>() + (DA_DIRECT_REQ + 1) * 4))      \
             return check_launch("decode_attn smem attribute");                                                            \
-        cudaLaunchConfig_t cfg = da_pdl_config(grid, DA_THREADS, smem, st, attr);                                         \
-        (void)cudaLaunchKernelEx(&cfg, kern, d);                                                                          \
+        launch_dependent(decode_attn_kernel<BITS, GS, DIRECT>, grid, DA_THREADS, smem, st, d);                            \
     } while (0)
-    if (bits == 8 && gs) PIKV_DA_LAUNCH(8, true);
-    else if (bits == 8) PIKV_DA_LAUNCH(8, false);
-    else if (gs) PIKV_DA_LAUNCH(4, true);
-    else PIKV_DA_LAUNCH(4, false);
+#define PIKV_DA_LAUNCH2(BITS, GS)                                                                                         \
+    do {                                                                                                                  \
+        if (direct) PIKV_DA_LAUNCH(BITS, GS, true);                                                                       \
+        else PIKV_DA_LAUNCH(BITS, GS, false);                                                                             \
+    } while (0)
+    if (bits == 8 && gs) PIKV_DA_LAUNCH2(8, true);
+    else if (bits == 8) PIKV_DA_LAUNCH2(8, false);
+    else if (gs) PIKV_DA_LAUNCH2(4, true);
+    else PIKV_DA_LAUNCH2(4, false);
+#undef PIKV_DA_LAUNCH2
 #undef PIKV_DA_LAUNCH
     rc = check_launch(bits == 8 ? "decode_attn_kernel<8>" : "decode_attn_kernel<4>");
     if (rc != PIKV_OK) return rc;
     const int units = p->B * p->n_q, per_cta = DA_MERGE_THREADS / 32;
     const int merge_ctas = (units + per_cta - 1) / per_cta;
-    // the sharded return walks its units with a grid that is resident at once (one system-scope fence per CTA)
-    cudaLaunchConfig_t mcfg = da_pdl_config(ret != nullptr ? min(merge_ctas, sm_count() * 8) : merge_ctas, DA_MERGE_THREADS, 0, st, attr);
     if (ret != nullptr) {
-        (void)cudaLaunchKernelEx(&mcfg, decode_return_kernel, d, *ret);
+        // the sharded return walks its units with a grid that is resident at once (one system-scope fence per CTA)
+        launch_dependent(decode_return_kernel, min(merge_ctas, sm_count() * 8), DA_MERGE_THREADS, 0, st, d, *ret);
         rc = check_launch("decode_return_kernel");
     } else {
-        (void)cudaLaunchKernelEx(&mcfg, decode_merge_kernel, d);
+        // four warps a unit while that keeps the merge inside one wave of sixteen CTAs per SM
+        if (units <= sm_count() * 16) launch_dependent(decode_merge_kernel<true>, units, DA_MERGE_THREADS, 0, st, d);
+        else launch_dependent(decode_merge_kernel<false>, merge_ctas, DA_MERGE_THREADS, 0, st, d);
         rc = check_launch("decode_merge_kernel");
     }
-    count_launch(3);
+    count_launch(direct ? 2 : 3);
     return rc;
 }
 
@@ -1164,7 +1288,7 @@ extern "C" int pikv_decode_attn_q8_static(const pikv_decode_params* p, pikv_stre
     PIKV_REQUIRE(p->B > 0 && p->n_q > 0 && p->n_kv > 0 && p->n_q % p->n_kv == 0 && p->max_pages > 0, PIKV_EINVAL,
                  "decode_attn_static: bad sizes");
     // the built-in array is smaller than the workspace the regular entry point asks for: fewer, longer blocks
-    const size_t need = da_layout(p->B, p->n_q, p->n_kv, max(1, da_workers() / p->n_kv)).total;
+    const size_t need = da_layout(p->B, p->n_q, p->n_kv, max(1, da_workers(8) / p->n_kv)).total;
     PIKV_REQUIRE(need <= DA_STATIC_SCRATCH_BYTES, PIKV_ELIMIT,
                  "decode_attn_static: %d streams x %d query heads need %zu bytes of scratch for the partial results, the "
                  "built-in array holds %zu; split the batch or use pikv_decode_attn_q8 with your own workspace",

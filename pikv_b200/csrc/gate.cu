@@ -598,27 +598,16 @@ static int launch_logits(const GateDev& g, cudaStream_t st) {
     return check_launch("gate_logits_kernel");
 }
 
-// launched as a programmatic dependent: the kernel's start overlaps the end of the one before
 template <typename... KArgs, typename... Args>
-static int launch_dependent(const char* what, void (*kern)(KArgs...), int grid, size_t smem, cudaStream_t st, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = GATE_THREADS;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kern, args...);
+static int launch_tail(const char* what, void (*kern)(KArgs...), int grid, size_t smem, cudaStream_t st, const Args&... args) {
+    launch_dependent(kern, grid, GATE_THREADS, smem, st, args...);
     return check_launch(what);
 }
 
 static int dispatch_launch(const int* topk_idx, const float* topk_w, const int* slot, const int* counts_k, const float* prob_sum,
                            int T, int E, int k, const pikv_dense_out& d, cudaStream_t st) {
     count_launch(1);
-    return launch_dependent("dispatch_scatter_kernel", dispatch_scatter_kernel, ceil_div(T * k, GATE_THREADS), 0, st, topk_idx, topk_w,
+    return launch_tail("dispatch_scatter_kernel", dispatch_scatter_kernel, ceil_div(T * k, GATE_THREADS), 0, st, topk_idx, topk_w,
                             slot, counts_k, prob_sum, T, E, k, d);
 }
 
@@ -630,14 +619,14 @@ static int launch_partial(GateDev& g, const float* part, int groups, const void*
         const size_t smem = sizeof(float) * GATE_THREADS * (EP + 1) + (size_t)GATE_THREADS * max(4, g.k) * (sizeof(int) + 1);
         if (smem > 48 * 1024 && !allow_smem<gate_cluster_kernel<EP>>(200 * 1024)) return check_launch("gate_cluster smem attribute");
         count_launch(1);
-        return launch_dependent("gate_cluster_kernel", gate_cluster_kernel<EP>, GC_CTAS, smem, st, g, part, groups, b2, b2_bf16,
+        return launch_tail("gate_cluster_kernel", gate_cluster_kernel<EP>, GC_CTAS, smem, st, g, part, groups, b2, b2_bf16,
                                 dense ? *dense : pikv_dense_out{});
     }
     const size_t smem = sizeof(int) * (GATE_WARPS * EP + EP + GATE_MAX_K * EP) + sizeof(float) * (GATE_WARPS * EP + GP_TOKENS * (EP + 1)) +
                         (size_t)g.chunk * g.k;
     if (smem > 48 * 1024 && !allow_smem<gate_partial_kernel<EP>>()) return check_launch("gate_partial smem attribute");
-    int rc = launch_dependent("gate_partial_kernel", gate_partial_kernel<EP>, g.G, smem, st, g, part, groups, b2, b2_bf16);
-    if (rc == PIKV_OK) rc = launch_dependent("gate_finalize_kernel", gate_finalize_kernel, g.G, 0, st, g);
+    int rc = launch_tail("gate_partial_kernel", gate_partial_kernel<EP>, g.G, smem, st, g, part, groups, b2, b2_bf16);
+    if (rc == PIKV_OK) rc = launch_tail("gate_finalize_kernel", gate_finalize_kernel, g.G, 0, st, g);
     count_launch(2);
     return rc != PIKV_OK || !dense ? rc : dispatch_launch(g.topk_idx, g.topk_w, g.slot, g.counts_k, g.prob_sum, g.T, g.E, g.k, *dense, st);
 }

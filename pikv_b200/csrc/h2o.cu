@@ -1331,45 +1331,86 @@ __global__ void h2o_accumulate_attn_kernel(const float* scores, int score_stride
 
 // the same increment from the decode kernel's compact output: f16 probabilities relative to the maximum of their
 // softmax step, that maximum per 16-position page (log2 domain), and the final log-sum-exp.  A thread owns eight
-// consecutive positions (one 16-byte load per query head, the step's factor once per thread, acc as two float4);
-// rows that are not 16-byte aligned, and the ragged end of a row, take the scalar path.
-__global__ void __launch_bounds__(256) h2o_accumulate_probs_kernel(const __half* probs, int probs_stride, const float* step_max,
+// consecutive positions: one 16-byte load per query head, four heads in flight, the step's factor once per head.  The
+// accumulator is updated as two float4, or, when its rows are not 16-byte aligned, 32 consecutive floats at a time after
+// a turn through shared memory (a row of 16385 positions took 20 us at 16 x 8 x 16384 with a thread's eight floats read
+// and written one by one).  Probability rows that are not 16-byte aligned, and the ragged end of a row, are read one by one.
+constexpr int AP_THREADS = 256;
+__global__ void __launch_bounds__(AP_THREADS) h2o_accumulate_probs_kernel(const __half* probs, int probs_stride, const float* step_max,
                                                                    int step_stride, const float* lse, const int* seq_len, int B,
-                                                                   int n_q, int n_kv, float* acc, int acc_stride, int vec_ok) {
-    const int pos0 = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
+                                                                   int n_q, int n_kv, float* acc, int acc_stride, int vec_probs, int vec_acc) {
+    __shared__ float4 turn[AP_THREADS / 32][64];
+    dependency_wait();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int pos0 = (blockIdx.x * AP_THREADS + threadIdx.x) * 8;
     const int bh = blockIdx.y;
     const int b = bh / n_kv, h = bh % n_kv;
     int len = seq_len ? seq_len[b] : probs_stride;
     len = min(min(len, acc_stride), min(probs_stride, step_stride * 16));
-    if (pos0 >= len) return;
+    if (pos0 - lane * 8 >= len) return;                   // the whole warp is past the end
     const int g = n_q / n_kv;
     float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    const bool full = vec_ok && pos0 + 8 <= len;
-    for (int i = 0; i < g; ++i) {
-        const size_t hq = (size_t)b * n_q + (size_t)h * g + i;
-        const float f = exp2f(step_max[hq * step_stride + (pos0 >> 4)] - lse[hq] * 1.4426950408889634f);
-        if (full) {
-            const uint4 v = ld_stream_16(probs + hq * probs_stride + pos0);
-            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    const bool whole = pos0 + 8 <= len;
+    for (int i0 = 0; i0 < g; i0 += 4) {
+        float f[4];
+        uint4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            f[u] = 0.f;
+            v[u] = make_uint4(0, 0, 0, 0);
+            if (i0 + u < g && pos0 < len) {
+                const size_t hq = (size_t)b * n_q + (size_t)h * g + i0 + u;
+                f[u] = exp2f(__ldg(step_max + hq * step_stride + (pos0 >> 4)) - __ldg(lse + hq) * 1.4426950408889634f);
+                const __half* p = probs + hq * probs_stride + pos0;
+                if (vec_probs && whole) {
+                    v[u] = ld_stream_16(p);
+                } else {
+                    uint32_t w[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+                    for (int e = 0; e < 8; ++e)
+                        if (pos0 + e < len) w[e >> 1] |= (uint32_t)__half_as_ushort(p[e]) << (16 * (e & 1));
+                    v[u] = make_uint4(w[0], w[1], w[2], w[3]);
+                }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const uint32_t w[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const float2 p2 = __half22float2(*reinterpret_cast<const __half2*>(&w[q]));
-                s[2 * q] += p2.x * f;
-                s[2 * q + 1] += p2.y * f;
+                s[2 * q] += p2.x * f[u];
+                s[2 * q + 1] += p2.y * f[u];
             }
-        } else {
-            for (int e = 0; e < 8 && pos0 + e < len; ++e) s[e] += __half2float(probs[hq * probs_stride + pos0 + e]) * f;
         }
     }
-    float* arow = acc + (size_t)bh * acc_stride + pos0;
-    if (full) {
-        float4 a0 = reinterpret_cast<float4*>(arow)[0], a1 = reinterpret_cast<float4*>(arow)[1];
+    float* arow = acc + (size_t)bh * acc_stride;
+    if (vec_acc && whole) {
+        float4* a4 = reinterpret_cast<float4*>(arow + pos0);
+        float4 a0 = a4[0], a1 = a4[1];
         a0.x += s[0]; a0.y += s[1]; a0.z += s[2]; a0.w += s[3];
         a1.x += s[4]; a1.y += s[5]; a1.z += s[6]; a1.w += s[7];
-        reinterpret_cast<float4*>(arow)[0] = a0;
-        reinterpret_cast<float4*>(arow)[1] = a1;
-    } else {
-        for (int e = 0; e < 8 && pos0 + e < len; ++e) arow[e] += s[e];
+        a4[0] = a0;
+        a4[1] = a1;
+    }
+    if (__all_sync(0xffffffffu, vec_acc && whole)) return;
+    turn[warp][2 * lane] = make_float4(s[0], s[1], s[2], s[3]);
+    turn[warp][2 * lane + 1] = make_float4(s[4], s[5], s[6], s[7]);
+    __syncwarp();
+    const float* mine = reinterpret_cast<const float*>(turn[warp]);
+    const int first = pos0 - lane * 8;
+    float a[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        const int pos = first + 32 * e + lane;
+        // positions of a thread that used the vector form are done
+        const bool todo = pos < len && !(vec_acc && (pos & ~7) + 8 <= len);
+        a[e] = todo ? arow[pos] : 0.f;
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        const int pos = first + 32 * e + lane;
+        if (pos < len && !(vec_acc && (pos & ~7) + 8 <= len)) arow[pos] = a[e] + mine[32 * e + lane];
     }
 }
 
@@ -1494,13 +1535,12 @@ extern "C" int pikv_h2o_accumulate_probs(const void* probs16, int32_t probs_stri
     PIKV_REQUIRE(probs16 && step_max && lse && acc, PIKV_EINVAL, "h2o_accumulate_probs: null pointer");
     PIKV_REQUIRE(B > 0 && n_q > 0 && n_kv > 0 && n_q % n_kv == 0 && probs_stride > 0 && step_stride > 0 && acc_stride > 0,
                  PIKV_EINVAL, "h2o_accumulate_probs: bad sizes");
-    dim3 grid(ceil_div(min(probs_stride, acc_stride), 256 * 8), B * n_kv);
+    const dim3 grid(ceil_div(min(probs_stride, acc_stride), AP_THREADS * 8), B * n_kv);
     // eight positions of a page never straddle two softmax steps; vector accesses need 16-byte aligned rows
-    const int vec_ok = (reinterpret_cast<uintptr_t>(probs16) & 15) == 0 && (probs_stride & 7) == 0 &&
-                       (reinterpret_cast<uintptr_t>(acc) & 15) == 0 && (acc_stride & 3) == 0;
-    h2o_accumulate_probs_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __half*>(probs16), probs_stride, step_max, step_stride, lse, seq_len, B, n_q, n_kv, acc, acc_stride,
-        vec_ok);
+    const int vec_probs = (reinterpret_cast<uintptr_t>(probs16) & 15) == 0 && (probs_stride & 7) == 0;
+    const int vec_acc = (reinterpret_cast<uintptr_t>(acc) & 15) == 0 && (acc_stride & 3) == 0;
+    launch_dependent(h2o_accumulate_probs_kernel, grid, AP_THREADS, 0, static_cast<cudaStream_t>(stream), static_cast<const __half*>(probs16),
+                     probs_stride, step_max, step_stride, lse, seq_len, B, n_q, n_kv, acc, acc_stride, vec_probs, vec_acc);
     count_launch(1);
     return check_launch("h2o_accumulate_probs_kernel");
 }
