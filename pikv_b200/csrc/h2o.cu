@@ -608,11 +608,9 @@ __global__ void __launch_bounds__(NT) h2o_select_kernel(const float* acc, const 
 // a register word: ties are resolved with a block-wide count of the equal keys in index order (skipped when all
 // of them are kept), and the evict mask and the ascending kept-index list need no atomics and no bit gathering
 // across lanes.  Small CTAs, four per SM: the segments of an SM overlap each other's barriers and load latencies.
-constexpr int SS_THREADS = 256;
 constexpr int SS_BUCKETS = 4096;
 constexpr int SS_LIST_CAP = 1024;
 constexpr int SS_RANK_CAP = 256;                    // listed keys ranked by counting up to this many
-constexpr int SS_BPT = SS_BUCKETS / SS_THREADS;     // buckets a thread owns in the suffix sums
 
 struct SsResult {
     int mode;            // 0: nothing kept, 1: every position, 2: positions >= lo, 3: keys above kth + need_eq keys equal to it
@@ -621,17 +619,18 @@ struct SsResult {
     int raw;             // the array's float bits serve as keys (no set sign bit), see ss_key
 };
 
+template <int NT>
 struct SsShared {
     // the search (histogram, candidate list) and the last pass (transpose tiles) never overlap in time
     union {
-        uint4 tile[SS_THREADS / 32][256];           // per warp: 32 words x 8 chunks of 16 bytes, chunk c of word r at c ^ (r & 7)
+        uint4 tile[NT / 32][256];           // per warp: 32 words x 8 chunks of 16 bytes, chunk c of word r at c ^ (r & 7)
         struct {
             int hist[SS_BUCKETS];
             uint32_t list[SS_LIST_CAP];
         };
     };
-    uint32_t red_a[SS_THREADS / 32], red_b[SS_THREADS / 32];
-    int red_i[SS_THREADS / 32];
+    uint32_t red_a[NT / 32], red_b[NT / 32];
+    int red_i[NT / 32];
     int list_n, bucket, above, bucket_cnt, sorted, need_count, negative;
     uint32_t kmin, kmax;
     SsResult res[2];
@@ -698,9 +697,10 @@ __device__ __forceinline__ int ss_block_scan(int v, int* red, int& total) {
     return before + inc - v;
 }
 
-// bucket holding the rem-th largest counted key: suffix sums over hist, thread t owns buckets [t * SS_BPT, ...)
+// bucket holding the rem-th largest counted key: suffix sums over hist, a thread owns consecutive buckets
 template <int NT>
-__device__ __forceinline__ void ss_pick_bucket(SsShared& sh, int rem) {
+__device__ __forceinline__ void ss_pick_bucket(SsShared<NT>& sh, int rem) {
+    constexpr int SS_BPT = SS_BUCKETS / NT;              // buckets a thread owns in the suffix sums
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     int c[SS_BPT], sum = 0;
 #pragma unroll
@@ -741,7 +741,7 @@ __device__ __forceinline__ int ss_shift_for(uint32_t width) {      // (width >> 
 // RAW: the float bits are taken as keys; returns false (nothing decided) when pass 1 meets a set sign bit, and the
 // caller runs the converting instance instead.
 template <int NT, bool ASCENDING_CHECK, bool RAW>
-__device__ bool ss_find(const float* __restrict__ src, int n, int m, bool aligned, SsShared& sh, SsResult* out) {
+__device__ bool ss_find(const float* __restrict__ src, int n, int m, bool aligned, SsShared<NT>& sh, SsResult* out) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (m <= 0 || m >= n) {
         if (tid == 0) {
@@ -1062,7 +1062,9 @@ __global__ void __launch_bounds__(NT, 1024 / NT) h2o_select_stream_kernel(const 
                                                                            int num_recent, uint8_t* evict_mask, int* keep_idx,
                                                                            int keep_stride, int* kept_count) {
     extern __shared__ __align__(16) unsigned char ss_raw[];
-    SsShared& sh = *reinterpret_cast<SsShared*>(ss_raw);
+    SsShared<NT>& sh = *reinterpret_cast<SsShared<NT>*>(ss_raw);
+    dependency_release();
+    dependency_wait();
     const int seg = blockIdx.x, tid = threadIdx.x, warp = tid >> 5;
     int n = seg_len ? seg_len[seg] : n_all;
     n = max(0, min(n, stride));
@@ -1238,6 +1240,7 @@ __global__ void __launch_bounds__(256, 5) h2o_compact_kernel(CompactDev c) {
         }
     };
 
+    dependency_wait();
     const int kept = min(__ldg(p.kept_count + seg), p.keep_stride);
     CompactTile cur, nxt, nxt2;
     int tile = blockIdx.y;
@@ -1447,6 +1450,14 @@ extern "C" int pikv_h2o_accumulate(float* acc, float* ts, int32_t n, const int32
     return check_launch("h2o_accumulate");
 }
 
+template <int NT>
+static void select_stream_launch(const float* acc, const float* ts, int segments, int stride, const int* seg_len, int n, int num_heavy,
+                                 int num_recent, uint8_t* evict_mask, int* keep_idx, int keep_stride, int* kept_count, cudaStream_t st) {
+    if (!allow_smem<h2o_select_stream_kernel<NT>>((int)sizeof(SsShared<NT>))) return;      // reported by check_launch
+    launch_dependent(h2o_select_stream_kernel<NT>, segments, NT, sizeof(SsShared<NT>), st, acc, ts, stride, seg_len, n, num_heavy,
+                     num_recent, evict_mask, keep_idx, keep_stride, kept_count);
+}
+
 extern "C" int pikv_h2o_select(const float* acc, const float* ts, int32_t segments, int32_t stride,
                                const int32_t* seg_len, int32_t n, int32_t num_heavy, int32_t num_recent,
                                uint8_t* evict_mask, int32_t* keep_idx, int32_t keep_stride, int32_t* kept_count,
@@ -1459,11 +1470,13 @@ extern "C" int pikv_h2o_select(const float* acc, const float* ts, int32_t segmen
     const size_t words = (size_t)(stride + 31) / 32 * 4;
     const int variant = h2o_select_variant_for_tests();
     if (variant == 0) {
-        auto kern = h2o_select_stream_kernel<SS_THREADS>;
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SsShared)) != cudaSuccess)
-            return check_launch("h2o_select smem attribute");
-        kern<<<segments, SS_THREADS, sizeof(SsShared), st>>>(acc, ts, stride, seg_len, n, num_heavy, num_recent, evict_mask,
-                                                             keep_idx, keep_stride, kept_count);
+        // 1024 threads of an SM in every case: four small CTAs that overlap each other's barriers when there are segments
+        // for them, one or two wide ones (a quarter or half of the dependent load batches each) when there are not.  A
+        // thread keeps at least one 32-position word.  256 segments x 32768: 46 us with 256 threads, 38 with 512; 8 segments: 27 us, 19 with 1024.
+        const int sms = sm_count(), words_all = ceil_div(n, 32);
+        if (segments <= sms && words_all >= 1024) select_stream_launch<1024>(acc, ts, segments, stride, seg_len, n, num_heavy, num_recent, evict_mask, keep_idx, keep_stride, kept_count, st);
+        else if (segments <= 2 * sms && words_all >= 512) select_stream_launch<512>(acc, ts, segments, stride, seg_len, n, num_heavy, num_recent, evict_mask, keep_idx, keep_stride, kept_count, st);
+        else select_stream_launch<256>(acc, ts, segments, stride, seg_len, n, num_heavy, num_recent, evict_mask, keep_idx, keep_stride, kept_count, st);
         count_launch(1);
         return check_launch("h2o_select_stream_kernel");
     }
@@ -1523,8 +1536,8 @@ extern "C" int pikv_h2o_compact(const pikv_compact_params* p, pikv_stream_t stre
     dim3 grid(segments, (unsigned)per_seg);
     PIKV_REQUIRE((long long)p->num_pages * p->n_kv * PIKV_PAGE_TOKENS < (1ll << 31), PIKV_ELIMIT,
                  "h2o_compact: the pools must hold fewer than 2^31 rows");
-    if (p->per_head) h2o_compact_kernel<true><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(c);
-    else h2o_compact_kernel<false><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(c);
+    if (p->per_head) launch_dependent(h2o_compact_kernel<true>, grid, 256, 0, static_cast<cudaStream_t>(stream), c);
+    else launch_dependent(h2o_compact_kernel<false>, grid, 256, 0, static_cast<cudaStream_t>(stream), c);
     count_launch(1);
     return check_launch("h2o_compact_kernel");
 }
