@@ -649,6 +649,45 @@ int pikv_a2a_unpack(const void* recv_buf, int32_t n_records, int32_t n_kv,
                     void* k_codes, void* v_codes, void* k_scale, void* v_scale,
                     uint32_t* status, pikv_stream_t stream);
 
+/* ------------------------------------------------------------------------
+ * PiKVMoE inference forward up to the vocabulary projection, fp32
+ * (core/single/pikv_moe.py:277-336, core/single/routing_strategy.py:100-150).
+ *   out[t] = sum_e r[t,e] (relu(dense_e(x[t]) + lora_e(x[t])) + cached_e), r the adaptive router's
+ *   weights, cached_e the mean of the importance-weighted value rows behind compressor and value LoRA;
+ *   then every cache's `slot` receives the mean token, mean expert output and mean importance, and
+ *   cache_ptrs[e] the slot after it.  logits_* [T,E] are the balanced and the importance gate's raw
+ *   logits and the logarithm of the mixture r, for pikv_gate_fused.
+ * H a multiple of 128 up to 1024, LoRA ranks up to 16, compressor width a multiple of 4; all pointers
+ * 16-byte aligned.
+ * ---------------------------------------------------------------------- */
+#define PIKV_MOE_MAX_EXPERTS 16
+typedef struct {
+    const float *w, *b, *lora_a, *lora_b;             /* dense [H,H], [H]; A [H,rank], B [rank,H] */
+    const float *c1_w, *c1_b, *c2_w, *c2_b;           /* compressor [mid,H], [mid], [H,mid], [H]  */
+    const float *v_a, *v_b;                           /* value LoRA [H,v_rank], [v_rank,H]        */
+    float *keys, *values, *importance;                /* ring cache [slots,H], [slots,H], [slots] */
+    float scale, v_scale;
+    int32_t rank, v_rank, mid, slots, slot;
+} pikv_moe_expert;
+typedef struct {
+    const float *w1, *b1, *w2, *b2;
+    float temperature;
+} pikv_moe_net;
+typedef struct {
+    const float* x;                                   /* [B,S,H] */
+    int32_t B, S, H, E;
+    const float *sel_w1, *sel_b1, *sel_w2, *sel_b2;   /* strategy selector H -> H/2 -> 2 */
+    pikv_moe_net lb, imp, pred;                       /* gate nets H -> H -> E, importance H -> H/2 -> 1 */
+    pikv_moe_expert expert[PIKV_MOE_MAX_EXPERTS];
+    int64_t* cache_ptrs;
+    float *logits_lb, *logits_imp, *logits_mix;
+    float* out;                                       /* [B,S,H] */
+    void* workspace;
+    size_t workspace_bytes;
+} pikv_moe_params;
+size_t pikv_moe_workspace_bytes(int32_t B, int32_t S, int32_t H, int32_t E);
+int pikv_moe_forward(const pikv_moe_params* p, pikv_stream_t stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -8,6 +8,8 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <ATen/ATen.h>
 #include <c10/core/GradMode.h>
+#include <c10/core/InferenceMode.h>
+#include <c10/cuda/CUDAFunctions.h>
 #include <ATen/ops/empty.h>
 #include <ATen/ops/empty_like.h>
 #include <c10/cuda/CUDAStream.h>
@@ -571,6 +573,243 @@ PyObject* lowrank_pair(PyObject* const* a, Py_ssize_t) {
     return tuple(y[0], y[1]);
 }
 
+// ---- PiKVMoE -----------------------------------------------------------------------------------------------
+// The forward's kernels take raw weights, so every module they stand for has to be what it was built as: walked on each
+// call, about 70 modules in a few microseconds.  Whatever does not fit leaves as NotApplicable and the caller runs the modules.
+struct NotApplicable : std::exception {};
+
+PyObject* interned(const char* s) {
+    PyObject* o = PyUnicode_InternFromString(s);
+    if (!o) throw Raised();
+    return o;
+}
+#define PIKV_NAME(text) ([]() { static PyObject* const name = interned(text); return name; }())
+
+void need(bool ok) {
+    if (!ok) throw NotApplicable();
+}
+
+struct Mod {
+    PyObject* dict;                            // borrowed: the module owns it and is held by its parent
+    // a module of exactly that class, without hooks and without a forward of its own
+    Mod(PyObject* m, PyObject* types, int type) {
+        need(m && (PyObject*)Py_TYPE(m) == PyTuple_GET_ITEM(types, type));
+        dict = PyObject_GenericGetDict(m, nullptr);
+        if (!dict) throw Raised();
+        Py_DECREF(dict);
+        need(empty(PIKV_NAME("_forward_hooks")) && empty(PIKV_NAME("_forward_pre_hooks")) && !PyDict_GetItem(dict, PIKV_NAME("forward")));
+    }
+    PyObject* get(PyObject* key) const {
+        PyObject* o = PyDict_GetItem(dict, key);
+        need(o);
+        return o;
+    }
+    bool empty(PyObject* key) const {
+        PyObject* o = PyDict_GetItem(dict, key);
+        return o && PyDict_Check(o) && PyDict_GET_SIZE(o) == 0;
+    }
+    PyObject* in(PyObject* table, PyObject* key) const {
+        PyObject* t = get(table);
+        need(PyDict_Check(t));
+        PyObject* o = PyDict_GetItem(t, key);
+        need(o);
+        return o;
+    }
+    PyObject* child(PyObject* key) const { return in(PIKV_NAME("_modules"), key); }
+    long integer(PyObject* key) const {
+        PyObject* o = get(key);
+        need(PyLong_CheckExact(o));
+        return num(o);
+    }
+    float number(PyObject* key) const {
+        PyObject* o = get(key);
+        need(PyFloat_Check(o) || PyLong_CheckExact(o));
+        return real(o);
+    }
+    bool is_false(PyObject* key) const { return get(key) == Py_False; }
+};
+
+struct MoeWalk {
+    PyObject* types;
+    c10::Device device;
+    enum { MOE, MODULES, EXPERT, LORA, LINEAR, DROPOUT, CACHE, COMPRESSOR, PYRAMID, ADAPTIVE, BALANCED, IMPORTANCE, SEQUENTIAL, RELU, SIGMOID, SOFTMAX,
+           NTYPES };
+
+    const at::Tensor& tensor(PyObject* o, at::IntArrayRef sizes, at::ScalarType type = at::kFloat) const {
+        need(THPVariable_Check(o));
+        const at::Tensor& t = THPVariable_Unpack(o);
+        need(t.layout() == at::kStrided && t.device() == device && t.scalar_type() == type && t.sizes() == sizes && t.is_contiguous() &&
+             (!t.is_inference() || c10::InferenceMode::is_enabled()) && !t.unsafeGetTensorImpl()->is_python_dispatch() &&
+             reinterpret_cast<uintptr_t>(t.const_data_ptr()) % (type == at::kFloat ? 16 : 8) == 0);
+        return t;
+    }
+    const float* param(const Mod& m, PyObject* key, at::IntArrayRef sizes) const {
+        return static_cast<const float*>(tensor(m.in(PIKV_NAME("_parameters"), key), sizes).const_data_ptr());
+    }
+    const at::Tensor& buf(const Mod& m, PyObject* key, at::IntArrayRef sizes, at::ScalarType type = at::kFloat) const {
+        return tensor(m.in(PIKV_NAME("_buffers"), key), sizes, type);
+    }
+    static PyObject* digit(int64_t i) {
+        static PyObject* names[PIKV_MOE_MAX_EXPERTS] = {};
+        need(i < PIKV_MOE_MAX_EXPERTS);
+        if (!names[i]) names[i] = interned(std::to_string(i).c_str());
+        return names[i];
+    }
+    Mod list(PyObject* m, int type, int64_t count) const {
+        const Mod l(m, types, type);
+        PyObject* c = l.get(PIKV_NAME("_modules"));
+        need(PyDict_Check(c) && (count < 0 || PyDict_GET_SIZE(c) == count));
+        return l;
+    }
+    void linear(PyObject* m, int64_t out, int64_t in, const float*& w, const float*& b) const {
+        const Mod l(m, types, LINEAR);
+        w = param(l, PIKV_NAME("weight"), {out, in});
+        b = param(l, PIKV_NAME("bias"), {out});
+    }
+    void lora(PyObject* m, int64_t H, const float*& a, const float*& b, int32_t& rank, float& scale) const {
+        const Mod l(m, types, LORA);
+        const Mod drop(l.child(PIKV_NAME("dropout")), types, DROPOUT);
+        need(drop.is_false(PIKV_NAME("training")) || drop.number(PIKV_NAME("p")) == 0.f);
+        const long r = l.integer(PIKV_NAME("rank"));
+        need(r > 0 && r <= 16);
+        rank = (int32_t)r;
+        scale = l.number(PIKV_NAME("scaling"));
+        a = param(l, PIKV_NAME("lora_A"), {H, r});
+        b = param(l, PIKV_NAME("lora_B"), {r, H});
+    }
+    void plain(PyObject* m, int type) const { Mod(m, types, type); }
+    // Linear(H, hidden), ReLU, Linear(hidden, out)[, tail]
+    void net(PyObject* m, int64_t H, int64_t hidden, int64_t out, int tail, const float*& w1, const float*& b1, const float*& w2, const float*& b2) const {
+        const Mod s = list(m, SEQUENTIAL, tail < 0 ? 3 : 4);
+        linear(s.child(digit(0)), hidden, H, w1, b1);
+        plain(s.child(digit(1)), RELU);
+        linear(s.child(digit(2)), out, hidden, w2, b2);
+        if (tail >= 0) plain(s.child(digit(3)), tail);
+        if (tail == SOFTMAX) {
+            const Mod t(s.child(digit(3)), types, tail);
+            PyObject* dim = t.get(PIKV_NAME("dim"));
+            need(PyLong_CheckExact(dim) && num(dim) == -1);
+        }
+    }
+};
+
+// moe(module, x, ring positions, classes) -> (weighted expert sum, three gate results), or None where the modules have to run
+PyObject* moe(PyObject* const* a, Py_ssize_t) {
+    PyObject *positions = a[2], *types = a[3];
+    if (!THPVariable_CheckExact(a[1])) Py_RETURN_NONE;
+    const at::Tensor& xin = THPVariable_Unpack(a[1]);
+    if (!xin.is_cuda() || xin.dim() != 3 || xin.scalar_type() != at::kFloat || !xin.numel() ||
+        xin.device().index() != c10::cuda::current_device() || !PyList_CheckExact(positions) || !PyTuple_CheckExact(types) ||
+        PyTuple_GET_SIZE(types) != MoeWalk::NTYPES)
+        Py_RETURN_NONE;
+    at::Tensor x = xin.contiguous();
+    if (reinterpret_cast<uintptr_t>(x.const_data_ptr()) % 16) x = x.clone();
+    using W = MoeWalk;
+    const W walk{types, x.device()};
+    pikv_moe_params p = {};
+    at::Tensor touched[3 * PIKV_MOE_MAX_EXPERTS + 1];
+    int n_touched = 0, topk[3];
+    float temperature[2];
+    try {
+        need(x.size(0) * x.size(1) <= (1 << 21));
+        p.B = (int32_t)x.size(0); p.S = (int32_t)x.size(1); p.H = (int32_t)x.size(2);
+        const int64_t H = p.H;
+        need(H % 128 == 0 && H <= 1024);
+        const Mod m(a[0], types, W::MOE);
+        const Mod experts = walk.list(m.child(PIKV_NAME("experts")), W::MODULES, -1), caches = walk.list(m.child(PIKV_NAME("kv_caches")), W::MODULES, -1);
+        const int64_t E = PyDict_GET_SIZE(experts.get(PIKV_NAME("_modules")));
+        need(E > 0 && E <= PIKV_MOE_MAX_EXPERTS && PyDict_GET_SIZE(caches.get(PIKV_NAME("_modules"))) >= E && PyList_GET_SIZE(positions) == E);
+        need(!PyDict_GetItem(m.dict, PIKV_NAME("update_cache")));
+        p.E = (int32_t)E;
+        touched[n_touched++] = walk.buf(m, PIKV_NAME("cache_ptrs"), {E}, at::kLong);
+        p.cache_ptrs = ptr<int64_t>(touched[0]);
+        // router
+        const Mod r(m.child(PIKV_NAME("router")), types, W::ADAPTIVE);
+        walk.net(r.child(PIKV_NAME("router_selector")), H, H / 2, 2, W::SOFTMAX, p.sel_w1, p.sel_b1, p.sel_w2, p.sel_b2);
+        const Mod lb(r.child(PIKV_NAME("load_balancing_router")), types, W::BALANCED), imp(r.child(PIKV_NAME("importance_router")), types, W::IMPORTANCE);
+        const Mod* gates[2] = {&lb, &imp};
+        pikv_moe_net* nets[2] = {&p.lb, &p.imp};
+        for (int i = 0; i < 2; ++i) {
+            const Mod& g = *gates[i];
+            walk.net(g.child(PIKV_NAME("router")), H, H, E, -1, nets[i]->w1, nets[i]->b1, nets[i]->w2, nets[i]->b2);
+            temperature[i] = nets[i]->temperature = g.number(PIKV_NAME("temperature"));
+            topk[i] = (int)g.integer(PIKV_NAME("top_k"));
+            need(g.integer(PIKV_NAME("num_experts")) == E && !PyDict_GetItem(g.dict, PIKV_NAME("_gate")));
+        }
+        topk[2] = (int)r.integer(PIKV_NAME("top_k"));
+        need(r.integer(PIKV_NAME("num_experts")) == E);
+        for (int k : topk) need(k >= 1 && k <= std::min<int64_t>(E, 8));
+        walk.net(imp.child(PIKV_NAME("importance_predictor")), H, H / 2, 1, W::SIGMOID, p.pred.w1, p.pred.b1, p.pred.w2, p.pred.b2);
+        // experts and their caches
+        for (int64_t e = 0; e < E; ++e) {
+            pikv_moe_expert& t = p.expert[e];
+            const Mod x_(experts.child(W::digit(e)), types, W::EXPERT), c(caches.child(W::digit(e)), types, W::CACHE);
+            walk.linear(x_.child(PIKV_NAME("dense")), H, H, t.w, t.b);
+            walk.lora(x_.child(PIKV_NAME("lora")), H, t.lora_a, t.lora_b, t.rank, t.scale);
+            need(c.is_false(PIKV_NAME("use_scheduling")) && !PyDict_GetItem(c.dict, PIKV_NAME("update")) && !PyDict_GetItem(c.dict, PIKV_NAME("get_all")));
+            const long size = c.integer(PIKV_NAME("size"));
+            need(size > 0 && size < (1 << 20));
+            t.slots = (int32_t)size;
+            PyObject* at = PyList_GET_ITEM(positions, e);
+            need(PyLong_Check(at));
+            t.slot = (int32_t)num(at);
+            need(t.slot >= 0 && t.slot < size);
+            const at::Tensor &k = walk.buf(c, PIKV_NAME("keys"), {size, H}), &v = walk.buf(c, PIKV_NAME("values"), {size, H}),
+                             &w = walk.buf(c, PIKV_NAME("importance"), {size});
+            for (int64_t q = 0; q < e; ++q) need(p.expert[q].values != ptr<float>(v));      // one cache under two names is read after it is written
+            t.keys = ptr<float>(k); t.values = ptr<float>(v); t.importance = ptr<float>(w);
+            touched[n_touched++] = k; touched[n_touched++] = v; touched[n_touched++] = w;
+            const Mod outer(c.child(PIKV_NAME("compressor")), types, W::COMPRESSOR), pyramid(outer.child(PIKV_NAME("compressor")), types, W::PYRAMID);
+            const Mod layers = walk.list(pyramid.child(PIKV_NAME("compression_layers")), W::MODULES, 2);
+            const Mod first(layers.child(W::digit(0)), types, W::LINEAR);
+            const long mid = first.integer(PIKV_NAME("out_features"));
+            need(mid > 0 && mid % 4 == 0 && mid <= 1024);
+            t.mid = (int32_t)mid;
+            walk.linear(layers.child(W::digit(0)), mid, H, t.c1_w, t.c1_b);
+            walk.linear(layers.child(W::digit(1)), H, mid, t.c2_w, t.c2_b);
+            walk.lora(c.child(PIKV_NAME("value_lora")), H, t.v_a, t.v_b, t.v_rank, t.v_scale);
+        }
+    } catch (const NotApplicable&) {
+        Py_RETURN_NONE;
+    }
+    const int T = p.B * p.S, E = p.E;
+    at::Tensor out = at::empty_like(x);
+    p.workspace_bytes = pikv_moe_workspace_bytes(p.B, p.S, p.H, E);
+    const size_t row = ((size_t)T * E * 4 + 255) & ~size_t(255), tail = pikv_gate_tail_workspace_bytes(T, E, std::max(topk[0], std::max(topk[1], topk[2])));
+    const at::Tensor ws = workspace(x, p.workspace_bytes + 3 * row + 256 + tail);
+    char* base = ptr<char>(ws);
+    p.workspace = base;
+    base += (p.workspace_bytes + 255) & ~size_t(255);
+    float* logits[3];
+    for (int i = 0; i < 3; ++i, base += row) logits[i] = reinterpret_cast<float*>(base);
+    p.x = ptr<float>(x); p.out = ptr<float>(out);
+    p.logits_lb = logits[0]; p.logits_imp = logits[1]; p.logits_mix = logits[2];
+    check(pikv_moe_forward(&p, stream()), "pikv_moe_forward");
+    for (int i = 0; i < n_touched; ++i)
+        if (!touched[i].is_inference()) touched[i].unsafeGetTensorImpl()->bump_version();
+    for (int e = 0; e < E; ++e) {
+        PyObject* next = PyLong_FromLong((p.expert[e].slot + 1) % p.expert[e].slots);
+        if (!next || PyList_SetItem(positions, e, next)) throw Raised();
+    }
+    PyObject* result = PyTuple_New(4);
+    if (!result) throw Raised();
+    PyTuple_SET_ITEM(result, 0, wrap(out));
+    for (int i = 0; i < 3; ++i) {
+        pikv_gate_params g = {};
+        g.T = T; g.E = E; g.top_k = topk[i]; g.dtype = PIKV_F32; g.logits_in = logits[i];
+        g.mask_mode = PIKV_MASK_NONE; g.temperature = i < 2 ? temperature[i] : 1.f;
+        GateOut o(Py_None, x, T, E, g.top_k, i < 2);
+        o.fill(g);
+        g.workspace = base; g.workspace_bytes = tail;
+        if (int rc = pikv_gate_fused(&g, stream())) {
+            Py_DECREF(result);
+            check(rc, "pikv_gate_fused");
+        }
+        PyTuple_SET_ITEM(result, 1 + i, o.result());
+    }
+    return result;
+}
+
 // ---- module ------------------------------------------------------------------------------------------------
 using Fn = PyObject* (*)(PyObject* const*, Py_ssize_t);
 template <Fn F, int N, int M = N>
@@ -606,6 +845,7 @@ PyMethodDef methods[] = {
     method<quant_pair, 9>("quant_pair"),
     method<lowrank, 6>("lowrank"),
     method<lowrank_pair, 10>("lowrank_pair"),
+    method<moe, 4>("moe"),
     {nullptr, nullptr, 0, nullptr},
 };
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

@@ -1,0 +1,410 @@
+// Inference forward of PiKVMoE (core/single/pikv_moe.py:139-336) up to the vocabulary projection, fp32: router nets,
+// LoRA experts, every expert's cached vector, the weighted sum of the experts and the ring update of the caches.
+//
+// As modules this is 180 launches, most of a few microseconds: at 8 x 128 tokens, 4 experts of width 256, 2310 us of host
+// time for 600 us of kernels (and 710 us of vocabulary projection).  Here it is three kernels, 57 us together; the whole
+// forward takes 800 us, bound by the projection:
+//   moe_stats_kernel    one CTA per expert: the mean of the importance-weighted value rows, taken through the
+//                       compressor and the value LoRA (both affine, so the mean may be taken first: 2 vectors instead of
+//                       2 x 128 rows); one CTA per sequence: sum of its tokens and the strategy selector.
+//   moe_gemm_kernel     x against the two gate nets' and the predictor's first layers and all experts' dense layers, one
+//                       grid of 64 x 64 tiles (bound by fp32 FMA: 0.87 GFLOP in 38 us at 8 x 128).  Gate tiles leave
+//                       partial logits instead of activations, expert tiles y = relu(dense + lora) + cached vector and
+//                       its column sums.  Runs beside moe_stats_kernel, whose results only its epilogue needs.
+//   moe_combine_kernel  logits, both softmaxes, the mixture, the experts' weighted sum; E extra CTAs update the caches.
+// All sums have a fixed order; nothing waits on another CTA.
+#include "common.cuh"
+
+namespace pikv {
+
+constexpr int MOE_TILE = 64, MOE_K = 16, MOE_PAD = MOE_TILE + 4;
+constexpr int MOE_MAX_H = 1024, MOE_MAX_RANK = 16;
+constexpr int MOE_STATS_THREADS = 512, MOE_THREADS = 256;
+constexpr int MOE_ROWS = 8;                    // tokens of a combine CTA
+
+struct MoeWork {                               // fp32 words of the workspace
+    float *cached, *sel, *xsum, *part_lb, *part_imp, *part_pred, *y, *ysum;
+};
+
+static size_t moe_layout(int B, int S, int H, int E, float* base, MoeWork* w) {
+    const size_t T = (size_t)B * S, nt = H / MOE_TILE, mt = (T + MOE_TILE - 1) / MOE_TILE;
+    size_t at = 0;
+    auto take = [&](size_t n) {
+        float* p = base ? base + at : nullptr;
+        at += (n + 63) & ~size_t(63);
+        return p;
+    };
+    MoeWork r;
+    r.cached = take((size_t)E * H);
+    r.sel = take((size_t)B * 2);
+    r.xsum = take((size_t)B * H);
+    r.part_lb = take(nt * T * E);
+    r.part_imp = take(nt * T * E);
+    r.part_pred = take(nt / 2 * T);
+    r.y = take((size_t)E * T * H);
+    r.ysum = take(mt * E * H);
+    if (w) *w = r;
+    return at * sizeof(float);
+}
+
+// out[j] = w[j, :] . in + b[j], four rows of a warp at a time; n_in a multiple of 4
+__device__ __forceinline__ void moe_gemv(const float* w, const float* b, const float* in, int n_out, int n_in, float* out, bool relu) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    for (int j0 = warp * 4; j0 < n_out; j0 += warps * 4) {
+        float s[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int i = lane * 4; i < n_in; i += 128) {
+            const float4 v = *reinterpret_cast<const float4*>(in + i);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                if (j0 + r >= n_out) continue;
+                const float4 a = __ldg(reinterpret_cast<const float4*>(w + (size_t)(j0 + r) * n_in + i));
+                s[r] = fmaf(a.x, v.x, fmaf(a.y, v.y, fmaf(a.z, v.z, fmaf(a.w, v.w, s[r]))));
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const float t = warp_sum(s[r]);
+            if (lane == 0 && j0 + r < n_out) {
+                const float o = t + b[j0 + r];
+                out[j0 + r] = relu && o < 0.f ? 0.f : o;
+            }
+        }
+    }
+    __syncthreads();
+}
+
+// sum over rows of src[rows, H] (each times weight[row], if given), left in out[H]; `part` holds 4 floats per thread
+__device__ __forceinline__ void moe_column_sum(const float* src, const float* weight, int rows, int H, float* part, float* out) {
+    const int c = threadIdx.x % (H / 4), g = threadIdx.x / (H / 4), groups = blockDim.x / (H / 4);
+    if (g < groups) {
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+        for (int r = g; r < rows; r += groups) {
+            const float4 v = *reinterpret_cast<const float4*>(src + (size_t)r * H + 4 * c);
+            const float f = weight ? weight[r] : 1.f;
+            s.x += v.x * f; s.y += v.y * f; s.z += v.z * f; s.w += v.w * f;
+        }
+        *reinterpret_cast<float4*>(part + (size_t)g * H + 4 * c) = s;
+    }
+    __syncthreads();
+    for (int h = threadIdx.x; h < H; h += blockDim.x) {
+        float s = 0.f;
+        for (int q = 0; q < groups; ++q) s += part[(size_t)q * H + h];
+        out[h] = s;
+    }
+    __syncthreads();
+}
+
+__global__ void __launch_bounds__(MOE_STATS_THREADS) moe_stats_kernel(const __grid_constant__ pikv_moe_params p, MoeWork w) {
+    dependency_release();
+    __shared__ __align__(16) float part[MOE_STATS_THREADS * 4], v0[MOE_MAX_H], v1[MOE_MAX_H], v2[MOE_MAX_H];
+    __shared__ float r[MOE_MAX_RANK];
+    const int H = p.H, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if ((int)blockIdx.x >= p.E) {              // a sequence: token sum, selector softmax(L2(relu(L1(mean))))
+        const int b = blockIdx.x - p.E;
+        moe_column_sum(p.x + (size_t)b * p.S * H, nullptr, p.S, H, part, v0);
+        for (int h = threadIdx.x; h < H; h += blockDim.x) {
+            w.xsum[(size_t)b * H + h] = v0[h];
+            v1[h] = v0[h] / (float)p.S;
+        }
+        __syncthreads();
+        moe_gemv(p.sel_w1, p.sel_b1, v1, H / 2, H, v2, true);
+        moe_gemv(p.sel_w2, p.sel_b2, v2, 2, H / 2, v0, false);
+        if (threadIdx.x == 0) {
+            const float m = fmaxf(v0[0], v0[1]), a = expf(v0[0] - m), c = expf(v0[1] - m);
+            w.sel[2 * b] = a / (a + c);
+            w.sel[2 * b + 1] = c / (a + c);
+        }
+        return;
+    }
+    const pikv_moe_expert& x = p.expert[blockIdx.x];
+    moe_column_sum(x.values, x.importance, x.slots, H, part, v0);
+    for (int h = threadIdx.x; h < H; h += blockDim.x) v0[h] /= (float)x.slots;
+    __syncthreads();
+    moe_gemv(x.c1_w, x.c1_b, v0, x.mid, H, v1, false);
+    moe_gemv(x.c2_w, x.c2_b, v1, H, x.mid, v2, false);
+    for (int h = threadIdx.x; h < H; h += blockDim.x) v2[h] += v0[h];
+    __syncthreads();
+    if (warp < x.v_rank) {
+        float s = 0.f;
+        for (int h = lane; h < H; h += 32) s = fmaf(v2[h], x.v_a[(size_t)h * x.v_rank + warp], s);
+        s = warp_sum(s);
+        if (lane == 0) r[warp] = s;
+    }
+    __syncthreads();
+    for (int h = threadIdx.x; h < H; h += blockDim.x) {
+        float s = 0.f;
+        for (int k = 0; k < x.v_rank; ++k) s = fmaf(r[k], x.v_b[(size_t)k * H + h], s);
+        w.cached[(size_t)blockIdx.x * H + h] = v2[h] + s * x.v_scale;
+    }
+}
+
+__device__ __forceinline__ uint64_t moe_pair(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void moe_fma2(uint64_t& d, uint64_t a, uint64_t b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b)); }
+
+// Tiles of 64 tokens x 64 outputs, 4 x 4 per thread: 416 tiles at 8 x 128 tokens, three resident per SM, so all of them
+// run at once (128-wide tiles leave a third of the SMs idle at that size).
+__global__ void __launch_bounds__(MOE_THREADS, 3) moe_gemm_kernel(const __grid_constant__ pikv_moe_params p, MoeWork w) {
+    __shared__ __align__(16) float xs[2][MOE_K][MOE_PAD], ws[2][MOE_K][MOE_PAD];
+    __shared__ float as[2][MOE_K][MOE_MAX_RANK];
+    __shared__ float lora[MOE_TILE][MOE_MAX_RANK + 1];
+    const int H = p.H, E = p.E, T = p.B * p.S, nt = H / MOE_TILE;
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    // which layer the tile belongs to, and its first output there: experts first (their epilogue is the longest)
+    int seg = blockIdx.x / nt, tile = blockIdx.x % nt;          // seg: E experts, balanced gate, importance gate, predictor
+    const int m0 = blockIdx.y * MOE_TILE, n0 = tile * MOE_TILE;
+    const bool expert = seg < E;
+    const float *wt, *bias;
+    int rank = 0;
+    const float* la = nullptr;
+    if (expert) { wt = p.expert[seg].w; bias = p.expert[seg].b; rank = p.expert[seg].rank; la = p.expert[seg].lora_a; }
+    else if (seg == E) { wt = p.lb.w1; bias = p.lb.b1; }
+    else if (seg == E + 1) { wt = p.imp.w1; bias = p.imp.b1; }
+    else { wt = p.pred.w1; bias = p.pred.b1; }
+
+    const int lr = tid >> 2, lk = (tid & 3) * 4;
+    const float* xp = p.x + (size_t)min(m0 + lr, T - 1) * H + lk;       // rows past the end are computed and dropped
+    const float* wp = wt + (size_t)(n0 + lr) * H + lk;
+    const int arow = tid / MOE_MAX_RANK, acol = tid % MOE_MAX_RANK;      // 16 x 16 entries of A
+    uint64_t acc[4][2] = {};
+    float lo[MOE_MAX_RANK / 4] = {};
+    float4 xv = *reinterpret_cast<const float4*>(xp), wv = __ldg(reinterpret_cast<const float4*>(wp));
+    float av = acol < rank ? la[(size_t)arow * rank + acol] : 0.f;
+    const int steps = H / MOE_K;
+    for (int s = 0; s < steps; ++s) {
+        const int q = s & 1;
+        xs[q][lk][lr] = xv.x; xs[q][lk + 1][lr] = xv.y; xs[q][lk + 2][lr] = xv.z; xs[q][lk + 3][lr] = xv.w;
+        ws[q][lk][lr] = wv.x; ws[q][lk + 1][lr] = wv.y; ws[q][lk + 2][lr] = wv.z; ws[q][lk + 3][lr] = wv.w;
+        if (rank) as[q][arow][acol] = av;
+        __syncthreads();
+        if (s + 1 < steps) {
+            xv = *reinterpret_cast<const float4*>(xp + (s + 1) * MOE_K);
+            wv = __ldg(reinterpret_cast<const float4*>(wp + (s + 1) * MOE_K));
+            if (acol < rank) av = la[(size_t)((s + 1) * MOE_K + arow) * rank + acol];
+        }
+#pragma unroll
+        for (int k = 0; k < MOE_K; ++k) {
+            const float4 a = *reinterpret_cast<const float4*>(&xs[q][k][ty * 4]);
+            const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(&ws[q][k][tx * 4]);
+            const float av4[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint64_t d = moe_pair(av4[i], av4[i]);
+                moe_fma2(acc[i][0], d, b.x);
+                moe_fma2(acc[i][1], d, b.y);
+            }
+        }
+        if (rank) {                            // x . A of this tile's tokens: thread (token, rank mod 4)
+#pragma unroll
+            for (int j = 0; j < MOE_MAX_RANK / 4; ++j) {
+                if (4 * j >= rank) break;
+#pragma unroll
+                for (int k = 0; k < MOE_K; ++k) lo[j] = fmaf(xs[q][k][lr], as[q][k][4 * j + (tid & 3)], lo[j]);
+            }
+        }
+    }
+    float v[4][4];
+    const float4 bv = __ldg(reinterpret_cast<const float4*>(bias + n0 + 4 * tx));
+    const float bb[4] = {bv.x, bv.y, bv.z, bv.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            float a, b;
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(acc[i][j]));
+            v[i][2 * j] = a + bb[2 * j];
+            v[i][2 * j + 1] = b + bb[2 * j + 1];
+        }
+    if (!expert) {
+        // the second layer's share of these 64 hidden units; x < 0 ? 0 : x keeps a NaN, as torch's relu does
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[i][j] = v[i][j] < 0.f ? 0.f : v[i][j];
+        const bool predictor = seg == E + 2;
+        const float* w2 = predictor ? p.pred.w2 : seg == E ? p.lb.w2 : p.imp.w2;
+        const int hidden = predictor ? H / 2 : H, outs = predictor ? 1 : E;
+        float* to = predictor ? w.part_pred : seg == E ? w.part_lb : w.part_imp;
+        for (int e = 0; e < outs; ++e) {
+            const float4 u = __ldg(reinterpret_cast<const float4*>(w2 + (size_t)e * hidden + n0 + 4 * tx));
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                float s = fmaf(v[i][0], u.x, fmaf(v[i][1], u.y, fmaf(v[i][2], u.z, v[i][3] * u.w)));
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+                const int t = m0 + ty * 4 + i;
+                if (tx == 0 && t < T) to[((size_t)tile * T + t) * outs + e] = s;
+            }
+        }
+        return;
+    }
+    const pikv_moe_expert& x = p.expert[seg];
+    for (int j = 0; j < MOE_MAX_RANK / 4; ++j) lora[lr][4 * j + (tid & 3)] = lo[j];
+    __syncthreads();
+    float l[4][4] = {};
+    for (int k = 0; k < rank; ++k) {
+        const float* bp = x.lora_b + (size_t)k * H + n0 + 4 * tx;
+        const float4 u = __ldg(reinterpret_cast<const float4*>(bp));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float a = lora[ty * 4 + i][k];
+            l[i][0] = fmaf(a, u.x, l[i][0]); l[i][1] = fmaf(a, u.y, l[i][1]);
+            l[i][2] = fmaf(a, u.z, l[i][2]); l[i][3] = fmaf(a, u.w, l[i][3]);
+        }
+    }
+    dependency_wait();                         // the cached vectors of moe_stats_kernel
+    const float4 cv = *reinterpret_cast<const float4*>(w.cached + (size_t)seg * H + n0 + 4 * tx);
+    const float cc[4] = {cv.x, cv.y, cv.z, cv.w};
+    float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int t = m0 + ty * 4 + i;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float a = v[i][j] + l[i][j] * x.scale;
+            v[i][j] = (a < 0.f ? 0.f : a) + cc[j];
+            if (t < T) sum[j] += v[i][j];
+        }
+        if (t < T) *reinterpret_cast<float4*>(w.y + ((size_t)seg * T + t) * H + n0 + 4 * tx) = make_float4(v[i][0], v[i][1], v[i][2], v[i][3]);
+    }
+    float (*red)[MOE_PAD] = xs[0];             // every thread has passed the barrier behind the last k step
+    *reinterpret_cast<float4*>(&red[ty][4 * tx]) = make_float4(sum[0], sum[1], sum[2], sum[3]);
+    __syncthreads();
+    if (tid < MOE_TILE) {
+        float s = 0.f;
+        for (int i = 0; i < 16; ++i) s += red[i][tid];
+        w.ysum[((size_t)blockIdx.y * E + seg) * H + n0 + tid] = s;
+    }
+}
+
+__device__ __forceinline__ float moe_importance(const pikv_moe_params& p, const MoeWork& w, int t, int T) {
+    float s = 0.f;
+    for (int q = 0; q < p.H / (2 * MOE_TILE); ++q) s += w.part_pred[(size_t)q * T + t];
+    return 1.f / (1.f + expf(-(s + p.pred.b2[0])));
+}
+
+// softmax((sum of partial logits + b2) / temperature) over the first E lanes of a group of 16; the raw logit goes to `raw`
+__device__ __forceinline__ float moe_softmax(const pikv_moe_net& net, const float* part, int nt, int t, int e, int T, int E, float* raw) {
+    float l = -INFINITY;
+    if (e < E) {
+        float s = 0.f;
+        for (int q = 0; q < nt; ++q) s += part[((size_t)q * T + t) * E + e];
+        s += net.b2[e];
+        raw[(size_t)t * E + e] = s;
+        l = net.temperature == 1.f ? s : s / net.temperature;
+    }
+    // a NaN among the logits has to stay: fmaxf would drop it, the exponentials below bring it back
+    float m = l;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    const float x = e < E ? expf(l - m) : 0.f;
+    float d = x;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+    return x / d;
+}
+
+__global__ void __launch_bounds__(MOE_THREADS) moe_combine_kernel(const __grid_constant__ pikv_moe_params p, MoeWork w) {
+    __shared__ float rw[MOE_ROWS][PIKV_MOE_MAX_EXPERTS];
+    __shared__ float red[MOE_THREADS / 32];
+    const int H = p.H, E = p.E, T = p.B * p.S, tid = threadIdx.x;
+    dependency_wait();
+    if ((int)blockIdx.x < E) {                 // a cache: mean token, mean expert output, mean importance into its slot
+        const int e = blockIdx.x;
+        const pikv_moe_expert& x = p.expert[e];
+        const int mt = (T + MOE_TILE - 1) / MOE_TILE;
+        for (int h = tid; h < H; h += blockDim.x) {
+            float k = 0.f, v = 0.f;
+#pragma unroll 8
+            for (int b = 0; b < p.B; ++b) k += w.xsum[(size_t)b * H + h];
+#pragma unroll 8
+            for (int m = 0; m < mt; ++m) v += w.ysum[((size_t)m * E + e) * H + h];
+            x.keys[(size_t)x.slot * H + h] = k / (float)T;
+            x.values[(size_t)x.slot * H + h] = v / (float)T;
+        }
+        float s = 0.f;
+        for (int t = tid; t < T; t += blockDim.x) s += moe_importance(p, w, t, T);
+        s = warp_sum(s);
+        if ((tid & 31) == 0) red[tid >> 5] = s;
+        __syncthreads();
+        if (tid == 0) {
+            float a = 0.f;
+            for (int i = 0; i < MOE_THREADS / 32; ++i) a += red[i];
+            x.importance[x.slot] = a / (float)T;
+            p.cache_ptrs[e] = (x.slot + 1) % x.slots;
+        }
+        return;
+    }
+    const int t0 = (blockIdx.x - E) * MOE_ROWS;
+    if (tid < MOE_ROWS * 16) {                 // 16 lanes per token
+        const int i = tid >> 4, e = tid & 15, t = min(t0 + i, T - 1), nt = H / MOE_TILE;
+        const float a = moe_softmax(p.lb, w.part_lb, nt, t, e, T, E, p.logits_lb);
+        const float c = moe_softmax(p.imp, w.part_imp, nt, t, e, T, E, p.logits_imp) * moe_importance(p, w, t, T);
+        float d = c;
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+        const int b = t / p.S;
+        if (e < E) {
+            const float r = w.sel[2 * b] * a + w.sel[2 * b + 1] * (c / d);
+            rw[i][e] = r;
+            p.logits_mix[(size_t)t * E + e] = logf(r);
+        }
+    }
+    __syncthreads();
+    const int words = H / 4;
+    for (int i = tid; i < MOE_ROWS * words; i += blockDim.x) {
+        const int r = i / words, t = t0 + r, c = i % words;
+        if (t >= T) break;
+        float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+        for (int e = 0; e < E; ++e) {
+            const float4 y = *reinterpret_cast<const float4*>(w.y + ((size_t)e * T + t) * H + 4 * c);
+            const float f = rw[r][e];
+            o.x += y.x * f; o.y += y.y * f; o.z += y.z * f; o.w += y.w * f;
+        }
+        *reinterpret_cast<float4*>(p.out + (size_t)t * H + 4 * c) = o;
+    }
+}
+
+}  // namespace pikv
+
+using namespace pikv;
+
+extern "C" {
+
+size_t pikv_moe_workspace_bytes(int32_t B, int32_t S, int32_t H, int32_t E) {
+    if (B <= 0 || S <= 0 || H <= 0 || E <= 0) return 0;
+    return moe_layout(B, S, H, E, nullptr, nullptr);
+}
+
+int pikv_moe_forward(const pikv_moe_params* p, pikv_stream_t stream) {
+    PIKV_REQUIRE(p && p->x && p->out && p->logits_lb && p->logits_imp && p->logits_mix && p->cache_ptrs && p->workspace, PIKV_EINVAL,
+                 "moe_forward: null argument");
+    PIKV_REQUIRE(p->B > 0 && p->S > 0 && (int64_t)p->B * p->S <= (1 << 21), PIKV_ELIMIT, "moe_forward: %d x %d tokens", p->B, p->S);
+    PIKV_REQUIRE(p->H > 0 && p->H % 128 == 0 && p->H <= MOE_MAX_H, PIKV_EUNSUPPORTED, "moe_forward: width %d (a multiple of 128 up to %d)", p->H,
+                 MOE_MAX_H);
+    PIKV_REQUIRE(p->E > 0 && p->E <= PIKV_MOE_MAX_EXPERTS, PIKV_EUNSUPPORTED, "moe_forward: %d experts (up to %d)", p->E, PIKV_MOE_MAX_EXPERTS);
+    for (int e = 0; e < p->E; ++e) {
+        const pikv_moe_expert& x = p->expert[e];
+        PIKV_REQUIRE(x.rank >= 0 && x.rank <= MOE_MAX_RANK && x.v_rank >= 0 && x.v_rank <= MOE_MAX_RANK, PIKV_EUNSUPPORTED,
+                     "moe_forward: LoRA rank above %d", MOE_MAX_RANK);
+        PIKV_REQUIRE(x.mid > 0 && x.mid % 4 == 0 && x.mid <= MOE_MAX_H, PIKV_EUNSUPPORTED, "moe_forward: compressor width %d", x.mid);
+        PIKV_REQUIRE(x.slots > 0 && x.slot >= 0 && x.slot < x.slots, PIKV_EINVAL, "moe_forward: slot %d of %d", x.slot, x.slots);
+    }
+    MoeWork w;
+    const size_t need = moe_layout(p->B, p->S, p->H, p->E, static_cast<float*>(p->workspace), &w);
+    PIKV_REQUIRE(p->workspace_bytes >= need, PIKV_EINVAL, "moe_forward: workspace of %zu bytes, %zu needed", p->workspace_bytes, need);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const int T = p->B * p->S, mt = ceil_div(T, MOE_TILE), nt = p->H / MOE_TILE;
+    moe_stats_kernel<<<p->E + p->B, MOE_STATS_THREADS, 0, st>>>(*p, w);
+    launch_dependent(moe_gemm_kernel, dim3((unsigned)((p->E + 2) * nt + nt / 2), (unsigned)mt), MOE_THREADS, 0, st, *p, w);
+    launch_dependent(moe_combine_kernel, dim3((unsigned)(p->E + ceil_div(T, MOE_ROWS))), MOE_THREADS, 0, st, *p, w);
+    count_launch(3);
+    return check_launch("moe_forward");
+}
+
+}  // extern "C"

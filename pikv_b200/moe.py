@@ -1,8 +1,9 @@
 """PiKVMoE with the constructor, forward and state-dict keys of core/single/pikv_moe.py.
 
-The embedding, the LoRA experts and the vocabulary projection are plain torch modules (they are
-outside the routed KV-cache path); the router tail, the cache compressor and the H2O-scheduled cache
-manager run on the CUDA kernels.  Parameters are created in the reference's order, so a model built
+Without gradients the router nets, the LoRA experts, the caches' compressors and the ring update run as a few
+fused CUDA kernels behind one native call; under autograd, with hooks, a `query` or scheduled caches they run as the
+modules they are, whose router tails and cache managers are CUDA kernels.  The embedding and the vocabulary projection
+are torch modules.  Parameters are created in the reference's order, so a model built
 after torch.manual_seed(s) has the reference's weights for the same seed.
 """
 from __future__ import annotations
@@ -12,10 +13,14 @@ import math
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+from torch.autograd import forward_ad as _fwd_ad
+from torch.nn.modules import module as _module
 
+from ._lib import host
 from .config import config
-from .kv_cache_compression import KVCacheCompressor
-from .routing_strategy import AdaptiveRouter
+from .kv_cache_compression import KVCacheCompressor, PyramidCompression
+from .ops import GateResult
+from .routing_strategy import AdaptiveRouter, ImportanceAwareRouter, LoadBalancingRouter
 from .scheduling import CacheSchedulingManager, SchedulingPolicy
 
 
@@ -216,6 +221,27 @@ class PiKVMoE(nn.Module):
             except ValueError:
                 pass
 
+    def _fused(self, x):
+        """(weighted expert sum, auxiliary loss) by the fused kernels, or None where the modules have to run: the
+        kernels see neither tracers, function transforms and tangents nor hooks and replaced modules."""
+        if (torch.is_autocast_enabled() or _module._has_any_global_hook() or _fwd_ad._current_level >= 0 or torch.jit.is_tracing()
+                or torch._C._functorch.peek_interpreter_stack() is not None or torch._C._len_torch_dispatch_stack()
+                or torch.compiler.is_compiling()):
+            return None
+        if self._host_ptrs is None:
+            self._host_ptrs = self.cache_ptrs.tolist()
+        res = host().moe(self, x, self._host_ptrs, _FUSED_CLASSES)
+        if res is None:
+            return None
+        router = self.router
+        lb = router.load_balancing_router
+        lb.last_gate, router.importance_router.last_gate, router.last_gate = (GateResult(*r) for r in res[1:])
+
+        def loss():
+            usage = lb.last_gate.prob_sum / float(x.shape[0] * x.shape[1])
+            return lb.balance_weight * (usage.std() / usage.mean())
+        return res[0], loss
+
     def forward(self, x, query=None, return_loss=False, targets=None, use_teacher=False):
         if x.dim() == 2:
             x = self.embedding(x)
@@ -223,6 +249,12 @@ class PiKVMoE(nn.Module):
             raise ValueError(f"Input must be 2D (token IDs) or 3D (embeddings), got shape: {x.shape}")
         if x.dtype != torch.float32:
             x = x.to(torch.float32)
+        if query is None and not self.use_cache_scheduling and not torch.is_grad_enabled():
+            fused = self._fused(x)
+            if fused is not None:
+                out, lb_loss = fused
+                logits = self.vocab_proj(out)
+                return (logits, lb_loss()) if return_loss else logits
         routing_weights, expert_indices, top_k_weights, lb_loss, importance = self.router(x)
         if query is not None:
             importance = self.compute_token_importance(query.to(torch.float32), x)
@@ -238,3 +270,8 @@ class PiKVMoE(nn.Module):
         if return_loss:
             return logits, lb_loss
         return logits
+
+
+# the classes the fused forward stands for, in the order of MoeWalk in csrc/host/host.cpp
+_FUSED_CLASSES = (PiKVMoE, nn.ModuleList, LoRAExpert, LoRALayer, nn.Linear, nn.Dropout, KVCache, KVCacheCompressor, PyramidCompression,
+                  AdaptiveRouter, LoadBalancingRouter, ImportanceAwareRouter, nn.Sequential, nn.ReLU, nn.Sigmoid, nn.Softmax)
