@@ -124,6 +124,9 @@ size_t pikv_gate_workspace_bytes(int32_t T, int32_t E, int32_t top_k);
 /* what pikv_gate_fused and pikv_route_append need of it (no partial logits of the two-layer net) */
 size_t pikv_gate_tail_workspace_bytes(int32_t T, int32_t E, int32_t top_k);
 int    pikv_gate_fused(const pikv_gate_params* p, pikv_stream_t stream);
+/* up to four gates on given logits in one launch (host array of parameter blocks that share T and E and
+ * have a workspace each); every other field as in pikv_gate_fused */
+int pikv_gate_logits(const pikv_gate_params* const* p, int32_t n, pikv_stream_t stream);
 /* bf16 activations run on the tcgen05 kernel (TMA + tensor memory), fp32 ones on the SIMT
  * kernel.  Reads and clears the tensor-core kernel's sticky error word (non-zero: a bounded
  * mbarrier wait ran out and the outputs are invalid); waits for the work queued before it. */
@@ -650,7 +653,7 @@ int pikv_a2a_unpack(const void* recv_buf, int32_t n_records, int32_t n_kv,
                     uint32_t* status, pikv_stream_t stream);
 
 /* ------------------------------------------------------------------------
- * PiKVMoE inference forward up to the vocabulary projection, fp32
+ * PiKVMoE inference forward, fp32, with the vocabulary projection where pikv_linear_f32 takes its width
  * (core/single/pikv_moe.py:277-336, core/single/routing_strategy.py:100-150).
  *   out[t] = sum_e r[t,e] (relu(dense_e(x[t]) + lora_e(x[t])) + cached_e), r the adaptive router's
  *   weights, cached_e the mean of the importance-weighted value rows behind compressor and value LoRA;
@@ -682,11 +685,23 @@ typedef struct {
     int64_t* cache_ptrs;
     float *logits_lb, *logits_imp, *logits_mix;
     float* out;                                       /* [B,S,H] */
-    void* workspace;
+    const float *vocab_w, *vocab_b;                   /* [V,H], [V]; V = 0: no projection */
+    float* vocab_out;                                 /* [B,S,V] = pikv_linear_f32(out) */
+    int32_t V;
+    void* workspace;                                  /* 256-byte aligned */
     size_t workspace_bytes;
 } pikv_moe_params;
-size_t pikv_moe_workspace_bytes(int32_t B, int32_t S, int32_t H, int32_t E);
+size_t pikv_moe_workspace_bytes(int32_t B, int32_t S, int32_t H, int32_t E, int32_t V);
 int pikv_moe_forward(const pikv_moe_params* p, pikv_stream_t stream);
+
+/* ------------------------------------------------------------------------
+ * fp32 linear layer out[M,N] = x[M,K] . w[N,K]^T + bias (bias may be NULL), on the tensor cores with every
+ * operand as two f16 limbs: the error of an fp32 sum or less.  K a multiple of 64 up to 256, any N; x and w
+ * 16-byte, workspace 256-byte aligned.  PiKVMoE's vocabulary projection, core/single/pikv_moe.py:334.
+ * ---------------------------------------------------------------------- */
+size_t pikv_linear_f32_workspace_bytes(int32_t M, int32_t N, int32_t K);
+int pikv_linear_f32(const float* x, const float* w, const float* bias, float* out, int32_t M, int32_t N, int32_t K,
+                    void* workspace, size_t workspace_bytes, pikv_stream_t stream);
 
 #ifdef __cplusplus
 }

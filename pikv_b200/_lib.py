@@ -190,8 +190,11 @@ SIGNATURES = {
     "pikv_lowrank_pair": (i32, [C.POINTER(vp), C.POINTER(vp), C.POINTER(vp), C.POINTER(vp), C.POINTER(vp), i32, C.POINTER(vp),
                                 i32, i32, i32, i32, vp]),
     "pikv_lowrank_error_state": (i32, []),
-    "pikv_moe_workspace_bytes": (sz, [i32, i32, i32, i32]),
+    "pikv_linear_f32_workspace_bytes": (sz, [i32, i32, i32]),
+    "pikv_linear_f32": (i32, [vp, vp, vp, vp, i32, i32, i32, vp, sz, vp]),
+    "pikv_moe_workspace_bytes": (sz, [i32, i32, i32, i32, i32]),
     "pikv_moe_forward": (i32, [vp, vp]),
+    "pikv_gate_logits": (i32, [vp, i32, vp]),
     "pikv_a2a_record_bytes": (sz, [i32]),
     "pikv_a2a_pack": (i32, [vp, vp, i32, i32, i32, i32, vp, vp, vp, vp, vp, vp]),
     "pikv_a2a_unpack": (i32, [vp, i32, i32, vp, i32, i32, i32, i32, i32, vp, vp, i32, vp, vp, vp, vp, vp, vp]),

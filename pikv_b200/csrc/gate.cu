@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(GATE_THREADS) gate_act_kernel(GateDev g) {
 
 // ---- gate from precomputed logits: one thread per token ---------------------------
 template <int EP>
-__global__ void __launch_bounds__(GATE_THREADS) gate_logits_kernel(GateDev g) {
+__device__ __forceinline__ void gate_logits_tokens(const GateDev& g) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     int* warp_cnt = reinterpret_cast<int*>(smem_raw);
     int* run = warp_cnt + GATE_WARPS * EP;
@@ -492,12 +492,24 @@ gate_cluster_kernel(GateDev g, const float* part, int groups, const void* b2, bo
     }
     cluster.sync();                                   // nobody reads this CTA's counters any more
 }
+template <int EP>
+__global__ void __launch_bounds__(GATE_THREADS) gate_logits_kernel(GateDev g) { gate_logits_tokens<EP>(g); }
+
+// Several gates of one batch: a kernel of a few microseconds each, in one launch (grid y = gate).
+struct GateDevs {
+    GateDev g[GATE_MAX_BATCH];
+};
+template <int EP>
+__global__ void __launch_bounds__(GATE_THREADS) gate_logits_batch_kernel(const __grid_constant__ GateDevs b) {
+    dependency_wait();
+    gate_logits_tokens<EP>(b.g[blockIdx.y]);
+}
 
 // ---- finalize: local ranks -> global slots; totals --------------------------------
 // Threads are laid out as (expert e, part): part p sums the per-CTA counters of CTAs p, p+parts, ...
 // so the reads of one prefix are spread over 256/EP2 threads and overlap; parts are combined in a
 // fixed order (the float sums stay run-to-run identical).
-__global__ void __launch_bounds__(GATE_THREADS) gate_finalize_kernel(GateDev g) {
+__device__ __forceinline__ void gate_finalize(const GateDev& g) {
     __shared__ int base_s[GATE_MAX_E];
     __shared__ int part_i[GATE_THREADS];
     __shared__ float part_f[GATE_THREADS];
@@ -555,6 +567,9 @@ __global__ void __launch_bounds__(GATE_THREADS) gate_finalize_kernel(GateDev g) 
     }
 }
 
+__global__ void __launch_bounds__(GATE_THREADS) gate_finalize_kernel(GateDev g) { gate_finalize(g); }
+__global__ void __launch_bounds__(GATE_THREADS) gate_finalize_batch_kernel(const __grid_constant__ GateDevs b) { gate_finalize(b.g[blockIdx.y]); }
+
 // ---- dense dispatch / combine ------------------------------------------------------
 __global__ void dispatch_scatter_kernel(const int* topk_idx, const float* topk_w, const int* slot, const int* counts_k,
                                         const float* prob_sum, int T, int E, int k, pikv_dense_out d) {
@@ -609,6 +624,17 @@ static int dispatch_launch(const int* topk_idx, const float* topk_w, const int* 
     count_launch(1);
     return launch_tail("dispatch_scatter_kernel", dispatch_scatter_kernel, ceil_div(T * k, GATE_THREADS), 0, st, topk_idx, topk_w,
                             slot, counts_k, prob_sum, T, E, k, d);
+}
+
+template <int EP>
+static int launch_batch(const GateDevs& b, int n, int k, cudaStream_t st) {
+    const size_t smem = sizeof(int) * (GATE_WARPS * EP + EP + GATE_MAX_K * EP) + sizeof(float) * GATE_WARPS * EP + (size_t)b.g[0].chunk * k;
+    if (smem > 48 * 1024 && !allow_smem<gate_logits_batch_kernel<EP>>()) return check_launch("gate_logits smem attribute");
+    const dim3 grid((unsigned)b.g[0].G, (unsigned)n);
+    launch_dependent(gate_logits_batch_kernel<EP>, grid, GATE_THREADS, smem, st, b);
+    launch_dependent(gate_finalize_batch_kernel, grid, GATE_THREADS, 0, st, b);
+    count_launch(2);
+    return check_launch("gate_logits_batch_kernel");
 }
 
 template <int EP>
@@ -739,6 +765,25 @@ extern "C" int pikv_gate_fused(const pikv_gate_params* p, pikv_stream_t stream) 
     const int what = phase == PIKV_GATE_SCORE ? GATE_DO_SCORE : phase == PIKV_GATE_SLOTS ? GATE_DO_SLOTS
                                                                                         : (GATE_DO_SCORE | GATE_DO_SLOTS);
     return gate_run(p, static_cast<cudaStream_t>(stream), what, nullptr);
+}
+
+extern "C" int pikv_gate_logits(const pikv_gate_params* const* p, int32_t n, pikv_stream_t stream) {
+    PIKV_REQUIRE(p != nullptr && n > 0 && n <= GATE_MAX_BATCH, PIKV_EINVAL, "gate_logits: %d gates (1 to %d)", n, GATE_MAX_BATCH);
+    GateDevs b = {};
+    int k = 0;
+    for (int i = 0; i < n; ++i) {
+        PIKV_REQUIRE(p[i] && p[i]->logits_in && p[i]->T == p[0]->T && p[i]->E == p[0]->E, PIKV_EINVAL, "gate_logits: the gates share T and E");
+        const int rc = gate_run(p[i], nullptr, 0, &b.g[i]);
+        if (rc != PIKV_OK) return rc;
+        k = max(k, p[i]->top_k);
+    }
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const int E = p[0]->E;
+    if (E <= 4) return launch_batch<4>(b, n, k, st);
+    if (E <= 8) return launch_batch<8>(b, n, k, st);
+    if (E <= 16) return launch_batch<16>(b, n, k, st);
+    if (E <= 32) return launch_batch<32>(b, n, k, st);
+    return launch_batch<64>(b, n, k, st);
 }
 
 extern "C" int pikv_dispatch_loss(const int32_t* topk_idx, const float* topk_w, const int32_t* slot,

@@ -8,6 +8,7 @@ namespace pikv {
 constexpr int GATE_THREADS = 256;
 constexpr int GATE_WARPS = GATE_THREADS / 32;
 constexpr int GATE_MAX_CTAS = 1024;
+constexpr int GATE_MAX_BATCH = 4;              // gates of one pikv_gate_logits call
 constexpr int GATE_MAX_CHUNK = 4096;   // tokens per CTA
 constexpr int GATE_MAX_K = 8;
 constexpr int GATE_MAX_E = 64;

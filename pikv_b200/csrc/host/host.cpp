@@ -573,6 +573,21 @@ PyObject* lowrank_pair(PyObject* const* a, Py_ssize_t) {
     return tuple(y[0], y[1]);
 }
 
+// linear_f32(x, w, bias) -> [..., N]
+at::Tensor linear_f32(const at::Tensor& x, const at::Tensor& w, const float* bias) {
+    const int K = (int)x.size(-1), N = (int)w.size(0), M = (int)(x.numel() / K);
+    at::Tensor y = at::empty(with_last(x, N), on(x, at::kFloat));
+    const size_t bytes = pikv_linear_f32_workspace_bytes(M, N, K);
+    const at::Tensor ws = workspace(x, bytes);
+    check(pikv_linear_f32(ptr<float>(x), ptr<float>(w), bias, ptr<float>(y), M, N, K, ptr(ws), bytes, stream()), "pikv_linear_f32");
+    return y;
+}
+PyObject* linear(PyObject* const* a, Py_ssize_t) {
+    const at::Tensor x = req(a[0], "x", at::kFloat), w = req(a[1], "w", at::kFloat), b = opt(a[2], "bias", at::kFloat);
+    if (x.dim() < 1 || w.dim() != 2 || w.size(1) != x.size(-1) || (b.defined() && b.numel() != w.size(0))) fail("linear_f32: x, w and bias do not fit");
+    return wrap(linear_f32(x, w, ptr<float>(b)));
+}
+
 // ---- PiKVMoE -----------------------------------------------------------------------------------------------
 // The forward's kernels take raw weights, so every module they stand for has to be what it was built as: walked on each
 // call, about 70 modules in a few microseconds.  Whatever does not fit leaves as NotApplicable and the caller runs the modules.
@@ -693,7 +708,7 @@ struct MoeWalk {
     }
 };
 
-// moe(module, x, ring positions, classes) -> (weighted expert sum, three gate results), or None where the modules have to run
+// moe(module, x, ring positions, classes) -> (weighted expert sum, logits or None, three gate results), or None where the modules have to run
 PyObject* moe(PyObject* const* a, Py_ssize_t) {
     PyObject *positions = a[2], *types = a[3];
     if (!THPVariable_CheckExact(a[1])) Py_RETURN_NONE;
@@ -773,17 +788,33 @@ PyObject* moe(PyObject* const* a, Py_ssize_t) {
         Py_RETURN_NONE;
     }
     const int T = p.B * p.S, E = p.E;
-    at::Tensor out = at::empty_like(x);
-    p.workspace_bytes = pikv_moe_workspace_bytes(p.B, p.S, p.H, E);
-    const size_t row = ((size_t)T * E * 4 + 255) & ~size_t(255), tail = pikv_gate_tail_workspace_bytes(T, E, std::max(topk[0], std::max(topk[1], topk[2])));
-    const at::Tensor ws = workspace(x, p.workspace_bytes + 3 * row + 256 + tail);
+    at::Tensor out = at::empty_like(x), logits;
+    // The vocabulary projection, unless it is hooked or of another kind, or has few rows: up to 32 of them read w once
+    // whichever way, and splitting w first costs more (256 -> 50257: 32 rows 36 us split, 34 as a plain layer; 64: 36, 58).
+    if (T > 32 && p.H <= 256) {
+        try {
+            const Mod m(a[0], types, W::MOE), v(m.child(PIKV_NAME("vocab_proj")), types, W::LINEAR);
+            const long V = v.integer(PIKV_NAME("out_features"));
+            need(V > 0 && V <= (1 << 24));
+            walk.linear(m.child(PIKV_NAME("vocab_proj")), V, p.H, p.vocab_w, p.vocab_b);
+            logits = at::empty({p.B, p.S, V}, on(x, at::kFloat));
+            p.vocab_out = ptr<float>(logits);
+            p.V = (int32_t)V;
+        } catch (const NotApplicable&) {
+        }
+    }
+    p.workspace_bytes = pikv_moe_workspace_bytes(p.B, p.S, p.H, E, p.V);
+    const size_t row = ((size_t)T * E * 4 + 255) & ~size_t(255);
+    size_t tail[3], total = ((p.workspace_bytes + 255) & ~size_t(255)) + 3 * row;
+    for (int i = 0; i < 3; ++i) total += tail[i] = (pikv_gate_tail_workspace_bytes(T, E, topk[i]) + 255) & ~size_t(255);
+    const at::Tensor ws = workspace(x, total);
     char* base = ptr<char>(ws);
     p.workspace = base;
     base += (p.workspace_bytes + 255) & ~size_t(255);
-    float* logits[3];
-    for (int i = 0; i < 3; ++i, base += row) logits[i] = reinterpret_cast<float*>(base);
+    float* raw[3];
+    for (int i = 0; i < 3; ++i, base += row) raw[i] = reinterpret_cast<float*>(base);
     p.x = ptr<float>(x); p.out = ptr<float>(out);
-    p.logits_lb = logits[0]; p.logits_imp = logits[1]; p.logits_mix = logits[2];
+    p.logits_lb = raw[0]; p.logits_imp = raw[1]; p.logits_mix = raw[2];
     check(pikv_moe_forward(&p, stream()), "pikv_moe_forward");
     for (int i = 0; i < n_touched; ++i)
         if (!touched[i].is_inference()) touched[i].unsafeGetTensorImpl()->bump_version();
@@ -791,22 +822,24 @@ PyObject* moe(PyObject* const* a, Py_ssize_t) {
         PyObject* next = PyLong_FromLong((p.expert[e].slot + 1) % p.expert[e].slots);
         if (!next || PyList_SetItem(positions, e, next)) throw Raised();
     }
-    PyObject* result = PyTuple_New(4);
+    pikv_gate_params g[3] = {};
+    const pikv_gate_params* list[3] = {&g[0], &g[1], &g[2]};
+    std::vector<GateOut> results;
+    results.reserve(3);
+    for (int i = 0; i < 3; ++i) {
+        g[i].T = T; g[i].E = E; g[i].top_k = topk[i]; g[i].dtype = PIKV_F32; g[i].logits_in = raw[i];
+        g[i].mask_mode = PIKV_MASK_NONE; g[i].temperature = i < 2 ? temperature[i] : 1.f;
+        results.emplace_back(Py_None, x, T, E, topk[i], i < 2);
+        results[i].fill(g[i]);
+        g[i].workspace = base; g[i].workspace_bytes = tail[i];
+        base += tail[i];
+    }
+    check(pikv_gate_logits(list, 3, stream()), "pikv_gate_logits");
+    PyObject* result = PyTuple_New(5);
     if (!result) throw Raised();
     PyTuple_SET_ITEM(result, 0, wrap(out));
-    for (int i = 0; i < 3; ++i) {
-        pikv_gate_params g = {};
-        g.T = T; g.E = E; g.top_k = topk[i]; g.dtype = PIKV_F32; g.logits_in = logits[i];
-        g.mask_mode = PIKV_MASK_NONE; g.temperature = i < 2 ? temperature[i] : 1.f;
-        GateOut o(Py_None, x, T, E, g.top_k, i < 2);
-        o.fill(g);
-        g.workspace = base; g.workspace_bytes = tail;
-        if (int rc = pikv_gate_fused(&g, stream())) {
-            Py_DECREF(result);
-            check(rc, "pikv_gate_fused");
-        }
-        PyTuple_SET_ITEM(result, 1 + i, o.result());
-    }
+    PyTuple_SET_ITEM(result, 1, wrap(logits));
+    for (int i = 0; i < 3; ++i) PyTuple_SET_ITEM(result, 2 + i, results[i].result());
     return result;
 }
 
@@ -845,6 +878,7 @@ PyMethodDef methods[] = {
     method<quant_pair, 9>("quant_pair"),
     method<lowrank, 6>("lowrank"),
     method<lowrank_pair, 10>("lowrank_pair"),
+    method<linear, 3>("linear_f32"),
     method<moe, 4>("moe"),
     {nullptr, nullptr, 0, nullptr},
 };

@@ -1,0 +1,334 @@
+// fp32 linear layer on the tensor cores: out[M,N] = x[M,K] . w[N,K]^T + bias, every operand as two f16 limbs.
+//
+// A row is scaled by a power of two so that its largest magnitude lies in [2^14, 2^15) and split into hi = f16(v) and
+// lo = f16(v - hi): v is met to 2^-24 of itself (2^-38 of the row's largest where lo is subnormal).  The product is
+// hi.hi + (hi.lo + lo.hi), what is left out, lo.lo, is below 2^-24 of each term.  The tensor cores' sums truncate, so
+// each bracket has an fp32 accumulator of its own and each half of K another pair; the epilogue adds the four.
+// Rows with an infinity, a NaN or a largest magnitude outside 2^-60 .. 2^60 are marked (scale 0) and their outputs formed
+// by plain fp32 sums in the epilogue.
+//
+//   lin_split_kernel   one warp per row of w and x: limbs [rows, hi K | lo K] and the inverse scales
+//   lin_gemm_kernel    persistent, one CTA per SM.  Items are 128 x 128 outputs, row tiles innermost, contiguous per CTA:
+//                      w's tile stays in shared memory (hi and lo of a 64-wide k block next to each other: one MMA of
+//                      N = 256 takes both products of an x hi block), x blocks stream through a ring.  Two accumulator
+//                      pairs of 256 columns, one per half of K: eight epilogue warps keep the first half's sums in
+//                      registers while the second is computed, turn 32 x 32 patches in shared memory and store whole rows (N is odd in earnest, so neither TMA nor vector stores apply).
+//
+// 1024 x 256 -> 50257: 115 us for the GEMM and 26 for the splits (140 us a call; cuBLAS's fp32 kernel and its bias pass 716),
+// relative error 2.0e-7 against 64 bits (cuBLAS 2.9e-7; one accumulator for all of K 3.5e-7).  The 79 GFLOP of the three
+// products would take 48 us at the measured bf16 rate and the output 32 us of HBM.
+#include "tc_common.cuh"
+
+namespace pikv {
+
+constexpr int LIN_BN = 128, LIN_BLOCK = 128 * 128;       // outputs per tile; bytes of a [128 x 64] f16 block
+constexpr int LIN_MAX_KB = 4, LIN_STAGES = 4;
+constexpr int LIN_EPI_WARPS = 8, LIN_THREADS = 64 + 32 * LIN_EPI_WARPS;
+constexpr int LIN_PATCH = 32 * 33 * 4;
+constexpr int LIN_SMEM = 2 * LIN_MAX_KB * LIN_BLOCK + LIN_STAGES * LIN_BLOCK + LIN_EPI_WARPS * LIN_PATCH + 256 + 1024;
+static_assert(LIN_SMEM <= 227 * 1024, "linear_f32: shared memory");
+
+__device__ unsigned g_linear_error = 0;                  // sticky: set when a bounded wait ran out
+
+struct LinArgs {
+    const float *x, *w, *bias, *sx, *sw;
+    float* out;
+    int M, N, K, mtiles;
+    long long items;
+};
+
+__global__ void __launch_bounds__(256) lin_split_kernel(const float* __restrict__ src, int rows, int K, __half* __restrict__ limbs, float* __restrict__ inv) {
+    dependency_release();
+    dependency_wait();
+    const int lane = threadIdx.x & 31;
+    const int words = K / 4;                             // at most 64: two per lane
+    for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows; r += gridDim.x * blockDim.x / 32) {
+        float4 v[2] = {};
+        float m = 0.f;
+        bool bad = false;
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int i = lane + 32 * q;
+            if (i < words) v[q] = *reinterpret_cast<const float4*>(src + (size_t)r * K + 4 * i);
+            const float a[4] = {fabsf(v[q].x), fabsf(v[q].y), fabsf(v[q].z), fabsf(v[q].w)};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                m = fmaxf(m, a[j]);
+                bad |= !(a[j] <= 3.402823466e38f);
+            }
+        }
+        m = warp_max(m);
+        const int e = (int)(__float_as_uint(m) >> 23) - 127;           // 2^e <= m < 2^(e+1)
+        bad = __any_sync(0xffffffffu, bad) || e > 60 || (e < -60 && m != 0.f);
+        const float up = bad ? 0.f : m == 0.f ? 1.f : __uint_as_float((uint32_t)(127 + 14 - e) << 23);
+        if (lane == 0) inv[r] = bad ? 0.f : m == 0.f ? 1.f : __uint_as_float((uint32_t)(127 - 14 + e) << 23);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int i = lane + 32 * q;
+            if (i >= words) continue;
+            const float a[4] = {v[q].x, v[q].y, v[q].z, v[q].w};
+            __align__(8) __half h[4], l[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float s = bad ? 0.f : a[j] * up;
+                h[j] = __float2half_rn(s);
+                l[j] = __float2half_rn(s - __half2float(h[j]));
+            }
+            __half* to = limbs + (size_t)r * 2 * K + 4 * i;
+            *reinterpret_cast<uint2*>(to) = *reinterpret_cast<const uint2*>(h);
+            *reinterpret_cast<uint2*>(to + K) = *reinterpret_cast<const uint2*>(l);
+        }
+    }
+}
+
+__device__ __noinline__ float lin_plain(const LinArgs& a, int m, int n) {
+    float s = 0.f;
+    for (int k = 0; k < a.K; ++k) s = fmaf(a.x[(size_t)m * a.K + k], a.w[(size_t)n * a.K + k], s);
+    return s;
+}
+
+__global__ void __launch_bounds__(LIN_THREADS, 1) lin_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w,
+                                                                  const __grid_constant__ LinArgs a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    unsigned char* smem = smem_raw + ((1024u - (lr_smem_u32(smem_raw) & 1023u)) & 1023u);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, kbs = a.K / 64;
+    unsigned char* ring_p = smem + 2 * LIN_MAX_KB * LIN_BLOCK;
+    float* patches = reinterpret_cast<float*>(ring_p + LIN_STAGES * LIN_BLOCK);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(patches + LIN_EPI_WARPS * LIN_PATCH / 4);
+    const uint32_t wt = lr_smem_u32(smem), ring = lr_smem_u32(ring_p);
+    const uint32_t full0 = lr_smem_u32(bars), empty0 = full0 + 8 * LIN_STAGES, wfull0 = empty0 + 8 * LIN_STAGES, wempty0 = wfull0 + 8 * LIN_MAX_KB,
+                   tfull0 = wempty0 + 8 * LIN_MAX_KB, tempty0 = tfull0 + 16;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * LIN_STAGES + 2 * LIN_MAX_KB + 4);
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < 2 * LIN_STAGES + 2 * LIN_MAX_KB + 2; ++s) lr_mbar_init(full0 + 8 * s, 1);
+        for (int s = 0; s < 2; ++s) lr_mbar_init(tempty0 + 8 * s, 32 * LIN_EPI_WARPS);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        lr_prefetch_tmap(&tm_x);
+        lr_prefetch_tmap(&tm_w);
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(lr_smem_u32(tmem_slot)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem_base = *tmem_slot;
+    dependency_wait();
+    const long long first = a.items * blockIdx.x / gridDim.x, last = a.items * (blockIdx.x + 1) / gridDim.x;
+    const int first_kbs = (kbs + 1) / 2;                 // k blocks of the first half
+    bool failed = false;
+
+    if (warp == 0) {
+        LrRing r;
+        uint32_t wph = 1;                                // parity of w's free barriers: the first tile finds them free
+        int held = -1;
+        for (long long item = first; item < last && !failed; ++item) {
+            const int nt = (int)(item / a.mtiles), mt = (int)(item % a.mtiles);
+            const bool load_w = nt != held;
+            for (int kb = 0; kb < kbs && !failed; ++kb) {
+                if (load_w) {
+                    if (!lr_mbar_wait(wempty0 + 8 * kb, wph)) { failed = true; break; }
+                    if (lr_elect()) {
+                        lr_mbar_expect_tx(wfull0 + 8 * kb, 2 * LIN_BLOCK);
+                        lr_tma_load_2d(wt + (uint32_t)(2 * kb) * LIN_BLOCK, &tm_w, kb * 64, nt * LIN_BN, wfull0 + 8 * kb);
+                        lr_tma_load_2d(wt + (uint32_t)(2 * kb + 1) * LIN_BLOCK, &tm_w, a.K + kb * 64, nt * LIN_BN, wfull0 + 8 * kb);
+                    }
+                    __syncwarp();
+                }
+                for (int limb = 0; limb < 2; ++limb, r.next(LIN_STAGES)) {
+                    if (!lr_mbar_wait(empty0 + 8 * r.s, r.ph ^ 1u)) { failed = true; break; }
+                    if (lr_elect()) {
+                        lr_mbar_expect_tx(full0 + 8 * r.s, LIN_BLOCK);
+                        lr_tma_load_2d(ring + (uint32_t)r.s * LIN_BLOCK, &tm_x, limb * a.K + kb * 64, mt * 128, full0 + 8 * r.s);
+                    }
+                    __syncwarp();
+                }
+            }
+            if (load_w) {
+                held = nt;
+                wph ^= 1u;
+            }
+        }
+    } else if (warp == 1) {
+        // f16 operands: the instruction descriptor without the bf16 format bits
+        constexpr uint32_t id = (1u << 4) | (8u << 24), wide = id | (256u >> 3) << 17, narrow = id | (128u >> 3) << 17;
+        LrRing r;
+        uint32_t wph = 0;
+        int held = -1, local = 0;
+        for (long long item = first; item < last && !failed; ++item, ++local) {
+            const int nt = (int)(item / a.mtiles);
+            const bool fresh = nt != held, leaves = item + 1 == last || (int)((item + 1) / a.mtiles) != nt;
+            for (int kb = 0; kb < kbs && !failed; ++kb) {
+                const int half = kb >= first_kbs;
+                const uint32_t d = tmem_base + (uint32_t)(half * 256);
+                const bool opens = kb == 0 || kb == first_kbs;
+                if (opens && !lr_mbar_wait(tempty0 + 8 * half, ((uint32_t)local & 1u) ^ 1u)) { failed = true; break; }
+                if (fresh && !lr_mbar_wait(wfull0 + 8 * kb, wph)) { failed = true; break; }
+                const uint32_t b_lo = lr_desc_lo(wt) + (uint32_t)(2 * kb) * (LIN_BLOCK >> 4);
+                for (int limb = 0; limb < 2; ++limb, r.next(LIN_STAGES)) {
+                    if (!lr_mbar_wait(full0 + 8 * r.s, r.ph)) { failed = true; break; }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    if (lr_elect()) {
+                        const uint32_t a_lo = lr_desc_lo(ring) + (uint32_t)r.s * (LIN_BLOCK >> 4);
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            if (limb == 0) lr_mma(d, lr_desc(a_lo + 2 * k), lr_desc(b_lo + 2 * k), wide, opens && k == 0 ? 0u : 1u);
+                            else lr_mma(d + 128, lr_desc(a_lo + 2 * k), lr_desc(b_lo + 2 * k), narrow, 1u);
+                        }
+                        lr_commit(empty0 + 8 * r.s);
+                        if (leaves && limb) lr_commit(wempty0 + 8 * kb);
+                        if (limb && (kb + 1 == first_kbs || kb + 1 == kbs)) lr_commit(tfull0 + 8 * half);
+                    }
+                    __syncwarp();
+                }
+            }
+            if (fresh) {
+                held = nt;
+                wph ^= 1u;
+            }
+        }
+    } else {
+        const int lg = warp & 3, side = (warp - 2) >> 2; // tensor-memory lane group, and which 64 of the 128 columns
+        float* patch = patches + (size_t)(warp - 2) * (LIN_PATCH / 4);
+        int local = 0;
+        for (long long item = first; item < last && !failed; ++item, ++local) {
+            const int nt = (int)(item / a.mtiles), mt = (int)(item % a.mtiles);
+            const int m0 = mt * 128 + lg * 32, n0 = nt * LIN_BN + side * 64;
+            const float sx = m0 + lane < a.M ? a.sx[m0 + lane] : 1.f;
+            const int rows = min(32, a.M - m0);
+            const uint32_t taddr = tmem_base + ((uint32_t)(lg * 32) << 16) + (uint32_t)(side * 64);
+            float acc[2][32] = {};
+            if (kbs > first_kbs) {
+                if (!lr_mbar_wait(tfull0, (uint32_t)local & 1u)) { failed = true; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    float u[32];
+                    lr_tmem_ld32(taddr + 32 * c, acc[c]);
+                    lr_tmem_ld32(taddr + 128 + 32 * c, u);
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) acc[c][i] += u[i];
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                lr_mbar_arrive(tempty0);
+            }
+            const int half = kbs > first_kbs;
+            if (!lr_mbar_wait(tfull0 + 8 * half, (uint32_t)local & 1u)) { failed = true; break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                float v[32];
+                lr_tmem_ld32(taddr + half * 256 + 128 + 32 * c, v);
+#pragma unroll
+                for (int i = 0; i < 32; ++i) acc[c][i] += v[i];
+                lr_tmem_ld32(taddr + half * 256 + 32 * c, v);
+#pragma unroll
+                for (int i = 0; i < 32; ++i) acc[c][i] += v[i];
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            lr_mbar_arrive(tempty0 + 8 * half);
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+#pragma unroll
+                for (int i = 0; i < 32; ++i) patch[lane * 33 + i] = acc[c][i];
+                __syncwarp();
+                const int n = n0 + 32 * c + lane;
+                const bool in = n < a.N;
+                const float sw = in ? a.sw[n] : 1.f, bias = in && a.bias ? a.bias[n] : 0.f;
+                float* to = a.out + (size_t)m0 * a.N + n;
+                const bool marked = __any_sync(0xffffffffu, sx == 0.f || sw == 0.f);
+                if (!marked && rows == 32) {
+#pragma unroll
+                    for (int r = 0; r < 32; ++r) {
+                        const float o = patch[r * 33 + lane] * __shfl_sync(0xffffffffu, sx, r) * sw + bias;
+                        if (in) to[(size_t)r * a.N] = o;
+                    }
+                } else {
+                    for (int r = 0; r < rows; ++r) {
+                        const float s = __shfl_sync(0xffffffffu, sx, r);
+                        if (!in) continue;
+                        const float o = s == 0.f || sw == 0.f ? lin_plain(a, m0 + r, n) : patch[r * 33 + lane] * s * sw;
+                        to[(size_t)r * a.N] = o + bias;
+                    }
+                }
+                __syncwarp();
+            }
+        }
+    }
+    if (failed) atomicOr(&g_linear_error, 1u);
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+}
+
+int linear_error_fetch() {
+    unsigned v = 0, zero = 0;
+    if (cudaMemcpyFromSymbol(&v, g_linear_error, sizeof(v)) != cudaSuccess) return -1;
+    if (v) cudaMemcpyToSymbol(g_linear_error, &zero, sizeof(zero));
+    return (int)v;
+}
+
+// workspace: limbs and inverse scales of w, then those of x
+static size_t lin_limbs(int64_t rows, int K) { return (size_t)rows * 2 * K * 2; }
+static size_t lin_scales(int64_t rows) { return ((size_t)rows * 4 + 255) & ~size_t(255); }
+
+bool linear_f32_supported(int K) { return K > 0 && K % 64 == 0 && K <= 64 * LIN_MAX_KB; }
+
+// w's half of the work, which needs nothing but w; the next kernel may start beside it
+int linear_f32_weights(const float* w, int N, int K, void* workspace, cudaStream_t st) {
+    char* p = static_cast<char*>(workspace);
+    lin_split_kernel<<<min(ceil_div(N, 8), 8 * sm_count()), 256, 0, st>>>(w, N, K, reinterpret_cast<__half*>(p),
+                                                                         reinterpret_cast<float*>(p + lin_limbs(N, K)));
+    count_launch(1);
+    return check_launch("lin_split_kernel");
+}
+
+// the rest, behind a kernel that itself has waited for linear_f32_weights
+int linear_f32_rows(const float* x, const float* w, const float* bias, float* out, int M, int N, int K, void* workspace, cudaStream_t st) {
+    char* p = static_cast<char*>(workspace);
+    __half* wl = reinterpret_cast<__half*>(p);
+    float* sw = reinterpret_cast<float*>(p += lin_limbs(N, K));
+    __half* xl = reinterpret_cast<__half*>(p += lin_scales(N));
+    float* sx = reinterpret_cast<float*>(p + lin_limbs(M, K));
+    CUtensorMap tm_x, tm_w;
+    int rc = make_tmap_of(&tm_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, xl, M, 2 * K, 128);
+    if (rc == PIKV_OK) rc = make_tmap_of(&tm_w, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, wl, N, 2 * K, 128);
+    if (rc != PIKV_OK) return rc;
+    if (!allow_smem<lin_gemm_kernel>()) return check_launch("linear_f32 smem attribute");
+    LinArgs a = {x, w, bias, sx, sw, out, M, N, K, ceil_div(M, 128), 0};
+    a.items = (long long)ceil_div(N, LIN_BN) * a.mtiles;
+    const int sms = sm_count();
+    launch_dependent(lin_split_kernel, dim3((unsigned)min(ceil_div(M, 8), 8 * sms)), 256, 0, st, x, M, K, xl, sx);
+    launch_dependent(lin_gemm_kernel, dim3((unsigned)min((long long)sms, a.items)), LIN_THREADS, LIN_SMEM, st, tm_x, tm_w, a);
+    count_launch(2);
+    return check_launch("linear_f32");
+}
+
+}  // namespace pikv
+
+using namespace pikv;
+
+extern "C" {
+
+size_t pikv_linear_f32_workspace_bytes(int32_t M, int32_t N, int32_t K) {
+    if (M <= 0 || N <= 0 || K <= 0) return 0;
+    return lin_limbs((int64_t)M + N, K) + lin_scales(M) + lin_scales(N);
+}
+
+int pikv_linear_f32(const float* x, const float* w, const float* bias, float* out, int32_t M, int32_t N, int32_t K, void* workspace,
+                    size_t workspace_bytes, pikv_stream_t stream) {
+    PIKV_REQUIRE(x && w && out && workspace, PIKV_EINVAL, "linear_f32: null pointer");
+    PIKV_REQUIRE(M > 0 && N > 0 && K > 0, PIKV_EINVAL, "linear_f32: bad sizes");
+    PIKV_REQUIRE(linear_f32_supported(K), PIKV_EUNSUPPORTED, "linear_f32: K=%d must be a multiple of 64 up to %d", K, 64 * LIN_MAX_KB);
+    PIKV_REQUIRE((uintptr_t)x % 16 == 0 && (uintptr_t)w % 16 == 0 && (uintptr_t)workspace % 256 == 0 && (uintptr_t)out % 4 == 0, PIKV_EINVAL,
+                 "linear_f32: misaligned pointer");
+    PIKV_REQUIRE(workspace_bytes >= pikv_linear_f32_workspace_bytes(M, N, K), PIKV_EINVAL, "linear_f32: workspace of %zu bytes", workspace_bytes);
+    PIKV_REQUIRE(M <= INT32_MAX - 128 && N <= INT32_MAX - 128, PIKV_ELIMIT, "linear_f32: too many rows");
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const int rc = linear_f32_weights(w, N, K, workspace, st);
+    return rc != PIKV_OK ? rc : linear_f32_rows(x, w, bias, out, M, N, K, workspace, st);
+}
+
+}  // extern "C"

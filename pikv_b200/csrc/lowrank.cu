@@ -320,7 +320,10 @@ extern "C" int pikv_lowrank_project(const void* x, const void* w, const float* b
     return pikv_lowrank_project_bias(x, w, bias, PIKV_F32, residual, out, out_dtype, M, N, K, relu, stream);
 }
 
-namespace pikv { int lowrank_pair_error_fetch(); }
+namespace pikv {
+int lowrank_pair_error_fetch();
+int linear_error_fetch();
+}  // namespace pikv
 
 // reads and clears the sticky error words of the tcgen05 kernels (synchronises the stream's device)
 extern "C" int pikv_lowrank_error_state(void) {
@@ -328,5 +331,6 @@ extern "C" int pikv_lowrank_error_state(void) {
     if (cudaMemcpyFromSymbol(&v, g_lowrank_error, sizeof(v)) != cudaSuccess) return -1;
     if (v) cudaMemcpyToSymbol(g_lowrank_error, &zero, sizeof(zero));
     const int pair = pikv::lowrank_pair_error_fetch();
-    return pair < 0 ? -1 : (int)v | pair;
+    const int linear = pikv::linear_error_fetch();
+    return pair < 0 || linear < 0 ? -1 : (int)v | pair | linear;
 }

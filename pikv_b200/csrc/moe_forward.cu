@@ -1,9 +1,9 @@
-// Inference forward of PiKVMoE (core/single/pikv_moe.py:139-336) up to the vocabulary projection, fp32: router nets,
+// Inference forward of PiKVMoE (core/single/pikv_moe.py:139-336), fp32: router nets,
 // LoRA experts, every expert's cached vector, the weighted sum of the experts and the ring update of the caches.
 //
 // As modules this is 180 launches, most of a few microseconds: at 8 x 128 tokens, 4 experts of width 256, 2310 us of host
-// time for 600 us of kernels (and 710 us of vocabulary projection).  Here it is three kernels, 57 us together; the whole
-// forward takes 800 us, bound by the projection:
+// time for 600 us of kernels and 710 us of vocabulary projection.  Here it is three kernels, 57 us together, in front of
+// the projection of linear_f32.cu (115 us); the whole forward takes 193 us:
 //   moe_stats_kernel    one CTA per expert: the mean of the importance-weighted value rows, taken through the
 //                       compressor and the value LoRA (both affine, so the mean may be taken first: 2 vectors instead of
 //                       2 x 128 rows); one CTA per sequence: sum of its tokens and the strategy selector.
@@ -16,6 +16,10 @@
 #include "common.cuh"
 
 namespace pikv {
+
+bool linear_f32_supported(int K);
+int linear_f32_weights(const float* w, int N, int K, void* workspace, cudaStream_t st);
+int linear_f32_rows(const float* x, const float* w, const float* bias, float* out, int M, int N, int K, void* workspace, cudaStream_t st);
 
 constexpr int MOE_TILE = 64, MOE_K = 16, MOE_PAD = MOE_TILE + 4;
 constexpr int MOE_MAX_H = 1024, MOE_MAX_RANK = 16;
@@ -137,6 +141,8 @@ __global__ void __launch_bounds__(MOE_STATS_THREADS) moe_stats_kernel(const __gr
         for (int k = 0; k < x.v_rank; ++k) s = fmaf(r[k], x.v_b[(size_t)k * H + h], s);
         w.cached[(size_t)blockIdx.x * H + h] = v2[h] + s * x.v_scale;
     }
+    // Nothing here reads what linear_f32_weights writes, but what waits for this grid has to find that kernel finished too.
+    dependency_wait();
 }
 
 __device__ __forceinline__ uint64_t moe_pair(float lo, float hi) {
@@ -295,7 +301,7 @@ __device__ __forceinline__ float moe_softmax(const pikv_moe_net& net, const floa
         for (int q = 0; q < nt; ++q) s += part[((size_t)q * T + t) * E + e];
         s += net.b2[e];
         raw[(size_t)t * E + e] = s;
-        l = net.temperature == 1.f ? s : s / net.temperature;
+        l = net.temperature == 1.f || net.temperature == 0.f ? s : s / net.temperature;     // as in the gate kernels
     }
     // a NaN among the logits has to stay: fmaxf would drop it, the exponentials below bring it back
     float m = l;
@@ -376,9 +382,9 @@ using namespace pikv;
 
 extern "C" {
 
-size_t pikv_moe_workspace_bytes(int32_t B, int32_t S, int32_t H, int32_t E) {
-    if (B <= 0 || S <= 0 || H <= 0 || E <= 0) return 0;
-    return moe_layout(B, S, H, E, nullptr, nullptr);
+size_t pikv_moe_workspace_bytes(int32_t B, int32_t S, int32_t H, int32_t E, int32_t V) {
+    if (B <= 0 || S <= 0 || H <= 0 || E <= 0 || V < 0) return 0;
+    return moe_layout(B, S, H, E, nullptr, nullptr) + (V ? pikv_linear_f32_workspace_bytes(B * S, V, H) : 0);
 }
 
 int pikv_moe_forward(const pikv_moe_params* p, pikv_stream_t stream) {
@@ -395,15 +401,28 @@ int pikv_moe_forward(const pikv_moe_params* p, pikv_stream_t stream) {
         PIKV_REQUIRE(x.mid > 0 && x.mid % 4 == 0 && x.mid <= MOE_MAX_H, PIKV_EUNSUPPORTED, "moe_forward: compressor width %d", x.mid);
         PIKV_REQUIRE(x.slots > 0 && x.slot >= 0 && x.slot < x.slots, PIKV_EINVAL, "moe_forward: slot %d of %d", x.slot, x.slots);
     }
+    PIKV_REQUIRE(p->V >= 0 && (p->V == 0 || (p->vocab_w && p->vocab_out && linear_f32_supported(p->H))), PIKV_EUNSUPPORTED,
+                 "moe_forward: no vocabulary projection of width %d", p->H);
+    PIKV_REQUIRE((uintptr_t)p->workspace % 256 == 0, PIKV_EINVAL, "moe_forward: misaligned workspace");
     MoeWork w;
-    const size_t need = moe_layout(p->B, p->S, p->H, p->E, static_cast<float*>(p->workspace), &w);
+    const size_t own = moe_layout(p->B, p->S, p->H, p->E, static_cast<float*>(p->workspace), &w);
+    const size_t need = pikv_moe_workspace_bytes(p->B, p->S, p->H, p->E, p->V);
     PIKV_REQUIRE(p->workspace_bytes >= need, PIKV_EINVAL, "moe_forward: workspace of %zu bytes, %zu needed", p->workspace_bytes, need);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    char* linear = static_cast<char*>(p->workspace) + own;
     const int T = p->B * p->S, mt = ceil_div(T, MOE_TILE), nt = p->H / MOE_TILE;
-    moe_stats_kernel<<<p->E + p->B, MOE_STATS_THREADS, 0, st>>>(*p, w);
+    // The projection's weights are split beside moe_stats_kernel: one streams memory, the other is a chain on a few SMs.
+    if (p->V) {
+        const int rc = linear_f32_weights(p->vocab_w, p->V, p->H, linear, st);
+        if (rc != PIKV_OK) return rc;
+    }
+    // Without the split in front it is a plain launch: it reads what earlier kernels left.
+    if (p->V) launch_dependent(moe_stats_kernel, dim3((unsigned)(p->E + p->B)), MOE_STATS_THREADS, 0, st, *p, w);
+    else moe_stats_kernel<<<p->E + p->B, MOE_STATS_THREADS, 0, st>>>(*p, w);
     launch_dependent(moe_gemm_kernel, dim3((unsigned)((p->E + 2) * nt + nt / 2), (unsigned)mt), MOE_THREADS, 0, st, *p, w);
     launch_dependent(moe_combine_kernel, dim3((unsigned)(p->E + ceil_div(T, MOE_ROWS))), MOE_THREADS, 0, st, *p, w);
     count_launch(3);
+    if (p->V) return linear_f32_rows(p->out, p->vocab_w, p->vocab_b, p->vocab_out, T, p->V, p->H, linear, st);
     return check_launch("moe_forward");
 }
 

@@ -1,9 +1,9 @@
 """PiKVMoE with the constructor, forward and state-dict keys of core/single/pikv_moe.py.
 
-Without gradients the router nets, the LoRA experts, the caches' compressors and the ring update run as a few
-fused CUDA kernels behind one native call; under autograd, with hooks, a `query` or scheduled caches they run as the
-modules they are, whose router tails and cache managers are CUDA kernels.  The embedding and the vocabulary projection
-are torch modules.  Parameters are created in the reference's order, so a model built
+Without gradients the router nets, the LoRA experts, the caches' compressors, the ring update and the vocabulary
+projection run as a few fused CUDA kernels behind one native call; under autograd, with hooks, a `query` or scheduled caches they run as the
+modules they are, whose router tails and cache managers are CUDA kernels.  The embedding is a torch module.
+Parameters are created in the reference's order, so a model built
 after torch.manual_seed(s) has the reference's weights for the same seed.
 """
 from __future__ import annotations
@@ -222,7 +222,7 @@ class PiKVMoE(nn.Module):
                 pass
 
     def _fused(self, x):
-        """(weighted expert sum, auxiliary loss) by the fused kernels, or None where the modules have to run: the
+        """(weighted expert sum, logits or None, auxiliary loss) by the fused kernels, or None where the modules have to run: the
         kernels see neither tracers, function transforms and tangents nor hooks and replaced modules."""
         if (torch.is_autocast_enabled() or _module._has_any_global_hook() or _fwd_ad._current_level >= 0 or torch.jit.is_tracing()
                 or torch._C._functorch.peek_interpreter_stack() is not None or torch._C._len_torch_dispatch_stack()
@@ -235,12 +235,12 @@ class PiKVMoE(nn.Module):
             return None
         router = self.router
         lb = router.load_balancing_router
-        lb.last_gate, router.importance_router.last_gate, router.last_gate = (GateResult(*r) for r in res[1:])
+        lb.last_gate, router.importance_router.last_gate, router.last_gate = (GateResult(*r) for r in res[2:])
 
         def loss():
             usage = lb.last_gate.prob_sum / float(x.shape[0] * x.shape[1])
             return lb.balance_weight * (usage.std() / usage.mean())
-        return res[0], loss
+        return res[0], res[1], loss
 
     def forward(self, x, query=None, return_loss=False, targets=None, use_teacher=False):
         if x.dim() == 2:
@@ -252,8 +252,9 @@ class PiKVMoE(nn.Module):
         if query is None and not self.use_cache_scheduling and not torch.is_grad_enabled():
             fused = self._fused(x)
             if fused is not None:
-                out, lb_loss = fused
-                logits = self.vocab_proj(out)
+                out, logits, lb_loss = fused
+                if logits is None:
+                    logits = self.vocab_proj(out)
                 return (logits, lb_loss()) if return_loss else logits
         routing_weights, expert_indices, top_k_weights, lb_loss, importance = self.router(x)
         if query is not None:

@@ -178,6 +178,12 @@ def quant_block_pair(k: torch.Tensor, v: torch.Tensor, group_size: int, qmin: in
     return host().quant_pair(k, v, group_size, qmin, qmax, symmetric, params_in, sample_count, count_add)
 
 
+# ------------------------------------------------------------------ fp32 linear layer
+def linear_f32(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """x [..., K] @ w [N, K].T + bias in fp32 on the tensor cores (two f16 limbs per operand); K a multiple of 64 up to 256."""
+    return host().linear_f32(x, w, bias)
+
+
 # ------------------------------------------------------------------ H2O
 def h2o_accumulate(acc: torch.Tensor, ts: torch.Tensor, idx: Optional[torch.Tensor], w: torch.Tensor, now: float,
                    decay: float = 1.0, status: Optional[torch.Tensor] = None) -> None:
