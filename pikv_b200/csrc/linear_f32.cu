@@ -11,10 +11,11 @@
 //   lin_gemm_kernel    persistent, one CTA per SM.  Items are 128 x 128 outputs, row tiles innermost, contiguous per CTA:
 //                      w's tile stays in shared memory (hi and lo of a 64-wide k block next to each other: one MMA of
 //                      N = 256 takes both products of an x hi block), x blocks stream through a ring.  Two accumulator
-//                      pairs of 256 columns, one per half of K: eight epilogue warps keep the first half's sums in
-//                      registers while the second is computed, turn 32 x 32 patches in shared memory and store whole rows (N is odd in earnest, so neither TMA nor vector stores apply).
+//                      pairs of 256 columns, one per half of K: sixteen epilogue warps, 32 x 32 outputs each, keep the
+//                      first half's sums in registers while the second is computed, turn their patches in shared
+//                      memory and store whole rows (N is odd in earnest, so neither TMA nor vector stores apply).
 //
-// 1024 x 256 -> 50257: 115 us for the GEMM and 26 for the splits (140 us a call; cuBLAS's fp32 kernel and its bias pass 716),
+// 1024 x 256 -> 50257: 110 us for the GEMM and 26 for the splits (135 us a call, 140 with eight epilogue warps; cuBLAS's fp32 kernel and its bias pass 716),
 // relative error 2.0e-7 against 64 bits (cuBLAS 2.9e-7; one accumulator for all of K 3.5e-7).  The 79 GFLOP of the three
 // products would take 48 us at the measured bf16 rate and the output 32 us of HBM.
 #include "tc_common.cuh"
@@ -23,8 +24,8 @@ namespace pikv {
 
 constexpr int LIN_BN = 128, LIN_BLOCK = 128 * 128;       // outputs per tile; bytes of a [128 x 64] f16 block
 constexpr int LIN_MAX_KB = 4, LIN_STAGES = 4;
-constexpr int LIN_EPI_WARPS = 8, LIN_THREADS = 64 + 32 * LIN_EPI_WARPS;
-constexpr int LIN_PATCH = 32 * 33 * 4;
+constexpr int LIN_EPI_WARPS = 16, LIN_THREADS = 64 + 32 * LIN_EPI_WARPS;
+constexpr int LIN_PATCH = 16 * 33 * 4;
 constexpr int LIN_SMEM = 2 * LIN_MAX_KB * LIN_BLOCK + LIN_STAGES * LIN_BLOCK + LIN_EPI_WARPS * LIN_PATCH + 256 + 1024;
 static_assert(LIN_SMEM <= 227 * 1024, "linear_f32: shared memory");
 
@@ -190,66 +191,55 @@ __global__ void __launch_bounds__(LIN_THREADS, 1) lin_gemm_kernel(const __grid_c
             }
         }
     } else {
-        const int lg = warp & 3, side = (warp - 2) >> 2; // tensor-memory lane group, and which 64 of the 128 columns
+        const int lg = warp & 3, side = (warp - 2) >> 2; // tensor-memory lane group, and which 32 of the 128 columns
         float* patch = patches + (size_t)(warp - 2) * (LIN_PATCH / 4);
         int local = 0;
         for (long long item = first; item < last && !failed; ++item, ++local) {
             const int nt = (int)(item / a.mtiles), mt = (int)(item % a.mtiles);
-            const int m0 = mt * 128 + lg * 32, n0 = nt * LIN_BN + side * 64;
+            const int m0 = mt * 128 + lg * 32, n0 = nt * LIN_BN + side * 32;
             const float sx = m0 + lane < a.M ? a.sx[m0 + lane] : 1.f;
             const int rows = min(32, a.M - m0);
-            const uint32_t taddr = tmem_base + ((uint32_t)(lg * 32) << 16) + (uint32_t)(side * 64);
-            float acc[2][32] = {};
-            if (kbs > first_kbs) {
-                if (!lr_mbar_wait(tfull0, (uint32_t)local & 1u)) { failed = true; break; }
+            const uint32_t taddr = tmem_base + ((uint32_t)(lg * 32) << 16) + (uint32_t)(side * 32);
+            // this item's column factors, in flight while its sums are computed
+            const int n = n0 + lane;
+            const bool in = n < a.N;
+            const float sw = in ? __ldg(a.sw + n) : 1.f, bias = in && a.bias ? __ldg(a.bias + n) : 0.f;
+            float acc[32] = {};
+            for (int half = kbs > first_kbs ? 0 : 1; half < 2; ++half) {
+                const int pair = kbs > first_kbs ? half : 0;         // a single k block has one half
+                if (!lr_mbar_wait(tfull0 + 8 * pair, (uint32_t)local & 1u)) { failed = true; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                    float u[32];
-                    lr_tmem_ld32(taddr + 32 * c, acc[c]);
-                    lr_tmem_ld32(taddr + 128 + 32 * c, u);
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) acc[c][i] += u[i];
-                }
-                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                lr_mbar_arrive(tempty0);
-            }
-            const int half = kbs > first_kbs;
-            if (!lr_mbar_wait(tfull0 + 8 * half, (uint32_t)local & 1u)) { failed = true; break; }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-            for (int c = 0; c < 2; ++c) {
                 float v[32];
-                lr_tmem_ld32(taddr + half * 256 + 128 + 32 * c, v);
+                lr_tmem_ld32(taddr + pair * 256 + 128, v);
 #pragma unroll
-                for (int i = 0; i < 32; ++i) acc[c][i] += v[i];
-                lr_tmem_ld32(taddr + half * 256 + 32 * c, v);
+                for (int i = 0; i < 32; ++i) acc[i] += v[i];
+                lr_tmem_ld32(taddr + pair * 256, v);
 #pragma unroll
-                for (int i = 0; i < 32; ++i) acc[c][i] += v[i];
+                for (int i = 0; i < 32; ++i) acc[i] += v[i];
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                lr_mbar_arrive(tempty0 + 8 * pair);
             }
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            lr_mbar_arrive(tempty0 + 8 * half);
+            if (failed) break;
+            const bool marked = __any_sync(0xffffffffu, sx == 0.f || sw == 0.f);
+            float* to = a.out + (size_t)m0 * a.N + n;
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
+            for (int h = 0; h < 32; h += 16) {           // half the warp's rows at a time: all 32 would cost two ring stages
+                if ((lane & 16) == h) {
 #pragma unroll
-                for (int i = 0; i < 32; ++i) patch[lane * 33 + i] = acc[c][i];
+                    for (int i = 0; i < 32; ++i) patch[(lane & 15) * 33 + i] = acc[i];
+                }
                 __syncwarp();
-                const int n = n0 + 32 * c + lane;
-                const bool in = n < a.N;
-                const float sw = in ? a.sw[n] : 1.f, bias = in && a.bias ? a.bias[n] : 0.f;
-                float* to = a.out + (size_t)m0 * a.N + n;
-                const bool marked = __any_sync(0xffffffffu, sx == 0.f || sw == 0.f);
                 if (!marked && rows == 32) {
 #pragma unroll
-                    for (int r = 0; r < 32; ++r) {
-                        const float o = patch[r * 33 + lane] * __shfl_sync(0xffffffffu, sx, r) * sw + bias;
-                        if (in) to[(size_t)r * a.N] = o;
+                    for (int r = 0; r < 16; ++r) {
+                        const float o = patch[r * 33 + lane] * __shfl_sync(0xffffffffu, sx, h + r) * sw + bias;
+                        if (in) to[(size_t)(h + r) * a.N] = o;
                     }
                 } else {
-                    for (int r = 0; r < rows; ++r) {
+                    for (int r = h; r < min(rows, h + 16); ++r) {
                         const float s = __shfl_sync(0xffffffffu, sx, r);
                         if (!in) continue;
-                        const float o = s == 0.f || sw == 0.f ? lin_plain(a, m0 + r, n) : patch[r * 33 + lane] * s * sw;
+                        const float o = s == 0.f || sw == 0.f ? lin_plain(a, m0 + r, n) : patch[(r - h) * 33 + lane] * s * sw;
                         to[(size_t)r * a.N] = o + bias;
                     }
                 }
