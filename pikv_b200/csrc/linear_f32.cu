@@ -15,8 +15,8 @@
 //                      first half's sums in registers while the second is computed, turn their patches in shared
 //                      memory and store whole rows (N is odd in earnest, so neither TMA nor vector stores apply).
 //
-// 1024 x 256 -> 50257: 110 us for the GEMM and 26 for the splits (135 us a call, 140 with eight epilogue warps; cuBLAS's fp32 kernel and its bias pass 716),
-// relative error 2.0e-7 against 64 bits (cuBLAS 2.9e-7; one accumulator for all of K 3.5e-7).  The 79 GFLOP of the three
+// 1024 x 256 -> 50257: 110 us for the GEMM and 26 for the splits (135 us a call, 140 with eight epilogue warps; cuBLAS's
+// fp32 kernel and its bias pass 716), relative error 2.0e-7 against 64 bits (cuBLAS 2.9e-7; one accumulator for all of K 3.5e-7).  The 79 GFLOP of the three
 // products would take 48 us at the measured bf16 rate and the output 32 us of HBM.
 #include "tc_common.cuh"
 
