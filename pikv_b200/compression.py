@@ -37,8 +37,7 @@ def _linear(layer: nn.Linear, x: torch.Tensor, relu: bool) -> torch.Tensor:
     """One Linear (+ReLU): tcgen05 kernel for bf16 inputs whose shapes fit, cuBLAS otherwise."""
     K, N = layer.in_features, layer.out_features
     if x.dtype == torch.bfloat16 and x.is_cuda and K % 16 == 0 and N % 16 == 0 and (N <= 256 or N % 256 == 0):
-        p = layer._parameters
-        return ops.lowrank_project(x, p["weight"].to(torch.bfloat16), p["bias"], relu=relu)
+        return ops.lowrank_project(x, layer.weight.to(torch.bfloat16), layer.bias, relu=relu)
     y = F.linear(x, layer.weight.to(x.dtype), None if layer.bias is None else layer.bias.to(x.dtype))
     return F.relu(y) if relu else y
 
@@ -157,11 +156,11 @@ class SVDCompressor(BaseCompressor):
     def _round_trip(self, keys: torch.Tensor, values: torch.Tensor):
         H, R = self.hidden_size, self.rank
         if (keys.shape == values.shape and keys.dtype == values.dtype == torch.bfloat16 and keys.is_cuda and R % 16 == 0 and R <= 64
-                and H % 16 == 0 and H <= 4096 and keys.numel() >= self.PAIR_ROWS * H):
-            m = self._modules
-            down, up = ([m[f"{which}_{part}"]._parameters for which in ("key", "value")] for part in ("projector", "reconstructor"))
-            return ops.lowrank_pair((keys, values), [p["weight"] for p in down], [p["bias"] for p in down],
-                                    [p["weight"] for p in up], [p["bias"] for p in up])
+                and H % 16 == 0 and H <= 4096 and keys.numel() >= self.PAIR_ROWS * H
+                and type(self).project is SVDCompressor.project and type(self).reconstruct is SVDCompressor.reconstruct):
+            down, up = (self.key_projector, self.value_projector), (self.key_reconstructor, self.value_reconstructor)
+            return ops.lowrank_pair((keys, values), [p.weight for p in down], [p.bias for p in down],
+                                    [p.weight for p in up], [p.bias for p in up])
         return (self.reconstruct(self.project(keys, "key"), "key"),
                 self.reconstruct(self.project(values, "value"), "value"))
 

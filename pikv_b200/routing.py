@@ -98,15 +98,14 @@ class BaseRouter(nn.Module):
 
     def _fused_net(self, mlp: nn.Sequential, x: torch.Tensor) -> bool:
         return (x.dtype == torch.bfloat16 and self.num_experts <= 32 and x.shape[-1] % 8 == 0
-                and mlp._modules["0"].out_features % 8 == 0)
+                and mlp[0].out_features % 8 == 0)
 
     def _net_weights(self, mlp: nn.Sequential):
         """w1, b1, w2, b2, the weights in bf16."""
         out = []
-        for name in ("0", "2"):
-            p = mlp._modules[name]._parameters
-            w = p["weight"]
-            out += [w if w.dtype == torch.bfloat16 else w.detach().to(torch.bfloat16), p["bias"]]
+        for layer in (mlp[0], mlp[2]):        # attributes: a reparametrised layer has its weight there, not among its parameters
+            w = layer.weight
+            out += [w if w.dtype == torch.bfloat16 else w.detach().to(torch.bfloat16), layer.bias]
         return out
 
     def _gate_net(self, mlp: nn.Sequential, x2d: torch.Tensor, **kw) -> ops.GateResult:
