@@ -673,22 +673,22 @@ __device__ __forceinline__ void ss_for_keys(const float* __restrict__ src, int n
     }
 }
 
-// exclusive prefix of v over the CTA in thread order, and the total; red: NT / 32 ints of shared memory
-template <int NT>
-__device__ __forceinline__ int ss_block_scan(int v, int* red, int& total) {
+// exclusive prefix of v over the CTA in thread order, and the total; red: NT / 32 words of shared memory
+template <int NT, typename V>
+__device__ __forceinline__ V ss_block_scan(V v, V* red, V& total) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int inc = v;
+    V inc = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const int x = __shfl_up_sync(0xffffffffu, inc, o);
+        const V x = __shfl_up_sync(0xffffffffu, inc, o);
         if (lane >= o) inc += x;
     }
     if (lane == 31) red[warp] = inc;
     __syncthreads();
-    int before = 0, tot = 0;
+    V before = 0, tot = 0;
 #pragma unroll
     for (int q = 0; q < NT / 32; ++q) {
-        const int x = red[q];
+        const V x = red[q];
         before += q < warp ? x : 0;
         tot += x;
     }
@@ -1094,14 +1094,16 @@ __global__ void __launch_bounds__(NT, 1024 / NT) h2o_select_stream_kernel(const 
         ss_word_bits<NT>(rt, t, w, wb, n, al_t, valid, sh.tile[warp], gtt, eqt);
         uint32_t keep = gta | gtt;
         if (ties_a || ties_t) {
-            // equal keys in index order: packed counts of both arrays (a chunk holds at most 32 * NT < 65536 positions)
-            int total;
-            const int packed = (ties_a ? __popc(eqa) : 0) | ((ties_t ? __popc(eqt) : 0) << 16);
-            const int before = ss_block_scan<NT>(packed, sh.red_i, total);
-            keep |= ties_a ? ss_lowest_bits(eqa, ra.need_eq - (eq_a_before + (before & 0xffff))) : eqa;
-            keep |= ties_t ? ss_lowest_bits(eqt, rt.need_eq - (eq_t_before + (before >> 16))) : eqt;
-            eq_a_before += total & 0xffff;
-            eq_t_before += total >> 16;
+            // equal keys in index order: counts of both arrays in the halves of an unsigned word (the 32768 positions
+            // of a 1024-thread chunk would be the sign bit of a signed one)
+            static_assert(32 * NT < 65536, "a chunk's count has to fit in half a word");
+            uint32_t total;
+            const uint32_t packed = (ties_a ? (uint32_t)__popc(eqa) : 0u) | ((ties_t ? (uint32_t)__popc(eqt) : 0u) << 16);
+            const uint32_t before = ss_block_scan<NT>(packed, sh.red_a, total);
+            keep |= ties_a ? ss_lowest_bits(eqa, ra.need_eq - (eq_a_before + (int)(before & 0xffffu))) : eqa;
+            keep |= ties_t ? ss_lowest_bits(eqt, rt.need_eq - (eq_t_before + (int)(before >> 16))) : eqt;
+            eq_a_before += (int)(total & 0xffffu);
+            eq_t_before += (int)(total >> 16);
         } else {
             keep |= eqa | eqt;
         }
