@@ -511,6 +511,11 @@ typedef struct {
     void* probs16; float* step_max; int32_t probs_stride, step_stride;
 } pikv_decode_params;
 
+/* out[i] = length[seq_ids[i]], or 0 where the id lies outside 0 .. num_seqs - 1 (such a stream is answered with a zero row
+ * and PIKV_ST_BAD_SEQ by the decode kernels); length [num_seqs], seq_ids and out [n] */
+int pikv_seq_lengths(const int32_t* length, const int32_t* seq_ids, int32_t n, int32_t num_seqs, int32_t* out,
+                     pikv_stream_t stream);
+
 size_t pikv_decode_attn_workspace_bytes(int32_t B, int32_t n_q, int32_t n_kv, int32_t max_ctx, int32_t splits);
 int    pikv_decode_attn_default_splits(int32_t B, int32_t n_kv, int32_t max_ctx);
 int    pikv_decode_attn_q8(const pikv_decode_params* p, pikv_stream_t stream);

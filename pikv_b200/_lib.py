@@ -177,6 +177,7 @@ SIGNATURES = {
     "pikv_h2o_accumulate": (i32, [vp, vp, i32, vp, vp, i32, f32, f32, vp, vp]),
     "pikv_h2o_select": (i32, [vp, vp, i32, i32, vp, i32, i32, i32, vp, vp, i32, vp, vp]),
     "pikv_h2o_compact": (i32, [C.POINTER(CompactParams), vp]),
+    "pikv_seq_lengths": (i32, [vp, vp, i32, i32, vp, vp]),
     "pikv_decode_attn_workspace_bytes": (sz, [i32, i32, i32, i32, i32]),
     "pikv_decode_attn_default_splits": (i32, [i32, i32, i32]),
     "pikv_decode_attn_q8": (i32, [C.POINTER(DecodeParams), vp]),

@@ -1138,6 +1138,25 @@ extern "C" int pikv_decode_attn_default_splits(int32_t B, int32_t n_kv, int32_t 
     return 1;
 }
 
+namespace pikv {
+__global__ void __launch_bounds__(256) seq_lengths_kernel(const int* length, const int* seq_ids, int n, int num_seqs, int* out) {
+    dependency_wait();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int seq = seq_ids[i];
+    out[i] = seq >= 0 && seq < num_seqs ? length[seq] : 0;
+}
+}  // namespace pikv
+
+extern "C" int pikv_seq_lengths(const int32_t* length, const int32_t* seq_ids, int32_t n, int32_t num_seqs, int32_t* out,
+                                pikv_stream_t stream) {
+    PIKV_REQUIRE(length && seq_ids && out, PIKV_EINVAL, "seq_lengths: null pointer");
+    PIKV_REQUIRE(n > 0 && num_seqs > 0, PIKV_EINVAL, "seq_lengths: bad sizes");
+    launch_dependent(seq_lengths_kernel, ceil_div(n, 256), 256, 0, static_cast<cudaStream_t>(stream), length, seq_ids, n, num_seqs, out);
+    count_launch(1);
+    return check_launch("seq_lengths_kernel");
+}
+
 extern "C" size_t pikv_decode_attn_workspace_bytes(int32_t B, int32_t n_q, int32_t n_kv, int32_t max_ctx,
                                                    int32_t splits) {
     (void)max_ctx; (void)splits;

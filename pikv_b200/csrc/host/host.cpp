@@ -389,7 +389,13 @@ PyObject* dispatch_loss(PyObject* const* a, Py_ssize_t) {
 at::Tensor lengths(const Cache& c, const at::Tensor& ids, PyObject* given) {
     if (given != Py_None) return req(given, "seq_len", at::kInt);
     const at::Tensor& len = buffer(c.buffers, s_length);
-    return ids.defined() ? len.index_select(0, ids) : len;
+    if (!ids.defined()) return len;
+    if (!len.defined() || len.scalar_type() != at::kInt || len.numel() < c.num_seqs) fail("the cache's length must be one int32 per sequence");
+    // ids outside the cache are for the kernels to report: their length is 0
+    at::Tensor out = at::empty({ids.numel()}, on(ids, at::kInt));
+    if (ids.numel())
+        check(pikv_seq_lengths(ptr<int32_t>(len), ptr<int32_t>(ids), (int32_t)ids.numel(), c.num_seqs, ptr<int32_t>(out), stream()), "pikv_seq_lengths");
+    return out;
 }
 
 // decode(cache..., q, seq_ids, seq_len, want_lse, scores)  /  decode_h2o(cache..., q, seq_ids, seq_len, acc, probs, step_max)
