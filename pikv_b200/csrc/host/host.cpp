@@ -60,6 +60,12 @@ at::Tensor f32(PyObject* o, const char* name) {
     return !t.defined() || t.scalar_type() == at::kFloat ? t : t.to(at::kFloat);
 }
 
+// rows of x [..., K]
+int rows_of(const at::Tensor& x, const char* name) {
+    if (x.dim() < 1 || x.size(-1) < 1) fail("%s must have a last dimension of at least 1", name);
+    return (int)(x.numel() / x.size(-1));
+}
+
 int dtype_code(const at::Tensor& t, const char* name) {
     if (t.scalar_type() == at::kFloat) return PIKV_F32;
     if (t.scalar_type() == at::kBFloat16) return PIKV_BF16;
@@ -349,7 +355,7 @@ PyObject* gate_mlp(PyObject* const* a, Py_ssize_t) {
     PyObject* given = a[5 + GateTail::ARGS];
     PyObject* const* da = a + 6 + GateTail::ARGS;
     pikv_gate_params g = {};
-    g.T = (int32_t)(x.numel() / x.size(-1)); g.H = (int32_t)w1.size(0); g.E = (int32_t)w2.size(0);
+    g.T = rows_of(x, "x"); g.H = (int32_t)w1.size(0); g.E = (int32_t)w2.size(0);
     g.dtype = PIKV_BF16; g.w2 = ptr(w2);
     tail.fill(g);
     GateOut out(given, x, g.T, g.E, g.top_k, tail.want_probs);
@@ -514,7 +520,7 @@ PyObject* compact(PyObject* const* a, Py_ssize_t) {
 PyObject* quant_pair(PyObject* const* a, Py_ssize_t) {
     const at::Tensor k = req(a[0], "keys"), v = req(a[1], "values", k.scalar_type());
     if (k.dim() < 1 || v.sizes() != k.sizes()) fail("keys and values must have the same shape");
-    const int H = (int)k.size(-1), N = (int)(k.numel() / H), gs = (int)num(a[2]);
+    const int N = rows_of(k, "keys"), H = (int)k.size(-1), gs = (int)num(a[2]);
     const at::Tensor params = opt(a[6], "params_in", at::kFloat);
     const at::Tensor counter = opt(a[7], "sample_count", at::kFloat);
     const size_t bytes = pikv_quant_block_pair_workspace_bytes(N, H, gs);
@@ -543,7 +549,7 @@ std::vector<int64_t> with_last(const at::Tensor& x, int64_t last) {
 PyObject* lowrank(PyObject* const* a, Py_ssize_t) {
     const at::Tensor x = req(a[0], "x", at::kBFloat16), w = half_of(a[1], "w"), b = bias_of(a[2]), r = opt(a[4], "residual", at::kBFloat16);
     if (x.dim() < 2 || w.dim() != 2 || w.size(1) != x.size(-1)) fail("w must be [N,%lld]", (long long)x.size(-1));
-    const int K = (int)x.size(-1), N = (int)w.size(0), M = (int)(x.numel() / K);
+    const int M = rows_of(x, "x"), K = (int)x.size(-1), N = (int)w.size(0);
     const bool f = truth(a[5]);
     at::Tensor y = at::empty(with_last(x, N), on(x, f ? at::kFloat : at::kBFloat16));
     check(pikv_lowrank_project_bias(ptr(x), ptr(w), ptr(b), b.defined() ? dtype_code(b, "bias") : PIKV_F32, ptr(r), ptr(y), f ? PIKV_F32 : PIKV_BF16,
@@ -573,15 +579,15 @@ PyObject* lowrank_pair(PyObject* const* a, Py_ssize_t) {
         y[i] = at::empty(with_last(x[i], w2[i].size(0)), on(x[i], at::kBFloat16));
         xp[i] = ptr(x[i]); w1p[i] = ptr(w1[i]); b1p[i] = ptr(b1[i]); w2p[i] = ptr(w2[i]); b2p[i] = ptr(b2[i]); yp[i] = ptr(y[i]);
     }
-    const int K = (int)x[0].size(-1);
-    check(pikv_lowrank_pair(xp, w1p, b1p, w2p, b2p, code < 0 ? PIKV_F32 : code, yp, (int32_t)(x[0].numel() / K), K, (int32_t)w1[0].size(0),
+    const int M = rows_of(x[0], "x"), K = (int)x[0].size(-1);
+    check(pikv_lowrank_pair(xp, w1p, b1p, w2p, b2p, code < 0 ? PIKV_F32 : code, yp, M, K, (int32_t)w1[0].size(0),
                             (int32_t)w2[0].size(0), stream()), "pikv_lowrank_pair");
     return tuple(y[0], y[1]);
 }
 
 // linear_f32(x, w, bias) -> [..., N]
 at::Tensor linear_f32(const at::Tensor& x, const at::Tensor& w, const float* bias) {
-    const int K = (int)x.size(-1), N = (int)w.size(0), M = (int)(x.numel() / K);
+    const int M = rows_of(x, "x"), K = (int)x.size(-1), N = (int)w.size(0);
     at::Tensor y = at::empty(with_last(x, N), on(x, at::kFloat));
     const size_t bytes = pikv_linear_f32_workspace_bytes(M, N, K);
     const at::Tensor ws = workspace(x, bytes);
