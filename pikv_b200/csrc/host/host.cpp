@@ -66,6 +66,12 @@ int rows_of(const at::Tensor& x, const char* name) {
     return (int)(x.numel() / x.size(-1));
 }
 
+// the kernels read (or write) that many elements
+const at::Tensor& holds(const at::Tensor& t, int64_t elements, const char* name) {
+    if (t.defined() && t.numel() < elements) fail("%s has %lld elements, %lld are needed", name, (long long)t.numel(), (long long)elements);
+    return t;
+}
+
 int dtype_code(const at::Tensor& t, const char* name) {
     if (t.scalar_type() == at::kFloat) return PIKV_F32;
     if (t.scalar_type() == at::kBFloat16) return PIKV_BF16;
@@ -244,6 +250,7 @@ struct GateTail {
         : k((int)num(a[0])), mode((int)num(a[2])), capacity((int)num(a[6])), mask(f32(a[1], "gate vector")), corr(f32(a[3], "gate vector")),
           base(opt(a[7], "slot_base", at::kInt)), temperature(real(a[4])), eps(real(a[5])), want_probs(truth(a[8])) {}
     void fill(pikv_gate_params& g) const {
+        holds(mask, g.E, "expert_mask"); holds(corr, g.E, "correction"); holds(base, g.E, "slot_base");
         g.top_k = k;
         g.expert_mask = ptr<float>(mask);
         g.mask_mode = mask.defined() ? mode : PIKV_MASK_NONE;
@@ -272,7 +279,7 @@ PyObject* gate(PyObject* const* a, Py_ssize_t) {
         if (act.dim() != 2 || w2.dim() != 2 || w2.size(1) != act.size(1)) fail("act must be [T,H] and w2 [E,H] with the same H");
         g.T = (int32_t)act.size(0); g.H = (int32_t)act.size(1); g.E = (int32_t)w2.size(0);
         g.dtype = dtype_code(act, "act");
-        g.act = ptr(act); g.w2 = ptr(w2); g.b2 = ptr<float>(b2);
+        g.act = ptr(act); g.w2 = ptr(w2); g.b2 = ptr<float>(holds(b2, g.E, "b2"));
     }
     const at::Tensor& like = logits.defined() ? logits : act;
     const GateTail tail(a + 4);
@@ -305,7 +312,7 @@ PyObject* route_append(PyObject* const* a, Py_ssize_t) {
     if (k.size(0) < act.size(0)) fail("route_append: %d tokens in act, %d in k", (int)act.size(0), (int)k.size(0));
     const GateTail tail(a + 5);
     pikv_gate_params g = {};
-    g.act = ptr(act); g.w2 = ptr(w2); g.b2 = ptr<float>(b2); g.dtype = dtype_code(act, "act");
+    g.act = ptr(act); g.w2 = ptr(w2); g.b2 = ptr<float>(holds(b2, c.num_seqs, "b2")); g.dtype = dtype_code(act, "act");
     g.T = (int32_t)act.size(0); g.H = (int32_t)act.size(1); g.E = c.num_seqs;
     tail.fill(g);
     GateOut out(a[5 + GateTail::ARGS], act, g.T, g.E, g.top_k, tail.want_probs);
@@ -357,6 +364,7 @@ PyObject* gate_mlp(PyObject* const* a, Py_ssize_t) {
     pikv_gate_params g = {};
     g.T = rows_of(x, "x"); g.H = (int32_t)w1.size(0); g.E = (int32_t)w2.size(0);
     g.dtype = PIKV_BF16; g.w2 = ptr(w2);
+    holds(b1, g.H, "b1"); holds(b2, g.E, "b2");
     tail.fill(g);
     GateOut out(given, x, g.T, g.E, g.top_k, tail.want_probs);
     out.fill(g);
@@ -384,7 +392,9 @@ PyObject* gate_mlp(PyObject* const* a, Py_ssize_t) {
 PyObject* dispatch_loss(PyObject* const* a, Py_ssize_t) {
     const at::Tensor idx = req(a[0], "topk_idx", at::kInt), w = req(a[1], "topk_w", at::kFloat), slot = req(a[2], "slot", at::kInt),
                      counts = req(a[3], "counts_k", at::kInt), psum = req(a[4], "prob_sum", at::kFloat);
+    if (idx.dim() != 2) fail("topk_idx must be [T,k]");
     const int T = (int)idx.size(0), k = (int)idx.size(1), E = (int)num(a[5]);
+    holds(w, idx.numel(), "topk_w"); holds(slot, idx.numel(), "slot"); holds(counts, (int64_t)k * E, "counts_k"); holds(psum, E, "prob_sum");
     Dense dense(a + 6, idx, {T}, E);
     check(pikv_dispatch_loss(ptr<int32_t>(idx), ptr<float>(w), ptr<int32_t>(slot), ptr<int32_t>(counts), ptr<float>(psum), T, E, k, &dense.o, stream()),
           "pikv_dispatch_loss");
@@ -426,11 +436,15 @@ PyObject* decode(PyObject* const* a, Py_ssize_t n) {
         step = req(a[5], "step_max", at::kFloat);
         p.probs16 = ptr(probs); p.step_max = ptr<float>(step);
         p.probs_stride = (int32_t)probs.size(-1); p.step_stride = (int32_t)step.size(-1);
+        holds(acc, (int64_t)p.B * p.n_kv * acc.size(-1), "acc");
+        holds(probs, (int64_t)p.B * p.n_q * probs.size(-1), "the workspace's probabilities");
+        holds(step, (int64_t)p.B * p.n_q * step.size(-1), "the workspace's step maxima");
     } else {
         scores = opt(a[4], "scores", at::kFloat);
         want_lse = truth(a[3]) || scores.defined();
         p.scores = ptr<float>(scores);
         p.score_stride = scores.defined() ? (int32_t)scores.size(-1) : 0;
+        holds(scores, (int64_t)p.B * p.n_q * p.score_stride, "scores");
     }
     // output, log-sum-exp and scratch from one allocation
     const size_t scratch = pikv_decode_attn_workspace_bytes(p.B, p.n_q, p.n_kv, 0, 0);
@@ -494,6 +508,7 @@ PyObject* compact(PyObject* const* a, Py_ssize_t) {
     p.dst_k_codes = d.at(s_k_codes); p.dst_v_codes = d.at(s_v_codes); p.dst_k_scale = d.at(s_k_scale); p.dst_v_scale = d.at(s_v_scale);
     p.dst_k_zp = d.at(s_k_zp); p.dst_v_zp = d.at(s_v_zp);
     const int64_t segments = (int64_t)s.num_seqs * (p.per_head ? s.n_kv : 1);
+    holds(keep, segments * keep.size(1), "keep_idx"); holds(count, segments, "kept_count");
     static const char* names[2] = {"acc", "ts"};
     at::Tensor from[2], to[2];
     for (int i = 0; i < 2; ++i) {
@@ -522,6 +537,7 @@ PyObject* quant_pair(PyObject* const* a, Py_ssize_t) {
     if (k.dim() < 1 || v.sizes() != k.sizes()) fail("keys and values must have the same shape");
     const int N = rows_of(k, "keys"), H = (int)k.size(-1), gs = (int)num(a[2]);
     const at::Tensor params = opt(a[6], "params_in", at::kFloat);
+    if (gs > 0) holds(params, 2 * (((int64_t)H + gs - 1) / gs), "params_in");
     const at::Tensor counter = opt(a[7], "sample_count", at::kFloat);
     const size_t bytes = pikv_quant_block_pair_workspace_bytes(N, H, gs);
     at::Tensor dk = at::empty_like(k), dv = at::empty_like(v), mse = at::empty({}, on(k, at::kFloat)), ws = workspace(k, bytes);
@@ -551,6 +567,7 @@ PyObject* lowrank(PyObject* const* a, Py_ssize_t) {
     if (x.dim() < 2 || w.dim() != 2 || w.size(1) != x.size(-1)) fail("w must be [N,%lld]", (long long)x.size(-1));
     const int M = rows_of(x, "x"), K = (int)x.size(-1), N = (int)w.size(0);
     const bool f = truth(a[5]);
+    holds(b, N, "bias"); holds(r, (int64_t)M * N, "residual");
     at::Tensor y = at::empty(with_last(x, N), on(x, f ? at::kFloat : at::kBFloat16));
     check(pikv_lowrank_project_bias(ptr(x), ptr(w), ptr(b), b.defined() ? dtype_code(b, "bias") : PIKV_F32, ptr(r), ptr(y), f ? PIKV_F32 : PIKV_BF16,
                                     M, N, K, truth(a[3]) ? 1 : 0, stream()), "pikv_lowrank_project_bias");
@@ -572,6 +589,7 @@ PyObject* lowrank_pair(PyObject* const* a, Py_ssize_t) {
             fail("lowrank_pair: x, w1 and w2 do not fit");
         for (const at::Tensor* b : {&b1[i], &b2[i]}) {
             if (!b->defined()) continue;
+            holds(*b, b == &b1[i] ? w1[i].size(0) : w2[i].size(0), "bias");
             const int own = dtype_code(*b, "bias");
             if (code >= 0 && own != code) fail("lowrank_pair: the biases must share their dtype");
             code = own;

@@ -18,6 +18,8 @@ from pikv_b200 import ops
 bf, f32, i32 = torch.bfloat16, torch.float32, torch.int32
 def t(*shape, dtype=bf):
     return torch.empty(*shape, dtype=dtype, device="cuda")
+with FakeTensorMode():               # what it imports on first use, once
+    t(1)
 for call in json.loads(sys.argv[1]):
     r, w = os.pipe()
     pid = os.fork()
@@ -42,7 +44,31 @@ ZERO_WIDTH = [
     "ops.gate_mlp_fused(t(4, 0), t(16, 0), None, t(8, 16), None)",
     "ops.quant_block_pair(t(4, 0), t(4, 0), 64, 0, 255, False)",
 ]
-CALLS = ZERO_WIDTH
+CACHE = "c = object.__new__(pikv_b200.PagedKVCache); torch.nn.Module.__init__(c); c.num_seqs, c.n_kv, c.bits, c.symmetric, c.max_pages, c.num_pages = 4, 2, 8, True, 2, 8; "
+CACHE += "[c.register_buffer(n, t(4, 2, dtype=i32)) for n in ('length', 'page_table')]; "
+# each lacks elements that a kernel would read or write
+SHORT = [
+    "ops.lowrank_project(t(4, 64), t(32, 64), t(31))",
+    "ops.lowrank_project(t(4, 64), t(32, 64), residual=t(3, 32))",
+    "ops.lowrank_pair((t(4, 64), t(4, 64)), [t(16, 64)] * 2, [t(16), t(15)], [t(32, 16)] * 2, [None] * 2)",
+    "ops.lowrank_pair((t(4, 64), t(4, 64)), [t(16, 64)] * 2, [None] * 2, [t(32, 16)] * 2, [t(32), t(16)])",
+    "ops.gate_mlp_fused(t(4, 64), t(16, 64), t(8), t(8, 16), None)",
+    "ops.gate_mlp_fused(t(4, 64), t(16, 64), None, t(8, 16), t(4))",
+    "ops.gate_fused(t(4, 64), t(8, 64), t(7))",
+    "ops.gate_fused(t(4, 64), t(8, 64), expert_mask=t(7, dtype=f32))",
+    "ops.gate_fused(logits=t(4, 8, dtype=f32), correction=t(4, dtype=f32))",
+    "ops.gate_fused(logits=t(4, 8, dtype=f32), slot_base=t(4, dtype=i32))",
+    "ops.dispatch_loss(ops.GateResult(None, t(4, 2, dtype=i32), t(4, 1, dtype=f32), t(4, 2, dtype=i32), t(2, 8, dtype=i32), t(8, dtype=f32), None), 8, 4)",
+    "ops.dispatch_loss(ops.GateResult(None, t(4, 2, dtype=i32), t(4, 2, dtype=f32), t(4, 2, dtype=i32), t(2, 4, dtype=i32), t(8, dtype=f32), None), 8, 4)",
+    "ops.quant_block_pair(t(4, 64), t(4, 64), 32, 0, 255, False, params_in=t(1, 2, dtype=f32))",
+    CACHE + "c.decode_attention_h2o(t(4, 8, 128), t(7, 32, dtype=f32), (t(4, 8, 32, dtype=torch.float16), t(4, 8, 2, dtype=f32)))",
+    CACHE + "c.decode_attention_h2o(t(4, 8, 128), t(8, 32, dtype=f32), (t(3, 8, 32, dtype=torch.float16), t(4, 8, 2, dtype=f32)))",
+    CACHE + "c.decode_attention_h2o(t(4, 8, 128), t(8, 32, dtype=f32), (t(4, 8, 32, dtype=torch.float16), t(4, 4, 2, dtype=f32)))",
+    CACHE + "c.decode_attention(t(4, 8, 128), scores=t(4, 4, 32, dtype=f32))",
+    CACHE + "c.compact_into(c, t(7, 4, dtype=i32), t(8, dtype=i32), True)",
+    CACHE + "c.compact_into(c, t(4, 4, dtype=i32), t(3, dtype=i32), False)",
+]
+CALLS = ZERO_WIDTH + SHORT
 
 
 @pytest.fixture(scope="module")
@@ -56,3 +82,8 @@ def answers():
 @pytest.mark.parametrize("call", ZERO_WIDTH)
 def test_zero_width(answers, call):
     assert answers[call].startswith("PikvError: ") and "last dimension" in answers[call], answers[call]
+
+
+@pytest.mark.parametrize("call", SHORT)
+def test_short_operands(answers, call):
+    assert answers[call].startswith("PikvError: ") and "are needed" in answers[call], answers[call]
