@@ -564,8 +564,9 @@ std::vector<int64_t> with_last(const at::Tensor& x, int64_t last) {
 // lowrank(x, w, bias, relu, residual, out_f32) -> [..., N]
 PyObject* lowrank(PyObject* const* a, Py_ssize_t) {
     const at::Tensor x = req(a[0], "x", at::kBFloat16), w = half_of(a[1], "w"), b = bias_of(a[2]), r = opt(a[4], "residual", at::kBFloat16);
-    if (x.dim() < 2 || w.dim() != 2 || w.size(1) != x.size(-1)) fail("w must be [N,%lld]", (long long)x.size(-1));
-    const int M = rows_of(x, "x"), K = (int)x.size(-1), N = (int)w.size(0);
+    const int M = rows_of(x, "x");
+    if (w.dim() != 2 || w.size(1) != x.size(-1)) fail("w must be [N,%lld]", (long long)x.size(-1));
+    const int K = (int)x.size(-1), N = (int)w.size(0);
     const bool f = truth(a[5]);
     holds(b, N, "bias"); holds(r, (int64_t)M * N, "residual");
     at::Tensor y = at::empty(with_last(x, N), on(x, f ? at::kFloat : at::kBFloat16));
