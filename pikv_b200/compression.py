@@ -155,10 +155,12 @@ class SVDCompressor(BaseCompressor):
 
     def _round_trip(self, keys: torch.Tensor, values: torch.Tensor):
         H, R = self.hidden_size, self.rank
+        down, up = (self.key_projector, self.value_projector), (self.key_reconstructor, self.value_reconstructor)
         if (keys.shape == values.shape and keys.dtype == values.dtype == torch.bfloat16 and keys.is_cuda and R % 16 == 0 and R <= 64
                 and H % 16 == 0 and H <= 4096 and keys.numel() >= self.PAIR_ROWS * H
+                and all((p.in_features, p.out_features) == (H, R) for p in down)       # layers a user has put in their place
+                and all((p.in_features, p.out_features) == (R, H) for p in up)
                 and type(self).project is SVDCompressor.project and type(self).reconstruct is SVDCompressor.reconstruct):
-            down, up = (self.key_projector, self.value_projector), (self.key_reconstructor, self.value_reconstructor)
             return ops.lowrank_pair((keys, values), [p.weight for p in down], [p.bias for p in down],
                                     [p.weight for p in up], [p.bias for p in up])
         return (self.reconstruct(self.project(keys, "key"), "key"),

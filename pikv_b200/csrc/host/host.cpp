@@ -580,27 +580,28 @@ PyObject* lowrank_pair(PyObject* const* a, Py_ssize_t) {
     at::Tensor x[2], w1[2], b1[2], w2[2], b2[2], y[2];
     const void *xp[2], *w1p[2], *b1p[2], *w2p[2], *b2p[2];
     void* yp[2];
-    int code = -1;
+    bool half = true;                          // the kernel takes one bias type: fp32 unless all are bf16 (exact either way)
     for (int i = 0; i < 2; ++i) {
         x[i] = req(a[i], "x", at::kBFloat16);
         w1[i] = half_of(a[2 + i], "w1"); b1[i] = bias_of(a[4 + i]);
         w2[i] = half_of(a[6 + i], "w2"); b2[i] = bias_of(a[8 + i]);
-        if (x[i].sizes() != x[0].sizes() || w1[i].sizes() != w1[0].sizes() || w2[i].sizes() != w2[0].sizes() || w1[i].size(1) != x[i].size(-1) ||
-            w2[i].size(1) != w1[i].size(0))
+        if (x[i].sizes() != x[0].sizes() || w1[i].dim() != 2 || w2[i].dim() != 2 || w1[i].sizes() != w1[0].sizes() || w2[i].sizes() != w2[0].sizes() ||
+            x[i].dim() < 1 || w1[i].size(1) != x[i].size(-1) || w2[i].size(1) != w1[i].size(0))
             fail("lowrank_pair: x, w1 and w2 do not fit");
-        for (const at::Tensor* b : {&b1[i], &b2[i]}) {
-            if (!b->defined()) continue;
-            holds(*b, b == &b1[i] ? w1[i].size(0) : w2[i].size(0), "bias");
-            const int own = dtype_code(*b, "bias");
-            if (code >= 0 && own != code) fail("lowrank_pair: the biases must share their dtype");
-            code = own;
+        holds(b1[i], w1[i].size(0), "bias"); holds(b2[i], w2[i].size(0), "bias");
+        for (const at::Tensor* b : {&b1[i], &b2[i]}) half = half && (!b->defined() || b->scalar_type() == at::kBFloat16);
+    }
+    for (int i = 0; i < 2; ++i) {
+        if (!half) {
+            if (b1[i].defined()) b1[i] = b1[i].to(at::kFloat);
+            if (b2[i].defined()) b2[i] = b2[i].to(at::kFloat);
         }
         y[i] = at::empty(with_last(x[i], w2[i].size(0)), on(x[i], at::kBFloat16));
         xp[i] = ptr(x[i]); w1p[i] = ptr(w1[i]); b1p[i] = ptr(b1[i]); w2p[i] = ptr(w2[i]); b2p[i] = ptr(b2[i]); yp[i] = ptr(y[i]);
     }
     const int M = rows_of(x[0], "x"), K = (int)x[0].size(-1);
-    check(pikv_lowrank_pair(xp, w1p, b1p, w2p, b2p, code < 0 ? PIKV_F32 : code, yp, M, K, (int32_t)w1[0].size(0),
-                            (int32_t)w2[0].size(0), stream()), "pikv_lowrank_pair");
+    check(pikv_lowrank_pair(xp, w1p, b1p, w2p, b2p, half ? PIKV_BF16 : PIKV_F32, yp, M, K, (int32_t)w1[0].size(0), (int32_t)w2[0].size(0), stream()),
+          "pikv_lowrank_pair");
     return tuple(y[0], y[1]);
 }
 

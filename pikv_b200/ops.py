@@ -227,8 +227,8 @@ def lowrank_project(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tenso
 
 
 def lowrank_pair(xs, w1s, b1s, w2s, b2s):
-    """relu(x @ w1.T + b1) @ w2.T + b2 for the two (x, w1, b1, w2, b2) of K and V in one launch; bf16, biases all fp32,
-    all bf16 or None.  See pikv_lowrank_pair for the shapes it takes."""
+    """relu(x @ w1.T + b1) @ w2.T + b2 for the two (x, w1, b1, w2, b2) of K and V in one launch; bf16 x.  See
+    pikv_lowrank_pair for the shapes it takes."""
     return host().lowrank_pair(*xs, *w1s, *b1s, *w2s, *b2s)
 
 
