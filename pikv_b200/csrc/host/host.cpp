@@ -4,8 +4,9 @@
 // tensor allocation at a time) - several times what the kernels of a decode step take.
 //
 // Conventions: arguments are positional (METH_FASTCALL); a cache is passed as its module's buffer dict and its geometry;
-// None stands for an absent tensor.  Errors are raised as pikv_b200.PikvError.
+// None stands for an absent tensor.  Errors are raised as pikv_b200.PikvError, torch's own as what they are.
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/Exceptions.h>
 #include <ATen/ATen.h>
 #include <c10/core/GradMode.h>
 #include <c10/core/InferenceMode.h>
@@ -887,8 +888,8 @@ PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
         c10::NoGradGuard no_grad;
         return F(args, n);
     } catch (const Raised&) {
-    } catch (const std::exception& e) {
-        PyErr_SetString(PyErr_Occurred() ? PyExc_RuntimeError : g_error, e.what());
+    } catch (...) {                            // torch's own errors keep their types, the allocator's among them
+        if (!PyErr_Occurred()) torch::translate_exception_to_python(std::current_exception());
     }
     return nullptr;
 }

@@ -68,7 +68,8 @@ SHORT = [
     CACHE + "c.compact_into(c, t(7, 4, dtype=i32), t(8, dtype=i32), True)",
     CACHE + "c.compact_into(c, t(4, 4, dtype=i32), t(3, dtype=i32), False)",
 ]
-CALLS = ZERO_WIDTH + SHORT
+TORCH_ERROR = CACHE + "c.append(t(4, 256), t(4, 256), t((), dtype=i32), t(4, dtype=i32))"      # a dst_seq without a dimension
+CALLS = ZERO_WIDTH + SHORT + [TORCH_ERROR]
 
 
 @pytest.fixture(scope="module")
@@ -87,3 +88,7 @@ def test_zero_width(answers, call):
 @pytest.mark.parametrize("call", SHORT)
 def test_short_operands(answers, call):
     assert answers[call].startswith("PikvError: ") and "are needed" in answers[call], answers[call]
+
+
+def test_torch_errors_keep_their_type(answers):
+    assert answers[TORCH_ERROR].startswith("IndexError: "), answers[TORCH_ERROR]
