@@ -213,9 +213,18 @@ struct GateOut {
         if (given != Py_None) {
             if (!PyTuple_Check(given) || PyTuple_GET_SIZE(given) != 8) fail("gate: a result has eight tensors");
             at::Tensor* to[8] = {&probs, &idx, &w, &slot, &counts, &psum, &len, &workspace};
+            static const char* names[8] = {"probs", "topk_idx", "topk_w", "slot", "counts_k", "prob_sum", "new_len", "workspace"};
+            const bool whole[8] = {false, true, false, true, true, false, true, false};
+            const int64_t size[8] = {(int64_t)T * E, (int64_t)T * k, (int64_t)T * k, (int64_t)T * k, (int64_t)k * E, E, E, 0};
             for (int i = 0; i < 8; ++i) {
                 PyObject* o = PyTuple_GET_ITEM(given, i);
-                if (o != Py_None) *to[i] = THPVariable_Unpack(o);
+                if (o == Py_None) continue;
+                // raw pointers of them go to the kernels as outputs
+                if (!THPVariable_Check(o)) fail("the result's %s must be a CUDA tensor", names[i]);
+                const at::Tensor& t = THPVariable_Unpack(o);
+                if (!t.is_cuda() || !t.is_contiguous() || (i < 7 && t.scalar_type() != (whole[i] ? at::kInt : at::kFloat)))
+                    fail("the result's %s must be a contiguous CUDA tensor%s", names[i], i == 7 ? "" : whole[i] ? " of int32" : " of float32");
+                *to[i] = holds(t, size[i], names[i]);
             }
             return;
         }

@@ -69,7 +69,13 @@ SHORT = [
     CACHE + "c.compact_into(c, t(4, 4, dtype=i32), t(3, dtype=i32), False)",
 ]
 TORCH_ERROR = CACHE + "c.append(t(4, 256), t(4, 256), t((), dtype=i32), t(4, dtype=i32))"      # a dst_seq without a dimension
-CALLS = ZERO_WIDTH + SHORT + [TORCH_ERROR]
+# a result given to be written into, one of its members unfit
+RESULT = "r = ops.GateResult(t(4, 8, dtype=f32), t(4, 2, dtype=i32), t(4, 2, dtype=f32), t(4, 2, dtype=i32), t(2, 8, dtype=i32), t(8, dtype=f32), t(8, dtype=i32)); "
+MEMBERS = [RESULT + "r.%s = %s; ops.gate_fused(t(4, 64), t(8, 64), out=r)" % m for m in [
+    ("topk_idx", "__import__('numpy').zeros((4, 2), 'int32')"), ("new_len", "[0] * 8"), ("workspace", "bytearray(1 << 20)"),
+    ("topk_w", "t(4, 2)"), ("slot", "t(2, 4, dtype=i32).t()"), ("counts_k", "t(1, 8, dtype=i32)"),
+    ("probs", "torch.empty(4, 8)"), ("prob_sum", "t(4, dtype=f32)")]]
+CALLS = MEMBERS + ZERO_WIDTH + SHORT + [TORCH_ERROR]
 
 
 @pytest.fixture(scope="module")
@@ -92,3 +98,8 @@ def test_short_operands(answers, call):
 
 def test_torch_errors_keep_their_type(answers):
     assert answers[TORCH_ERROR].startswith("IndexError: "), answers[TORCH_ERROR]
+
+
+@pytest.mark.parametrize("call", MEMBERS)
+def test_members_of_a_given_result(answers, call):
+    assert answers[call].startswith("PikvError: ") and ("must be a" in answers[call] or "are needed" in answers[call]), answers[call]
