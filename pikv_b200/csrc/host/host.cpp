@@ -55,6 +55,13 @@ at::Tensor req(PyObject* o, const char* name, OptType type = c10::nullopt) {
 }
 at::Tensor opt(PyObject* o, const char* name, OptType type = c10::nullopt) { return o == Py_None ? at::Tensor() : req(o, name, type); }
 
+// a tensor that is written: a contiguous copy would take the update and be dropped
+at::Tensor written(PyObject* o, const char* name, OptType type) {
+    if (o == Py_None) return at::Tensor();
+    if (THPVariable_Check(o) && !THPVariable_Unpack(o).is_contiguous()) fail("%s is updated in place and must be contiguous", name);
+    return req(o, name, type);
+}
+
 // an fp32 vector, converted if it has another type
 at::Tensor f32(PyObject* o, const char* name) {
     at::Tensor t = opt(o, name);
@@ -441,7 +448,8 @@ PyObject* decode(PyObject* const* a, Py_ssize_t n) {
     at::Tensor acc, probs, step, scores;
     bool want_lse = true;
     if (h2o) {
-        acc = req(a[3], "acc", at::kFloat);
+        if (a[3] == Py_None) fail("acc must be a CUDA tensor");
+        acc = written(a[3], "acc", at::kFloat);
         probs = req(a[4], "probs", at::kHalf);
         step = req(a[5], "step_max", at::kFloat);
         p.probs16 = ptr(probs); p.step_max = ptr<float>(step);
@@ -450,7 +458,7 @@ PyObject* decode(PyObject* const* a, Py_ssize_t n) {
         holds(probs, (int64_t)p.B * p.n_q * probs.size(-1), "the workspace's probabilities");
         holds(step, (int64_t)p.B * p.n_q * step.size(-1), "the workspace's step maxima");
     } else {
-        scores = opt(a[4], "scores", at::kFloat);
+        scores = written(a[4], "scores", at::kFloat);
         want_lse = truth(a[3]) || scores.defined();
         p.scores = ptr<float>(scores);
         p.score_stride = scores.defined() ? (int32_t)scores.size(-1) : 0;
@@ -524,7 +532,7 @@ PyObject* compact(PyObject* const* a, Py_ssize_t) {
     for (int i = 0; i < 2; ++i) {
         if ((a[3 + i] == Py_None) != (a[5 + i] == Py_None)) fail("compact_into: give src_%s and dst_%s together", names[i], names[i]);
         from[i] = opt(a[3 + i], "src scores", at::kFloat);
-        to[i] = opt(a[5 + i], "dst scores", at::kFloat);
+        to[i] = written(a[5 + i], i ? "dst_ts" : "dst_acc", at::kFloat);
         if (!from[i].defined()) continue;
         if (from[i].numel() != segments * from[i].size(-1) || to[i].numel() != segments * to[i].size(-1))
             fail("compact_into: src_%s / dst_%s must have one row per segment (%lld)", names[i], names[i], (long long)segments);

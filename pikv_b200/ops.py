@@ -37,6 +37,13 @@ def _req(t: torch.Tensor, name: str, dtype=None) -> torch.Tensor:
     return t if t.is_contiguous() else t.contiguous()
 
 
+def _written(t: torch.Tensor, name: str, dtype) -> torch.Tensor:
+    """A tensor that is updated in place: a contiguous copy would take the update and be dropped."""
+    if isinstance(t, torch.Tensor) and not t.is_contiguous():
+        raise PikvError(f"{name} is updated in place and must be contiguous")
+    return _req(t, name, dtype)
+
+
 def _dtype_code(t: torch.Tensor, name: str) -> int:
     if t.dtype == torch.float32:
         return _lib.PIKV_F32
@@ -188,8 +195,8 @@ def linear_f32(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = 
 def h2o_accumulate(acc: torch.Tensor, ts: torch.Tensor, idx: Optional[torch.Tensor], w: torch.Tensor, now: float,
                    decay: float = 1.0, status: Optional[torch.Tensor] = None) -> None:
     """In place: acc[idx] += w ; ts[idx] = now (acc *= decay first when decay != 1)."""
-    acc = _req(acc, "acc", torch.float32)
-    ts = _req(ts, "ts", torch.float32)
+    acc = _written(acc, "acc", torch.float32)
+    ts = _written(ts, "ts", torch.float32)
     w = _req(w, "w", torch.float32)
     if idx is not None:
         idx = _req(idx, "idx", torch.int32)
@@ -211,7 +218,7 @@ def h2o_accumulate_attn(scores: torch.Tensor, lse: torch.Tensor, seq_len: Option
     """In place: acc[b*n_kv+h, pos] += sum over the group's query heads of exp(scores - lse)."""
     scores = _req(scores, "scores", torch.float32)
     lse = _req(lse, "lse", torch.float32)
-    acc = _req(acc, "acc", torch.float32)
+    acc = _written(acc, "acc", torch.float32)
     B, n_q, stride = scores.shape
     check(lib().pikv_h2o_accumulate_attn(_p(scores), stride, _p(lse), _p(seq_len), B, n_q, n_kv, _p(acc),
                                          acc.shape[-1], _stream()), "pikv_h2o_accumulate_attn")

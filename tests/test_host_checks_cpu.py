@@ -75,7 +75,17 @@ MEMBERS = [RESULT + "r.%s = %s; ops.gate_fused(t(4, 64), t(8, 64), out=r)" % m f
     ("topk_idx", "__import__('numpy').zeros((4, 2), 'int32')"), ("new_len", "[0] * 8"), ("workspace", "bytearray(1 << 20)"),
     ("topk_w", "t(4, 2)"), ("slot", "t(2, 4, dtype=i32).t()"), ("counts_k", "t(1, 8, dtype=i32)"),
     ("probs", "torch.empty(4, 8)"), ("prob_sum", "t(4, dtype=f32)")]]
-CALLS = MEMBERS + ZERO_WIDTH + SHORT + [TORCH_ERROR]
+# what is updated in place, as a strided view
+WRITTEN = [
+    CACHE + "c.decode_attention_h2o(t(4, 8, 128), t(8, 64, dtype=f32)[:, :32], (t(4, 8, 32, dtype=torch.float16), t(4, 8, 2, dtype=f32)))",
+    CACHE + "c.decode_attention(t(4, 8, 128), scores=t(4, 8, 64, dtype=f32)[:, :, :32])",
+    CACHE + "c.compact_into(c, t(8, 4, dtype=i32), t(8, dtype=i32), True, t(8, 32, dtype=f32), None, t(8, 64, dtype=f32)[:, :32], None)",
+    CACHE + "c.compact_into(c, t(8, 4, dtype=i32), t(8, dtype=i32), True, None, t(8, 32, dtype=f32), None, t(8, 64, dtype=f32)[:, :32])",
+    "ops.h2o_accumulate(t(64, dtype=f32)[::2], t(32, dtype=f32), None, t(32, dtype=f32), 1.0)",
+    "ops.h2o_accumulate(t(32, dtype=f32), t(64, dtype=f32)[::2], None, t(32, dtype=f32), 1.0)",
+    "ops.h2o_accumulate_attn(t(4, 8, 32, dtype=f32), t(4, 8, dtype=f32), None, 2, t(8, 64, dtype=f32)[:, :32])",
+]
+CALLS = WRITTEN + MEMBERS + ZERO_WIDTH + SHORT + [TORCH_ERROR]
 
 
 @pytest.fixture(scope="module")
@@ -103,3 +113,8 @@ def test_torch_errors_keep_their_type(answers):
 @pytest.mark.parametrize("call", MEMBERS)
 def test_members_of_a_given_result(answers, call):
     assert answers[call].startswith("PikvError: ") and ("must be a" in answers[call] or "are needed" in answers[call]), answers[call]
+
+
+@pytest.mark.parametrize("call", WRITTEN)
+def test_strided_views_that_are_written(answers, call):
+    assert answers[call].startswith("PikvError: ") and "must be contiguous" in answers[call], answers[call]
