@@ -8,13 +8,15 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/Exceptions.h>
 #include <ATen/ATen.h>
+#include <ATen/EmptyTensor.h>
 #include <c10/core/GradMode.h>
 #include <c10/core/InferenceMode.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <ATen/ops/empty.h>
 #include <ATen/ops/empty_like.h>
 #include <c10/cuda/CUDAStream.h>
-#include <c10/core/StorageImpl.h>
 
 #include <cstdarg>
 #include <exception>
@@ -119,25 +121,20 @@ float real(PyObject* o) {
 }
 bool truth(PyObject* o) { return PyObject_IsTrue(o) == 1; }
 
-// ---- several small outputs in one allocation --------------------------------------------------------------
-// Pieces of one storage, each at a 256-byte boundary: a routing result is seven tensors of a few hundred bytes.
-struct Pack {
-    at::Tensor like, buf;
-    int64_t used = 0;
-    explicit Pack(const at::Tensor& t) : like(t) {}
-    int64_t add(int64_t bytes) {
-        const int64_t at = used;
-        used += (bytes + 255) & ~int64_t(255);
-        return at;
+// ---- small outputs ------------------------------------------------------------------------------------------
+// at::empty on the device of `like`, straight from the caching allocator where nothing watches the dispatcher: a routing
+// result is seven tensors of a few hundred bytes, and a decode batch's call is about as long as its host path (64 tokens:
+// 16.4 us of host in a call of 16.5 us, 17.9 and 18.0 with at::empty).
+struct Fresh {
+    at::TensorOptions options;
+    c10::Allocator* allocator = nullptr;
+    explicit Fresh(const at::Tensor& like) : options(at::TensorOptions().device(like.device())) {
+        if (like.device().index() == c10::cuda::current_device() && !c10::impl::TorchDispatchModeTLS::any_modes_set())
+            allocator = c10::cuda::CUDACachingAllocator::get();
     }
-    void allocate() { buf = at::empty({used}, on(like, at::kByte)); }
-    at::Tensor piece(int64_t at, at::ScalarType type, at::IntArrayRef sizes) {
-        c10::Storage storage = buf.storage();
-        at::Tensor t = at::detail::make_tensor<c10::TensorImpl>(std::move(storage), c10::DispatchKeySet(c10::DispatchKey::CUDA),
-                                                                c10::scalarTypeToTypeMeta(type));
-        t.unsafeGetTensorImpl()->set_sizes_contiguous(sizes);
-        t.unsafeGetTensorImpl()->set_storage_offset(buf.storage_offset() * 1 + at / (int64_t)c10::elementSize(type));
-        return t;
+    at::Tensor operator()(at::ScalarType type, at::IntArrayRef sizes) const {
+        if (!allocator) return at::empty(sizes, options.dtype(type));
+        return at::Tensor(at::detail::empty_generic(sizes, allocator, c10::DispatchKeySet(c10::DispatchKey::CUDA), type, c10::nullopt));
     }
 };
 
@@ -235,18 +232,15 @@ struct GateOut {
             }
             return;
         }
-        Pack p(like);
-        const int64_t Tk = (int64_t)T * k;
-        const int64_t o0 = want_probs ? p.add((int64_t)T * E * 4) : 0, o1 = p.add(Tk * 4), o2 = p.add(Tk * 4), o3 = p.add(Tk * 4),
-                      o4 = p.add((int64_t)k * E * 4), o5 = p.add(E * 4), o6 = p.add(E * 4);
-        p.allocate();
-        if (want_probs) probs = p.piece(o0, at::kFloat, {T, E});
-        idx = p.piece(o1, at::kInt, {T, k});
-        w = p.piece(o2, at::kFloat, {T, k});
-        slot = p.piece(o3, at::kInt, {T, k});
-        counts = p.piece(o4, at::kInt, {k, E});
-        psum = p.piece(o5, at::kFloat, {E});
-        len = p.piece(o6, at::kInt, {E});
+        // a storage each: a caller may keep, save or resize one without the others
+        const Fresh fresh(like);
+        if (want_probs) probs = fresh(at::kFloat, {T, E});
+        idx = fresh(at::kInt, {T, k});
+        w = fresh(at::kFloat, {T, k});
+        slot = fresh(at::kInt, {T, k});
+        counts = fresh(at::kInt, {k, E});
+        psum = fresh(at::kFloat, {E});
+        len = fresh(at::kInt, {E});
     }
     void fill(pikv_gate_params& g) const {
         g.probs = ptr<float>(probs); g.topk_idx = ptr<int32_t>(idx); g.topk_w = ptr<float>(w); g.slot = ptr<int32_t>(slot);
