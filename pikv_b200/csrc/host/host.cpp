@@ -695,7 +695,7 @@ struct MoeWalk {
            NTYPES };
 
     const at::Tensor& tensor(PyObject* o, at::IntArrayRef sizes, at::ScalarType type = at::kFloat) const {
-        need(THPVariable_Check(o));
+        need(THPVariable_CheckExact(o));               // a subclass may have calls of its own
         const at::Tensor& t = THPVariable_Unpack(o);
         need(t.layout() == at::kStrided && t.device() == device && t.scalar_type() == type && t.sizes() == sizes && t.is_contiguous() &&
              (!t.is_inference() || c10::InferenceMode::is_enabled()) && !t.unsafeGetTensorImpl()->is_python_dispatch() &&

@@ -15,6 +15,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 from torch.autograd import forward_ad as _fwd_ad
 from torch.nn.modules import module as _module
+from torch.utils._device import DeviceContext
 
 from ._lib import host
 from .config import config
@@ -109,6 +110,11 @@ class KVCache(nn.Module):
     def change_scheduling_policy(self, new_policy: SchedulingPolicy):
         if self.use_scheduling and self.scheduling_manager is not None:
             self.scheduling_manager.change_policy(new_policy)
+
+
+def _calls_watched() -> bool:
+    """Whether a torch function mode sees the modules' calls; a default device is one that only concerns new tensors."""
+    return any(type(torch._C._get_function_stack_at(i)) is not DeviceContext for i in range(torch._C._len_torch_function_stack()))
 
 
 class PiKVMoE(nn.Module):
@@ -223,10 +229,10 @@ class PiKVMoE(nn.Module):
 
     def _fused(self, x):
         """(weighted expert sum, logits or None, auxiliary loss) by the fused kernels, or None where the modules have to run: the
-        kernels see neither tracers, function transforms and tangents nor hooks and replaced modules."""
+        kernels see neither tracers, function modes, function transforms and tangents nor hooks and replaced modules."""
         if (torch.is_autocast_enabled() or _module._has_any_global_hook() or _fwd_ad._current_level >= 0 or torch.jit.is_tracing()
                 or torch._C._functorch.peek_interpreter_stack() is not None or torch._C._len_torch_dispatch_stack()
-                or torch.compiler.is_compiling()):
+                or torch.compiler.is_compiling() or _calls_watched()):
             return None
         if self._host_ptrs is None:
             self._host_ptrs = self.cache_ptrs.tolist()
