@@ -97,8 +97,8 @@ def gate_fused(act: Optional[torch.Tensor] = None, w2: Optional[torch.Tensor] = 
     phase 2 (slot finalisation only, same arguments, ordered after phase 1 by the caller) keep their state
     in out.workspace, which is allocated on first use and must not be shared between batches in flight.
     """
-    res = host().gate(act, w2, b2, logits, top_k, expert_mask, mask_mode, correction, temperature, renorm_eps, capacity,
-                      slot_base, want_probs, None if out is None else out.tensors(), phase)
+    res = host().gate(act, w2, b2, logits, top_k, expert_mask, mask_mode, correction, temperature, renorm_eps, int(capacity),
+                      slot_base, want_probs, None if out is None else out.tensors(), int(phase))
     if out is None:
         return GateResult(*res)
     out.workspace = res[7]
@@ -112,7 +112,7 @@ def gate_mlp_fused(x: torch.Tensor, w1: torch.Tensor, b1: Optional[torch.Tensor]
                    want_probs: bool = True, out: Optional[GateResult] = None) -> GateResult:
     """The whole gate net on tensor cores: relu(x @ w1.T + b1) @ w2.T + b2, then the tail of gate_fused (same
     keyword arguments and result); bf16 x [T,K], w1 [H,K], w2 [E,H].  See pikv_gate_mlp_fused."""
-    res = host().gate_mlp(x, w1, b1, w2, b2, top_k, expert_mask, mask_mode, correction, temperature, renorm_eps, capacity,
+    res = host().gate_mlp(x, w1, b1, w2, b2, top_k, expert_mask, mask_mode, correction, temperature, renorm_eps, int(capacity),
                           slot_base, want_probs, None if out is None else out.tensors(), 0, 0, 0, 0.0)
     return GateResult(*res) if out is None else out
 
@@ -126,7 +126,7 @@ def gate_mlp_dense(x: torch.Tensor, w1: torch.Tensor, b1: Optional[torch.Tensor]
                    capacity: int = 0):
     """gate_mlp_fused on x [..., K] and dispatch_loss (`rows` = capacity dimension of the dense tensors) in one call: the
     dense tensors are cleared beside the tensor-core work.  Returns (gate result, (dispatch, combine, aux))."""
-    res = host().gate_mlp(x, w1, b1, w2, b2, top_k, expert_mask, mask_mode, None, 1.0, renorm_eps, capacity, None, True, None,
+    res = host().gate_mlp(x, w1, b1, w2, b2, top_k, expert_mask, mask_mode, None, 1.0, renorm_eps, int(capacity), None, True, None,
                           rows, position_mode, BALANCE[balance], coefficient)
     return GateResult(*res[:8]), res[8:]
 

@@ -109,7 +109,7 @@ class PagedKVCache(torch.nn.Module):
         append kernel.  Sequences are the experts.  Returns the gate result."""
         res = host().route_append(self._buffers, self.num_seqs, self.n_kv, self.bits, self.symmetric, self.max_pages,
                                   self.num_pages, act, w2, b2, k, v, top_k, None, 0, None, 1.0, 0.0,
-                                  self.capacity if capacity is None else capacity, slot_base, want_probs,
+                                  self.capacity if capacity is None else int(capacity), slot_base, want_probs,
                                   None if out is None else out.tensors())
         if out is None:
             return ops.GateResult(*res)
