@@ -399,14 +399,15 @@ PyObject* gate_mlp(PyObject* const* a, Py_ssize_t) {
     return tuple(out.probs, out.idx, out.w, out.slot, out.counts, out.psum, out.len, out.workspace, dense.d, dense.c, dense.aux);
 }
 
-// dispatch_loss(topk_idx, topk_w, slot, counts_k, prob_sum, E, rows, position_mode, balance, coefficient)
+// dispatch_loss(topk_idx, topk_w, slot, counts_k, prob_sum, E, rows, position_mode, balance, coefficient); no loss without prob_sum
 PyObject* dispatch_loss(PyObject* const* a, Py_ssize_t) {
-    const at::Tensor idx = req(a[0], "topk_idx", at::kInt), w = req(a[1], "topk_w", at::kFloat), slot = req(a[2], "slot", at::kInt),
-                     counts = req(a[3], "counts_k", at::kInt), psum = req(a[4], "prob_sum", at::kFloat);
+    const at::Tensor idx = req(a[0], "topk_idx", at::kInt), w = req(a[1], "topk_w", at::kFloat), slot = opt(a[2], "slot", at::kInt),
+                     counts = opt(a[3], "counts_k", at::kInt), psum = opt(a[4], "prob_sum", at::kFloat);
     if (idx.dim() != 2) fail("topk_idx must be [T,k]");
     const int T = (int)idx.size(0), k = (int)idx.size(1), E = (int)num(a[5]);
     holds(w, idx.numel(), "topk_w"); holds(slot, idx.numel(), "slot"); holds(counts, (int64_t)k * E, "counts_k"); holds(psum, E, "prob_sum");
     Dense dense(a + 6, idx, {T}, E);
+    if (!psum.defined()) dense.o.aux = nullptr, dense.aux = at::Tensor();
     check(pikv_dispatch_loss(ptr<int32_t>(idx), ptr<float>(w), ptr<int32_t>(slot), ptr<int32_t>(counts), ptr<float>(psum), T, E, k, &dense.o, stream()),
           "pikv_dispatch_loss");
     return tuple(dense.d, dense.c, dense.aux);

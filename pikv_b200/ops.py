@@ -139,7 +139,7 @@ def dispatch_scatter(g: GateResult, num_experts: int, capacity: int, position_mo
 def dispatch_loss(g: GateResult, num_experts: int, capacity: int, position_mode: int = 0, balance: Optional[str] = None,
                   coefficient: float = 0.0):
     """dispatch_scatter and the router's auxiliary loss (0-dim): the base term of core/single/pikv_routing.py:155-159
-    plus `coefficient` times the balance term of :185-222."""
+    plus `coefficient` times the balance term of :185-222.  The loss is None for a result without probability sums."""
     return host().dispatch_loss(g.topk_idx, g.topk_w, g.slot, g.counts_k, g.prob_sum, num_experts, capacity, position_mode,
                                 BALANCE[balance], coefficient)
 
