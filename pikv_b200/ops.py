@@ -169,10 +169,10 @@ def quant_block_pair(k: torch.Tensor, v: torch.Tensor, group_size: int, qmin: in
                      params_in: Optional[torch.Tensor] = None, sample_count: Optional[torch.Tensor] = None,
                      count_add: float = 0.0):
     """quant_block on K and V [..., H] of one forward, both tensors in each launch when they agree in shape and dtype.
-    Returns (dk, dv in the input's dtype, mean squared error of V's last group as a 0-dim tensor); sample_count (a
-    one-element counter) grows by count_add."""
-    if sample_count is not None and (sample_count.dtype != torch.float32 or sample_count.device != k.device):
-        sample_count += count_add                     # not a word the kernel can add to
+    Returns (dk, dv in the input's dtype, mean squared error of V's last group as a 0-dim tensor); sample_count grows by
+    count_add."""
+    if sample_count is not None and (sample_count.dtype != torch.float32 or sample_count.device != k.device or sample_count.numel() != 1):
+        sample_count += count_add                     # not one word that the kernel can add to
         sample_count = None
     if k.shape != v.shape or k.dtype != v.dtype:
         kf, vf = k.reshape(-1, k.shape[-1]), v.reshape(-1, v.shape[-1])
