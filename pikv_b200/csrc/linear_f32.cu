@@ -1,23 +1,28 @@
 // fp32 linear layer on the tensor cores: out[M,N] = x[M,K] . w[N,K]^T + bias, every operand as two f16 limbs.
 //
 // A row is scaled by a power of two so that its largest magnitude lies in [2^14, 2^15) and split into hi = f16(v) and
-// lo = f16(v - hi): v is met to 2^-24 of itself (2^-38 of the row's largest where lo is subnormal).  The product is
-// hi.hi + (hi.lo + lo.hi), what is left out, lo.lo, is below 2^-24 of each term.  The tensor cores' sums truncate, so
+// lo = f16(2^11 (v - hi)): hi + 2^-11 lo meets v to 2^-23 of itself down to 2^-27 of the row's largest.  (With lo at v's own
+// scale an entry of 2^-18 of the largest lost bits and one of 2^-39 vanished, which shows where the large entry meets a zero:
+// relative error 1.3e-5 at a spread of 2^24, 0.7 at 2^40, against 2.9e-7 of fp32 sums.)  The product is
+// hi.hi + 2^-11 (hi.lo + lo.hi), what is left out, lo.lo, is at most 2^-22 of each term.  The tensor cores' sums truncate, so
 // each bracket has an fp32 accumulator of its own and each half of K another pair; the epilogue adds the four.
-// Rows with an infinity, a NaN or a largest magnitude outside 2^-60 .. 2^60 are marked (scale 0) and their outputs formed
-// by plain fp32 sums in the epilogue.
+// Rows with an entry that the limbs miss by more than 2^-23 of itself (one entry in 60 million of normal inputs), an infinity,
+// a NaN or a largest magnitude outside 2^-60 .. 2^60 are marked (scale 0) and their outputs formed by fp32 sums.
 //
-//   lin_split_kernel   one warp per row of w and x: limbs [rows, hi K | lo K] and the inverse scales
+//   lin_split_kernel   one warp per row of w and x: limbs [rows, hi K | lo K], the inverse scales and whether
+//                      each CTA marked a row
 //   lin_gemm_kernel    persistent, one CTA per SM.  Items are 128 x 128 outputs, row tiles innermost, contiguous per CTA:
 //                      w's tile stays in shared memory (hi and lo of a 64-wide k block next to each other: one MMA of
 //                      N = 256 takes both products of an x hi block), x blocks stream through a ring.  Two accumulator
 //                      pairs of 256 columns, one per half of K: sixteen epilogue warps, 32 x 32 outputs each, keep the
 //                      first half's sums in registers while the second is computed, turn their patches in shared
 //                      memory and store whole rows (N is odd in earnest, so neither TMA nor vector stores apply).
+//                      At its end all CTAs share out the outputs of marked rows, if there are any (lin_fix).
 //
-// 1024 x 256 -> 50257: 110 us for the GEMM and 26 for the splits (135 us a call, 140 with eight epilogue warps; cuBLAS's
-// fp32 kernel and its bias pass 716), relative error 2.0e-7 against 64 bits (cuBLAS 2.9e-7; one accumulator for all of K 3.5e-7).  The 79 GFLOP of the three
-// products would take 48 us at the measured bf16 rate and the output 32 us of HBM.
+// 1024 x 256 -> 50257: 137 us a call, about 28 of them the splits (134 with the low limb unscaled and entries lost; cuBLAS's fp32
+// kernel and its bias pass 715), relative error 2.0e-7 against 64 bits (cuBLAS 2.9e-7; one accumulator for all of K 3.5e-7).
+// A marked row of w adds 6 us, one of x 45, all 1024 of x 3.2 ms.  The 79 GFLOP of the three products would take 48 us at the
+// measured bf16 rate and the output 32 us of HBM.
 #include "tc_common.cuh"
 
 namespace pikv {
@@ -26,6 +31,9 @@ constexpr int LIN_BN = 128, LIN_BLOCK = 128 * 128;       // outputs per tile; by
 constexpr int LIN_MAX_KB = 4, LIN_STAGES = 4;
 constexpr int LIN_EPI_WARPS = 16, LIN_THREADS = 64 + 32 * LIN_EPI_WARPS;
 constexpr int LIN_PATCH = 16 * 33 * 4;
+constexpr float LIN_LO_SCALE = 2048.f;
+constexpr int LIN_FIX_LIST = 2048, LIN_FIX_GROUP = 8;
+static_assert(LIN_FIX_GROUP * 64 * LIN_MAX_KB * 4 + (LIN_FIX_LIST + LIN_THREADS + 2) * 4 <= LIN_STAGES * LIN_BLOCK, "linear_f32: marked rows");
 constexpr int LIN_SMEM = 2 * LIN_MAX_KB * LIN_BLOCK + LIN_STAGES * LIN_BLOCK + LIN_EPI_WARPS * LIN_PATCH + 256 + 1024;
 static_assert(LIN_SMEM <= 227 * 1024, "linear_f32: shared memory");
 
@@ -33,19 +41,24 @@ __device__ unsigned g_linear_error = 0;                  // sticky: set when a b
 
 struct LinArgs {
     const float *x, *w, *bias, *sx, *sw;
+    const int *mx, *mw;                                  // whether a CTA of the split marked a row
+    int ctas_x, ctas_w;
     float* out;
     int M, N, K, mtiles;
     long long items;
 };
 
-__global__ void __launch_bounds__(256) lin_split_kernel(const float* __restrict__ src, int rows, int K, __half* __restrict__ limbs, float* __restrict__ inv) {
+__global__ void __launch_bounds__(256, 8) lin_split_kernel(const float* __restrict__ src, int rows, int K, __half* __restrict__ limbs, float* __restrict__ inv,
+                                                         int* __restrict__ marked) {
     dependency_release();
     dependency_wait();
     const int lane = threadIdx.x & 31;
     const int words = K / 4;                             // at most 64: two per lane
+    bool marked_any = false;
     for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows; r += gridDim.x * blockDim.x / 32) {
         float4 v[2] = {};
         float m = 0.f;
+        uint32_t least = 0xffffffffu;                    // bits of the smallest magnitude but zero, less one
         bool bad = false;
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
@@ -55,6 +68,7 @@ __global__ void __launch_bounds__(256) lin_split_kernel(const float* __restrict_
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 m = fmaxf(m, a[j]);
+                least = min(least, __float_as_uint(a[j]) - 1u);
                 bad |= !(a[j] <= 3.402823466e38f);
             }
         }
@@ -62,7 +76,6 @@ __global__ void __launch_bounds__(256) lin_split_kernel(const float* __restrict_
         const int e = (int)(__float_as_uint(m) >> 23) - 127;           // 2^e <= m < 2^(e+1)
         bad = __any_sync(0xffffffffu, bad) || e > 60 || (e < -60 && m != 0.f);
         const float up = bad ? 0.f : m == 0.f ? 1.f : __uint_as_float((uint32_t)(127 + 14 - e) << 23);
-        if (lane == 0) inv[r] = bad ? 0.f : m == 0.f ? 1.f : __uint_as_float((uint32_t)(127 - 14 + e) << 23);
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
             const int i = lane + 32 * q;
@@ -73,19 +86,117 @@ __global__ void __launch_bounds__(256) lin_split_kernel(const float* __restrict_
             for (int j = 0; j < 4; ++j) {
                 const float s = bad ? 0.f : a[j] * up;
                 h[j] = __float2half_rn(s);
-                l[j] = __float2half_rn(s - __half2float(h[j]));
+                l[j] = __float2half_rn((s - __half2float(h[j])) * LIN_LO_SCALE);            // exact before it is rounded
             }
             __half* to = limbs + (size_t)r * 2 * K + 4 * i;
             *reinterpret_cast<uint2*>(to) = *reinterpret_cast<const uint2*>(h);
             *reinterpret_cast<uint2*>(to + K) = *reinterpret_cast<const uint2*>(l);
         }
+        // at and above 2^-13 both limbs are normal f16 numbers and the entry is met; below (2^-27 of the largest) it is looked at
+        if (!bad && __any_sync(0xffffffffu, least < (uint32_t)max(0, 127 + e - 27) << 23)) {
+            bool missed = false;
+#pragma unroll 1
+            for (int i = lane; i < K; i += 32) {
+                const float a = src[(size_t)r * K + i], s = a * up, rest = s - __half2float(__float2half_rn(s));
+                // met to 2^-23, and with a low limb of 2^-11 at most, as the products of two are left out; a scaled entry below
+                // 2^-126 was rounded itself, perhaps to zero
+                missed |= fabsf(s) < 1.f / 8192.f && (fabsf(rest - __half2float(__float2half_rn(rest * LIN_LO_SCALE)) / LIN_LO_SCALE) > fabsf(s) / 8388608.f ||
+                                                      fabsf(rest) > fabsf(s) / LIN_LO_SCALE || (s == 0.f && a != 0.f));
+            }
+            bad = __any_sync(0xffffffffu, missed);
+        }
+        marked_any |= bad;
+        if (lane == 0) inv[r] = bad ? 0.f : m == 0.f ? 1.f : __uint_as_float((uint32_t)(127 - 14 + e) << 23);
     }
+    const int marks = __syncthreads_or(marked_any);
+    if (threadIdx.x == 0) marked[blockIdx.x] = marks;
 }
 
-__device__ __noinline__ float lin_plain(const LinArgs& a, int m, int n) {
-    float s = 0.f;
-    for (int k = 0; k < a.K; ++k) s = fmaf(a.x[(size_t)m * a.K + k], a.w[(size_t)n * a.K + k], s);
-    return s;
+// ---- outputs of marked rows ----
+// The lane's share of eight sums over a warp: the sum of v[i] ends in the lanes with (lane >> 2) == the bits of i reversed
+__device__ __forceinline__ float lin_sum8(float (&v)[8], int lane) {
+#pragma unroll
+    for (int half = 4; half > 0; half >>= 1) {
+        const bool upper = lane & (4 * half);
+#pragma unroll
+        for (int i = 0; i < half; ++i) {
+            const float send = upper ? v[i] : v[half + i];
+            v[i] = (upper ? v[half + i] : v[i]) + __shfl_xor_sync(0xffffffffu, send, 4 * half);
+        }
+    }
+    float s = v[0];
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    return s + __shfl_xor_sync(0xffffffffu, s, 1);
+}
+
+// The outputs of the marked rows of x and of w, by all CTAs: eight marked rows in shared memory, a warp per row of the other operand
+__device__ __noinline__ void lin_fix(const LinArgs& a, unsigned char* smem) {
+    float (*group)[64 * LIN_MAX_KB] = reinterpret_cast<float (*)[64 * LIN_MAX_KB]>(smem);
+    int* list = reinterpret_cast<int*>(group + LIN_FIX_GROUP);             // rows, at most LIN_FIX_LIST
+    int* slots = list + LIN_FIX_LIST;                                      // CTAs of the split, at most LIN_THREADS
+    int &listed = slots[LIN_THREADS], &found = slots[LIN_THREADS + 1];
+    const int tid = threadIdx.x, lane = tid & 31, K = a.K;
+    const long long worker = (long long)blockIdx.x * (LIN_THREADS / 32) + (tid >> 5), workers = (long long)gridDim.x * (LIN_THREADS / 32);
+    for (int side = 0; side < 2; ++side) {
+        const float *own = side == 0 ? a.x : a.w, *other = side == 0 ? a.w : a.x, *inv = side == 0 ? a.sx : a.sw;
+        const int* marked = side == 0 ? a.mx : a.mw;
+        const int count = side == 0 ? a.M : a.N, others = side == 0 ? a.N : a.M, ctas = side == 0 ? a.ctas_x : a.ctas_w, stride = ctas * 8;
+        auto flush = [&]() {
+            for (int g0 = 0; g0 < listed; g0 += LIN_FIX_GROUP) {
+                const int n = min(LIN_FIX_GROUP, listed - g0);
+                __syncthreads();
+                for (int i = tid; i < LIN_FIX_GROUP * K; i += LIN_THREADS) group[i / K][i % K] = i / K < n ? own[(size_t)list[g0 + i / K] * K + i % K] : 0.f;
+                __syncthreads();
+                for (long long o = worker; o < others; o += workers) {
+                    float v[LIN_FIX_GROUP] = {};
+#pragma unroll
+                    for (int c = 0; c < LIN_MAX_KB; ++c) {
+                        if (64 * c >= K) break;
+                        const float2 u = __ldg(reinterpret_cast<const float2*>(other + (size_t)o * K + 64 * c) + lane);
+#pragma unroll
+                        for (int q = 0; q < LIN_FIX_GROUP; ++q) {
+                            const float2 t = *(reinterpret_cast<const float2*>(&group[q][64 * c]) + lane);
+                            v[q] = fmaf(u.x, t.x, fmaf(u.y, t.y, v[q]));
+                        }
+                    }
+                    const float s = lin_sum8(v, lane);
+                    const int q = (lane >> 4 & 1) * 4 + (lane >> 3 & 1) * 2 + (lane >> 2 & 1);
+                    if ((lane & 3) == 0 && q < n) {
+                        const int mine = list[g0 + q];
+                        const size_t m = side == 0 ? (size_t)mine : (size_t)o;
+                        const int col = side == 0 ? (int)o : mine;
+                        a.out[m * a.N + col] = s + (a.bias ? __ldg(a.bias + col) : 0.f);
+                    }
+                }
+            }
+            __syncthreads();
+            if (tid == 0) listed = 0;
+            __syncthreads();
+        };
+        if (tid == 0) listed = 0;
+        __syncthreads();
+        for (int c0 = 0; c0 < ctas; c0 += LIN_THREADS) {
+            const bool has = c0 + tid < ctas && marked[c0 + tid] != 0;
+            if (tid == 0) found = 0;
+            if (!__syncthreads_or(has)) continue;
+            if (has) slots[atomicAdd(&found, 1)] = c0 + tid;
+            __syncthreads();
+            for (int q = 0; q < found; ++q) {
+                // this CTA of the split had the rows c * 8 + (0 .. 7), and again every `stride` rows
+                const long long c = slots[q], mine = (count - c * 8 + stride - 1) / stride * 8;
+                for (long long i0 = 0; i0 < mine; i0 += LIN_THREADS) {
+                    const long long i = i0 + tid, r = c * 8 + (i & 7) + (i >> 3) * stride;
+                    if (i < mine && r < count && inv[r] == 0.f) list[atomicAdd(&listed, 1)] = (int)r;
+                    __syncthreads();
+                    const int have = listed;
+                    __syncthreads();                     // before the next row is listed
+                    if (have > LIN_FIX_LIST - LIN_THREADS) flush();
+                }
+            }
+            __syncthreads();                             // `found` and `slots` have been read
+        }
+        if (listed) flush();
+    }
 }
 
 __global__ void __launch_bounds__(LIN_THREADS, 1) lin_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w,
@@ -119,7 +230,7 @@ __global__ void __launch_bounds__(LIN_THREADS, 1) lin_gemm_kernel(const __grid_c
     dependency_wait();
     const long long first = a.items * blockIdx.x / gridDim.x, last = a.items * (blockIdx.x + 1) / gridDim.x;
     const int first_kbs = (kbs + 1) / 2;                 // k blocks of the first half
-    bool failed = false;
+    bool failed = false, marks = false;
 
     if (warp == 0) {
         LrRing r;
@@ -194,6 +305,9 @@ __global__ void __launch_bounds__(LIN_THREADS, 1) lin_gemm_kernel(const __grid_c
         const int lg = warp & 3, side = (warp - 2) >> 2; // tensor-memory lane group, and which 32 of the 128 columns
         float* patch = patches + (size_t)(warp - 2) * (LIN_PATCH / 4);
         int local = 0;
+        // marked rows anywhere, read while the first sums are computed
+        for (int i = threadIdx.x - 64; i < a.ctas_x; i += 32 * LIN_EPI_WARPS) marks |= a.mx[i] != 0;
+        for (int i = threadIdx.x - 64; i < a.ctas_w; i += 32 * LIN_EPI_WARPS) marks |= a.mw[i] != 0;
         for (long long item = first; item < last && !failed; ++item, ++local) {
             const int nt = (int)(item / a.mtiles), mt = (int)(item % a.mtiles);
             const int m0 = mt * 128 + lg * 32, n0 = nt * LIN_BN + side * 32;
@@ -212,7 +326,7 @@ __global__ void __launch_bounds__(LIN_THREADS, 1) lin_gemm_kernel(const __grid_c
                 float v[32];
                 lr_tmem_ld32(taddr + pair * 256 + 128, v);
 #pragma unroll
-                for (int i = 0; i < 32; ++i) acc[i] += v[i];
+                for (int i = 0; i < 32; ++i) acc[i] = fmaf(v[i], 1.f / LIN_LO_SCALE, acc[i]);
                 lr_tmem_ld32(taddr + pair * 256, v);
 #pragma unroll
                 for (int i = 0; i < 32; ++i) acc[i] += v[i];
@@ -237,10 +351,8 @@ __global__ void __launch_bounds__(LIN_THREADS, 1) lin_gemm_kernel(const __grid_c
                     }
                 } else {
                     for (int r = h; r < min(rows, h + 16); ++r) {
-                        const float s = __shfl_sync(0xffffffffu, sx, r);
-                        if (!in) continue;
-                        const float o = s == 0.f || sw == 0.f ? lin_plain(a, m0 + r, n) : patch[(r - h) * 33 + lane] * s * sw;
-                        to[(size_t)r * a.N] = o + bias;
+                        const float s = __shfl_sync(0xffffffffu, sx, r), o = patch[(r - h) * 33 + lane] * s * sw + bias;
+                        if (in && s != 0.f && sw != 0.f) to[(size_t)r * a.N] = o;
                     }
                 }
                 __syncwarp();
@@ -248,6 +360,8 @@ __global__ void __launch_bounds__(LIN_THREADS, 1) lin_gemm_kernel(const __grid_c
         }
     }
     if (failed) atomicOr(&g_linear_error, 1u);
+    const bool whole = !__syncthreads_or(failed);        // after a timeout copies may still land in the ring
+    if (__syncthreads_or(marks) && whole) lin_fix(a, ring_p);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
@@ -260,37 +374,48 @@ int linear_error_fetch() {
     return (int)v;
 }
 
-// workspace: limbs and inverse scales of w, then those of x
+// workspace: limbs, inverse scales and mark counts of w, then those of x
 static size_t lin_limbs(int64_t rows, int K) { return (size_t)rows * 2 * K * 2; }
 static size_t lin_scales(int64_t rows) { return ((size_t)rows * 4 + 255) & ~size_t(255); }
+static int lin_split_ctas(int rows) { return (int)min((int64_t)8 * sm_count(), ((int64_t)rows + 7) / 8); }
+struct LinPart {
+    __half* limbs;
+    float* inv;
+    int* marked;
+};
+static LinPart lin_part(char*& at, int rows, int K) {
+    LinPart p;
+    p.limbs = reinterpret_cast<__half*>(at);
+    p.inv = reinterpret_cast<float*>(at += lin_limbs(rows, K));
+    p.marked = reinterpret_cast<int*>(at += lin_scales(rows));
+    at += lin_scales(lin_split_ctas(rows));
+    return p;
+}
 
 bool linear_f32_supported(int K) { return K > 0 && K % 64 == 0 && K <= 64 * LIN_MAX_KB; }
 
 // w's half of the work, which needs nothing but w; the next kernel may start beside it
 int linear_f32_weights(const float* w, int N, int K, void* workspace, cudaStream_t st) {
-    char* p = static_cast<char*>(workspace);
-    lin_split_kernel<<<min(ceil_div(N, 8), 8 * sm_count()), 256, 0, st>>>(w, N, K, reinterpret_cast<__half*>(p),
-                                                                         reinterpret_cast<float*>(p + lin_limbs(N, K)));
+    char* at = static_cast<char*>(workspace);
+    const LinPart p = lin_part(at, N, K);
+    lin_split_kernel<<<lin_split_ctas(N), 256, 0, st>>>(w, N, K, p.limbs, p.inv, p.marked);
     count_launch(1);
     return check_launch("lin_split_kernel");
 }
 
 // the rest, behind a kernel that itself has waited for linear_f32_weights
 int linear_f32_rows(const float* x, const float* w, const float* bias, float* out, int M, int N, int K, void* workspace, cudaStream_t st) {
-    char* p = static_cast<char*>(workspace);
-    __half* wl = reinterpret_cast<__half*>(p);
-    float* sw = reinterpret_cast<float*>(p += lin_limbs(N, K));
-    __half* xl = reinterpret_cast<__half*>(p += lin_scales(N));
-    float* sx = reinterpret_cast<float*>(p + lin_limbs(M, K));
+    char* at = static_cast<char*>(workspace);
+    const LinPart pw = lin_part(at, N, K), px = lin_part(at, M, K);
     CUtensorMap tm_x, tm_w;
-    int rc = make_tmap_of(&tm_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, xl, M, 2 * K, 128);
-    if (rc == PIKV_OK) rc = make_tmap_of(&tm_w, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, wl, N, 2 * K, 128);
+    int rc = make_tmap_of(&tm_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, px.limbs, M, 2 * K, 128);
+    if (rc == PIKV_OK) rc = make_tmap_of(&tm_w, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, pw.limbs, N, 2 * K, 128);
     if (rc != PIKV_OK) return rc;
     if (!allow_smem<lin_gemm_kernel>()) return check_launch("linear_f32 smem attribute");
-    LinArgs a = {x, w, bias, sx, sw, out, M, N, K, ceil_div(M, 128), 0};
+    LinArgs a = {x, w, bias, px.inv, pw.inv, px.marked, pw.marked, lin_split_ctas(M), lin_split_ctas(N), out, M, N, K, ceil_div(M, 128), 0};
     a.items = (long long)ceil_div(N, LIN_BN) * a.mtiles;
     const int sms = sm_count();
-    launch_dependent(lin_split_kernel, dim3((unsigned)min(ceil_div(M, 8), 8 * sms)), 256, 0, st, x, M, K, xl, sx);
+    launch_dependent(lin_split_kernel, dim3((unsigned)lin_split_ctas(M)), 256, 0, st, x, M, K, px.limbs, px.inv, px.marked);
     launch_dependent(lin_gemm_kernel, dim3((unsigned)min((long long)sms, a.items)), LIN_THREADS, LIN_SMEM, st, tm_x, tm_w, a);
     count_launch(2);
     return check_launch("linear_f32");
@@ -304,7 +429,7 @@ extern "C" {
 
 size_t pikv_linear_f32_workspace_bytes(int32_t M, int32_t N, int32_t K) {
     if (M <= 0 || N <= 0 || K <= 0) return 0;
-    return lin_limbs((int64_t)M + N, K) + lin_scales(M) + lin_scales(N);
+    return lin_limbs((int64_t)M + N, K) + lin_scales(M) + lin_scales(N) + lin_scales(lin_split_ctas(M)) + lin_scales(lin_split_ctas(N));
 }
 
 int pikv_linear_f32(const float* x, const float* w, const float* bias, float* out, int32_t M, int32_t N, int32_t K, void* workspace,
