@@ -209,7 +209,7 @@ class PeerShardedKVCache:
             out = ops.gate_fused(act, w2, b2, top_k=top_k, capacity=0)
         # gate scratch owned by this binding: several prepared steps (lanes, buffer sets) run concurrently on
         # different streams, and the scratch holds the per-CTA counts the slot finalisation reads
-        ws = torch.empty(max(1, L.lib().pikv_gate_workspace_bytes(T, E, top_k)), dtype=torch.uint8, device=self.device)
+        ws = torch.empty(max(1, L.lib().pikv_gate_tail_workspace_bytes(T, E, top_k)), dtype=torch.uint8, device=self.device)
         out.workspace = ws
         b2f = None if b2 is None else ops._req(b2.to(torch.float32), "b2", torch.float32)
         gp = L.GateParams()
