@@ -775,6 +775,13 @@ PyObject* moe(PyObject* const* a, Py_ssize_t) {
         p.B = (int32_t)x.size(0); p.S = (int32_t)x.size(1); p.H = (int32_t)x.size(2);
         const int64_t H = p.H;
         need(H % 128 == 0 && H <= 1024);
+        // Wide models with many tokens: the fused layers run at a third of fp32 FMA rate and save the modules' launches, cuBLAS
+        // runs at two thirds.  Modules / fused, 4 experts: H = 1024, 5040 tokens 1.21 to 1.31 (one sequence, eight), 7128 tokens 1.06
+        // to 1.17, 10080 tokens 0.93 to 1.01, 65536 tokens 0.72 to 0.77; H = 768, 8960 tokens 1.04 to 1.19, 17920 tokens 0.87 to 0.98.  At
+        // H = 512 only a long single sequence loses (its sums are one CTA's): 28512 tokens 1.07, 65536 tokens 0.93, eight
+        // sequences 1.16 at 40328.  H = 256: 1.3 to 1.6 at 161312 tokens.  More experts move the line up (16, H = 1024: 1.68 at 3536 tokens).
+        const int64_t rows = H > 512 ? (int64_t)p.B * p.S : H > 256 ? p.S : 0;
+        need(rows * H * H <= (H > 512 ? int64_t(1) << 33 : int64_t(11) << 30));
         const Mod m(a[0], types, W::MOE);
         const Mod experts = walk.list(m.child(PIKV_NAME("experts")), W::MODULES, -1), caches = walk.list(m.child(PIKV_NAME("kv_caches")), W::MODULES, -1);
         const int64_t E = PyDict_GET_SIZE(experts.get(PIKV_NAME("_modules")));
