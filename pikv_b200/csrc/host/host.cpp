@@ -859,7 +859,12 @@ PyObject* moe(PyObject* const* a, Py_ssize_t) {
     const size_t row = ((size_t)T * E * 4 + 255) & ~size_t(255);
     size_t tail[3], total = ((p.workspace_bytes + 255) & ~size_t(255)) + 3 * row;
     for (int i = 0; i < 3; ++i) total += tail[i] = (pikv_gate_tail_workspace_bytes(T, E, topk[i]) + 255) & ~size_t(255);
-    const at::Tensor ws = workspace(x, total);
+    at::Tensor ws;                             // all experts' outputs among it, where the modules hold one at a time
+    try {
+        ws = workspace(x, total);
+    } catch (const c10::OutOfMemoryError&) {
+        Py_RETURN_NONE;
+    }
     char* base = ptr<char>(ws);
     p.workspace = base;
     base += (p.workspace_bytes + 255) & ~size_t(255);

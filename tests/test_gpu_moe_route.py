@@ -58,3 +58,26 @@ def test_route_and_results(taken, hidden, batch, seq, fused):
             for a, b in zip(m.kv_caches, other.kv_caches):
                 for n in ("keys", "values", "importance"):
                     assert float((getattr(a, n) - getattr(b, n)).norm()) <= 1e-4 * float(getattr(b, n).norm()) + 1e-6
+
+
+def test_modules_run_where_the_workspace_does_not_fit(taken):
+    m = _model(16, 128)
+    other = copy.deepcopy(m)
+    x = torch.randn(8, 16384, 128, device="cuda")
+    needs = 16 * x.numel() * 4                            # all experts' outputs
+    other._fused = lambda x: None
+    with torch.no_grad():
+        torch.cuda.empty_cache()
+        torch.cuda.reset_peak_memory_stats()
+        want = other(x).cpu()
+        peak = torch.cuda.max_memory_reserved()
+        torch.cuda.empty_cache()
+        if peak + (64 << 20) >= torch.cuda.memory_reserved() + needs:
+            pytest.skip("the modules need as much")
+        torch.cuda.set_per_process_memory_fraction((peak + (64 << 20)) / torch.cuda.get_device_properties(0).total_memory)
+        try:
+            got = m(x).cpu()
+        finally:
+            torch.cuda.set_per_process_memory_fraction(1.0)
+    assert taken == [False]
+    assert float((got - want).norm() / want.norm()) < 1e-5
