@@ -19,6 +19,7 @@ struct AppendDev {
     const void* k;
     const void* v;
     int T, n_kv, top_k, log2_nkv;
+    int few;                     // the grid leaves SMs free: kernels behind it may become resident at once
     const int* dst_seq;
     const int* slot;
     const int* page_table;
@@ -178,7 +179,7 @@ __device__ __forceinline__ void kv_append_body(const AppendDev& a) {
     typename GQ::Raw k0, v0, k1, v1;
     // a decode step's few rows: whatever follows may become resident at once (not behind a grid that fills the GPU: its
     // waiting CTAs would hold the registers that kernels of other streams need)
-    if (gridDim.x <= 148) dependency_release();
+    if (a.few) dependency_release();
     // MODE 2: the K / V loads need nothing from the gate and go out before the wait
     if (MODE != 2) dependency_wait();
     if (any) append_stage_kv<TIn, BITS, SYM>(a, pair, total, sub, k0, v0);
@@ -438,12 +439,18 @@ static void append_fill_common(const pikv_append_params* p, AppendDev& a) {
     append_clear_gate(a);
 }
 
-template <typename TIn>
-static int launch_append(const AppendDev& a, int bits, int symmetric, cudaStream_t st) {
+// persistent grid: eight lanes per row and head, at most `per_sm` CTAs per SM
+static int append_grid(AppendDev& a, int per_sm) {
     const long long lanes = (long long)a.T * a.n_kv * 8;
+    const int grid = (int)std::min<long long>(ceil_div64(lanes, APPEND_THREADS), (long long)sm_count() * per_sm);
+    a.few = grid <= sm_count();
+    return grid;
+}
+
+template <typename TIn>
+static int launch_append(AppendDev& a, int bits, int symmetric, cudaStream_t st) {
     // persistent: at most three resident CTAs per SM, each group strides over its items
-    long long want = ceil_div64(lanes, APPEND_THREADS), cap_ctas = (long long)sm_count() * 3;
-    const int grid = (int)(want < cap_ctas ? want : cap_ctas);
+    const int grid = append_grid(a, 3);
 #define PIKV_APPEND_LAUNCH(BITS, SYM)                                                                   \
     do {                                                                                                \
         if (a.top_k <= 1) launch_dependent(kv_append_quant_kernel<TIn, BITS, SYM, 1, 0>, grid, APPEND_THREADS, 0, st, a);      \
@@ -505,9 +512,7 @@ extern "C" int pikv_kv_append_rope(const pikv_append_params* p, const float* rop
     append_fill_common(p, a);
     a.rope_cos = rope_cos; a.rope_sin = rope_sin; a.rope_pos = positions; a.rope_max_pos = max_pos;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const long long lanes = (long long)a.T * a.n_kv * 8;
-    long long want = ceil_div64(lanes, APPEND_THREADS), cap_ctas = (long long)sm_count() * 3;
-    const int grid = (int)(want < cap_ctas ? want : cap_ctas);
+    const int grid = append_grid(a, 3);
     if (a.top_k <= 1) launch_dependent(kv_append_quant_kernel<__nv_bfloat16, 8, true, 1, 4>, grid, APPEND_THREADS, 0, st, a);
     else if (a.top_k <= 2) launch_dependent(kv_append_quant_kernel<__nv_bfloat16, 8, true, 2, 4>, grid, APPEND_THREADS, 0, st, a);
     else if (a.top_k <= 4) launch_dependent(kv_append_quant_kernel<__nv_bfloat16, 8, true, 4, 4>, grid, APPEND_THREADS, 0, st, a);
@@ -567,9 +572,7 @@ extern "C" int pikv_route_append(const pikv_gate_params* gp, const pikv_append_p
     a.gG = g.G; a.gchunk = g.chunk; a.gE = g.E; a.gcap = g.capacity;
     a.slot = g.slot;               // chunk-local ranks, in the gate's workspace
     a.g_slot_out = gp->slot; a.g_counts_k = g.counts_k; a.g_prob_sum = g.prob_sum; a.g_new_len = g.new_len;
-    const long long lanes = (long long)a.T * a.n_kv * 8;
-    long long want = ceil_div64(lanes, APPEND_THREADS), cap_ctas = (long long)sm_count() * 3;
-    const int grid = (int)(want < cap_ctas ? want : cap_ctas);
+    const int grid = append_grid(a, 3);
     // programmatic dependent launch: the append CTAs are scheduled as soon as every gate CTA has started (the gate
     // kernel signals that at its top), so the launch latency and the first loads overlap the gate's tail
     cudaLaunchConfig_t cfg = {};
@@ -847,11 +850,9 @@ extern "C" int pikv_kv_append_sharded(const pikv_append_sharded_params* sp, pikv
         a.pscale[1][r] = on ? static_cast<uint16_t*>(sp->peer_v_scale[r]) : nullptr;
     }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const long long lanes = (long long)a.T * a.n_kv * 8;
     // two CTAs per SM: the link, not the SMs, bounds this launch (one, two and three per SM measured within 5 %),
     // and kernels of the other steps in flight still find room beside them
-    long long want = ceil_div64(lanes, APPEND_THREADS), cap_ctas = (long long)sm_count() * 2;
-    const int grid = (int)(want < cap_ctas ? want : cap_ctas);
+    const int grid = append_grid(a, 2);
     if (a.top_k <= 1) kv_append_quant_kernel<__nv_bfloat16, 8, true, 1, 1><<<grid, APPEND_THREADS, 0, st>>>(a);
     else if (a.top_k <= 2) kv_append_quant_kernel<__nv_bfloat16, 8, true, 2, 1><<<grid, APPEND_THREADS, 0, st>>>(a);
     else if (a.top_k <= 4) kv_append_quant_kernel<__nv_bfloat16, 8, true, 4, 1><<<grid, APPEND_THREADS, 0, st>>>(a);
@@ -904,9 +905,7 @@ extern "C" int pikv_kv_append_striped(const pikv_append_striped_params* sp, pikv
         a.pscale[1][r] = on ? static_cast<uint16_t*>(sp->peer_v_scale[r]) : nullptr;
     }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const long long lanes = (long long)a.T * a.n_kv * 8;
-    long long want = ceil_div64(lanes, APPEND_THREADS), cap_ctas = (long long)sm_count() * (sp->world > 1 ? 2 : 3);
-    const int grid = (int)(want < cap_ctas ? want : cap_ctas);
+    const int grid = append_grid(a, sp->world > 1 ? 2 : 3);
     if (a.top_k <= 1) kv_append_quant_kernel<__nv_bfloat16, 8, true, 1, 3><<<grid, APPEND_THREADS, 0, st>>>(a);
     else if (a.top_k <= 2) kv_append_quant_kernel<__nv_bfloat16, 8, true, 2, 3><<<grid, APPEND_THREADS, 0, st>>>(a);
     else if (a.top_k <= 4) kv_append_quant_kernel<__nv_bfloat16, 8, true, 4, 3><<<grid, APPEND_THREADS, 0, st>>>(a);

@@ -7,6 +7,7 @@
 #include <stdint.h>
 #include <stdio.h>
 #include <stdarg.h>
+#include <algorithm>
 #include <atomic>
 
 #include "../../include/pikv_b200.h"
