@@ -574,7 +574,8 @@ extern "C" int pikv_route_append(const pikv_gate_params* gp, const pikv_append_p
     a.g_slot_out = gp->slot; a.g_counts_k = g.counts_k; a.g_prob_sum = g.prob_sum; a.g_new_len = g.new_len;
     const int grid = append_grid(a, 3);
     // programmatic dependent launch: the append CTAs are scheduled as soon as every gate CTA has started (the gate
-    // kernel signals that at its top), so the launch latency and the first loads overlap the gate's tail
+    // kernel signals that at its top), so the launch latency and the first loads overlap the gate's tail.  The gate has to stay
+    // a plain launch: the first K and V rows are read before the wait, and only that launch orders them behind their producer.
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(APPEND_THREADS);

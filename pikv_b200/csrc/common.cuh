@@ -44,7 +44,10 @@ static inline bool allow_smem(int bytes = 227 * 1024) {
 
 // Launches a kernel that may become resident before the previous kernel of the stream has finished: it executes
 // griddepcontrol.wait before it touches memory, so only its start-up overlaps the predecessor's end (the gap between two
-// dependent launches is 2 to 2.5 us without it).
+// dependent launches is 2 to 2.5 us without it).  A wait is for the previous kernel alone: some thread of every kernel in a
+// chain has to wait before its grid ends, or what follows does not see the kernels before it.  Kernels that read or write
+// before their wait (the fused append's first K and V rows, moe_stats_kernel, moe_gemm_kernel) rely on a plain launch in
+// front of them, as their launchers say.
 template <typename... KArgs, typename... Args>
 static inline void launch_dependent(void (*kern)(KArgs...), dim3 grid, int block, size_t smem, cudaStream_t st, const Args&... args) {
     cudaLaunchConfig_t cfg = {};

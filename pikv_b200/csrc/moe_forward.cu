@@ -411,6 +411,9 @@ int pikv_moe_forward(const pikv_moe_params* p, pikv_stream_t stream) {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     char* linear = static_cast<char*>(p->workspace) + own;
     const int T = p->B * p->S, mt = ceil_div(T, MOE_TILE), nt = p->H / MOE_TILE;
+    // The first kernel has to stay a plain launch: moe_stats_kernel and the gate tiles of moe_gemm_kernel read x, weights and
+    // caches and write the workspace without a wait, and only this launch orders them behind what came before.  The expert
+    // CTAs of both wait before they end, so what waits for either kernel finds its predecessors finished too.
     // The projection's weights are split beside moe_stats_kernel: one streams memory, the other is a chain on a few SMs.
     if (p->V) {
         const int rc = linear_f32_weights(p->vocab_w, p->V, p->H, linear, st);
