@@ -149,8 +149,10 @@ class SVDCompressor(BaseCompressor):
     def reconstruct(self, latent: torch.Tensor, which: str = "key") -> torch.Tensor:
         return _linear(self.key_reconstructor if which == "key" else self.value_reconstructor, latent, False)
 
-    #: rows of K (and of V) from which the round trip of both is one kernel: it has one CTA per 128 rows, and below
-    #: this (64 CTAs) the separate products, which also spread over their columns, use more of the chip
+    #: rows of K (and of V) from which the round trip of both is one kernel.  It has one CTA per 128 rows, the separate products
+    #: also spread over their columns, so the line depends on the width.  One kernel / separate products in us, rank 64: width 512,
+    #: 4096 rows 12 / 23; width 1024, 512 rows 18 / 24, 4096 rows 19 / 29; width 2048, 512 rows 31 / 31, 4096 rows 34 / 42; width 4096,
+    #: 2048 rows 69 / 57, 4096 rows 88 / 79, 8192 rows 98 / 105.  4096 is safe up to a width of 2048 and late below it.
     PAIR_ROWS = 4096
 
     def _round_trip(self, keys: torch.Tensor, values: torch.Tensor):

@@ -19,7 +19,9 @@
 // Bound by the tensor cores and by what L2 delivers to an SM: a pair shares each operand tile, 32 KB per SM for
 // 128 x 256 x 64 multiply-adds.  bn is 256, or narrower while that leaves pairs without an item.
 // 4096 -> 4096 -> 8: 2048 tokens 632 us with one CTA per 128 tokens walking all hidden units (16 CTAs), 52 us now = 1.32
-// PFLOP/s; 16384 tokens 783 us, now 424 us with the tail = 1.30 PFLOP/s (a library GEMM, ReLU and the gate: 475 us).
+// PFLOP/s; 16384 tokens 783 us, now 442 us with the tail in a short burst = 1.25 PFLOP/s and 546 us back to back for seconds
+// under the power cap.  The library is ahead there: its GEMM with bias and ReLU in the epilogue and the gate behind it take 382
+// and 442 us (with a separate ReLU 413 and 484).
 // Of the 52, 13 us came from keeping the operands of the issuing instructions warp-uniform (lr_elect).
 // Every mbarrier wait is bounded; on a timeout the CTA raises the gate's sticky error word and drains.
 #include "gate_common.cuh"

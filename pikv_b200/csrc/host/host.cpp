@@ -459,7 +459,7 @@ PyObject* decode(PyObject* const* a, Py_ssize_t n) {
         p.score_stride = scores.defined() ? (int32_t)scores.size(-1) : 0;
         holds(scores, (int64_t)p.B * p.n_q * p.score_stride, "scores");
     }
-    // output, log-sum-exp and scratch from one allocation
+    // scratch sized for this call's batch
     const size_t scratch = pikv_decode_attn_workspace_bytes(p.B, p.n_q, p.n_kv, 0, 0);
     at::Tensor out = at::empty_like(q), lse, ws = workspace(q, scratch);
     if (want_lse) lse = at::empty({p.B, p.n_q}, on(q, at::kFloat));
